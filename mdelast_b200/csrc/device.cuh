@@ -100,12 +100,10 @@ struct TablesView {
     double rhomax[kMaxTypes];
     double mass[kMaxTypes];
     // mixed precision: the r tables in FP32 with lengths in angstrom and values in eV
-    // (phi) or angstrom^-3 (rho). rbf: per type pair (a <= b) and interval one record of
-    // TabFmt<IP>::kB floats holding phi_ab, rho_a, rho_b at strides of kFb (the force
-    // pass reads all three at one r, from one place); rrf: per type and interval one
-    // record of kFf floats holding rho (the density pass reads one function per pair).
-    // Cutoffs in angstrom.
-    const float *rbf, *rrf;
+    // (phi) or angstrom^-3 (rho), one record of TabFmt<IP>::kFf floats per function and
+    // interval: phf phi_ab of every type pair (a <= b), rrf rho of every type. Cutoffs in
+    // angstrom.
+    const float *phf, *rrf;
     float finv_hr, finv_hr2, fr_cut_sq, fpad;
     // Staged copy for the shared-memory force pass (quintic only): the intervals
     // [st_lo, st_lo + st_n) of every phi_ab (slot s at s * st_n) followed by every rho_a
@@ -261,13 +259,13 @@ __device__ __forceinline__ void ld6(const double *p, double c[6]) {
 // a pair-table bundle holds three functions (phi_ab, rho_a, rho_b).
 template <int IP> struct TabFmt {
     static constexpr int kF = IP == MDELAST_BSPLINE ? 12 : 6;
-    // FP32 records of the mixed-precision tables, packed (a quintic's 6 coefficients in 24
-    // bytes, 3 x 24 = 72 bytes per pair bundle): the pair passes are limited by how much of
-    // the tables the L1 cache holds (measured: 96- and 128-byte bundles make the force pass
-    // 7 % and 19 % slower; 32-byte rho records make the density pass 4.5 % slower).
-    static constexpr int kFf = IP == MDELAST_BSPLINE ? 12 : 6;
-    static constexpr int kFb = IP == MDELAST_BSPLINE ? 12 : 6;
-    static constexpr int kB = 3 * kFb;
+    // FP32 records of the mixed-precision tables: a quintic's 6 coefficients and two pads in
+    // 32 bytes (one 256-bit load), a bspline's 12 in 48. The pair passes are bound by the L1's
+    // data pipe, which serves about 32 scattered bytes per cycle however they are asked for
+    // (force pass, wavefronts per gather of 32 lanes: 8 bytes 9, 16 bytes 16, 32 bytes 27), so
+    // one record per function, read once per pair of one type, replaced a 72-byte bundle of
+    // phi_ab, rho_a, rho_b read with nine 8-byte loads.
+    static constexpr int kFf = IP == MDELAST_BSPLINE ? 12 : 8;
 };
 
 __device__ __forceinline__ double cubic_at(const double *p, double t) {

@@ -132,8 +132,8 @@ int default_tpa(int n_atoms) {
 // atom group of kBlock/tpa atoms. Fills each replica's block range and the block ->
 // replica map; returns the grid size.
 constexpr int kTargetBlocks = 148 * 32;
-// shared memory for the staged force tables: beside it the kernel keeps its FP64
-// accumulators (40 KB at 4 lanes per atom) within the 227 KB a block may take
+// shared memory for the staged force tables: the rest of the SM's 228 KB is the L1 of the
+// partner gathers
 constexpr long kStageBudget = 184 * 1024;
 // k_sublist grid: one wave, 5 resident blocks of 256 threads (48 registers each: 5 blocks
 // fill the register file) on each of the 148 SMs
@@ -211,7 +211,7 @@ struct mdelast_driver_s {
     int precision = MDELAST_PRECISION_FP64;
     float4 *d_posf = nullptr;
     float2 *d_dF2f = nullptr;
-    float *d_rbf = nullptr, *d_rrf = nullptr;
+    float *d_phf = nullptr, *d_rrf = nullptr;
     void pass_density(bool obs, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED)
             launch_density_mx(obs, tpa_d, grid_d, s, A, T);
@@ -345,7 +345,7 @@ mdelast_driver_s::~mdelast_driver_s() {
     dfree(d_dF2);
     dfree(d_posf);
     dfree(d_dF2f);
-    dfree(d_rbf);
+    dfree(d_phf);
     dfree(d_rrf);
     dfree(d_stf);
     dfree(d_nbr);
@@ -1305,11 +1305,11 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
     }
     d->precision = c0.precision;
     if (c0.precision == MDELAST_PRECISION_MIXED) {
-        // The r tables in FP32, angstrom / eV (phi) and angstrom^-3 (rho): per type pair
-        // and interval a bundle of phi_ab, rho_a, rho_b; per type and interval rho. Quintic
+        // The r tables in FP32, angstrom / eV (phi) and angstrom^-3 (rho): per type pair and
+        // interval a record of phi_ab, per type and interval one of rho. Quintic
         // coefficients carry the function's unit (derivatives come with 1/h in angstrom);
         // the bspline cubics of f' and f'' carry one and two more 1/length.
-        size_t const kFf = bsp ? 12 : 6, kFb = bsp ? 12 : 6, kB = 3 * kFb;
+        size_t const kFf = bsp ? TabFmt<MDELAST_BSPLINE>::kFf : TabFmt<MDELAST_QUINTIC>::kFf;
         double const a3 = kAng * kAng * kAng;
         auto pack = [&](const double *src, double unit, float *dst) {
             for (size_t c = 0; c < kF; ++c) {
@@ -1319,34 +1319,26 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
                 dst[c] = static_cast<float>(src[c] * f);
             }
         };
-        std::vector<float> rbf(static_cast<size_t>(npot) * nri * kB, 0.f);
+        std::vector<float> phf(static_cast<size_t>(npot) * nri * kFf, 0.f);
         std::vector<float> rrf(static_cast<size_t>(nt) * nri * kFf, 0.f);
-        for (int b = 0; b < nt; ++b)
-            for (int a = 0; a <= b; ++a) {
-                int const s = b * (b + 1) / 2 + a;
-                for (int k = 0; k < nri; ++k) {
-                    float *o = rbf.data() + (static_cast<size_t>(s) * nri + k) * kB;
-                    pack(fun(c0.pair[s]->table, k), 1. / kEv, o);
-                    if (c0.n_eam) {
-                        pack(fun(c0.eam[a]->rho, k), a3, o + kFb);
-                        pack(fun(c0.eam[b]->rho, k), a3, o + 2 * kFb);
-                    }
-                }
-            }
+        for (int q = 0; q < npot; ++q)
+            for (int k = 0; k < nri; ++k)
+                pack(fun(c0.pair[q]->table, k), 1. / kEv,
+                     phf.data() + (static_cast<size_t>(q) * nri + k) * kFf);
         for (int t = 0; t < c0.n_eam; ++t)
             for (int k = 0; k < nri; ++k)
                 pack(fun(c0.eam[t]->rho, k), a3,
                      rrf.data() + (static_cast<size_t>(t) * nri + k) * kFf);
-        TRY(dalloc(&d->d_rbf, rbf.size()));
+        TRY(dalloc(&d->d_phf, phf.size()));
         TRY(dalloc(&d->d_rrf, rrf.size()));
-        if (cudaMemcpy(d->d_rbf, rbf.data(), sizeof(float) * rbf.size(), cudaMemcpyHostToDevice) ||
+        if (cudaMemcpy(d->d_phf, phf.data(), sizeof(float) * phf.size(), cudaMemcpyHostToDevice) ||
             cudaMemcpy(d->d_rrf, rrf.data(), sizeof(float) * rrf.size(), cudaMemcpyHostToDevice))
             return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
-        T.rbf = d->d_rbf;
+        T.phf = d->d_phf;
         T.rrf = d->d_rrf;
         // The staged copy of the force pass: every phi_ab, then every rho_a, over the top
         // intervals of the r grid (those below r_cut, as many as kStageBudget holds), the
-        // same FP32 values as the bundles. Quintic EAM tables only.
+        // same FP32 values as phf and rrf. Quintic EAM tables only.
         if (!bsp && c0.n_eam) {
             int const n_fun = npot + nt;
             double rc_max = 0.;

@@ -29,18 +29,6 @@ __device__ __forceinline__ int tab_locate_f(float x, float inv_h, int n, float &
     return i;
 }
 
-// the 6 quintic coefficients of a packed (8-byte aligned) record
-__device__ __forceinline__ void ld6f(const float *p, float c[6]) {
-    const float2 *q = reinterpret_cast<const float2 *>(p);
-    float2 const a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
-    c[0] = a.x;
-    c[1] = a.y;
-    c[2] = b.x;
-    c[3] = b.y;
-    c[4] = d.x;
-    c[5] = d.y;
-}
-
 // The pair force is evaluated from both of its atoms, in different code paths of the
 // force pass; its arithmetic is written with explicit rounding (no contraction left to
 // the compiler) so that both evaluations give the same bits.
@@ -78,8 +66,8 @@ __device__ __forceinline__ void tabf_eval(const float *p, float t, float inv_h, 
         if (ND2)
             d2 = cubicf_at(p + 8, t);
     } else {
-        float c[6];
-        ld6f(p, c);
+        float c[8]; // 6 coefficients, 2 pads
+        ld256(p, c);
         if (NV)
             v = tabf_v(c, t);
         if (ND1)
@@ -158,25 +146,24 @@ __device__ __forceinline__ void dens_loop(AtomsView const &A, TablesView const &
 }
 
 // Density pass of md_driver.cpp:195-277 in mixed precision (see k_density for the roles).
-// The block's FP64 sums (embedding energy, the per-atom Born term F''_i g_i g_i^T and
-// Laplacian term) are folded warp by warp after each atom group into per-warp shared
-// accumulators instead of being carried in registers through the pair loop: the loop then
-// runs with about half the registers, so twice the warps per SM hide the latency of the
-// partner gathers.
+// The atom's terms of the block's FP64 sums (embedding energy, the per-atom Born term
+// F''_i g_i g_i^T and the Laplacian term) are formed in every lane of the atom, so that
+// warp_slots spreads them over the lanes with 7 exchanges at 4 lanes per atom; each lane
+// carries one running sum. (Before, 23 warp sums per atom group: 18 % of the pass's L1 data
+// pipe went to their shuffles.)
 //
 // Bounded to 8 blocks of 128 threads per SM (64 registers; the compiler's own choice is 72,
 // 7 blocks): a few bytes of spills, and the extra warps hide more of the gather latency
 // (0.194 -> 0.182 ms at 16 x 13,500 atoms; 9 and 10 blocks spilled more and ran slower).
+// Bound by the L1 data pipe (65 % of its wavefront rate, issue 49 %): at 16 x 13,500 atoms and
+// 4 lanes per atom 0.195 -> 0.162 ms with the 32-byte records and warp_slots.
 template <bool OBS, int TPA, int IP, typename IX>
 __global__ void __launch_bounds__(kBlock, 8) k_density_mx(AtomsView A, TablesView T) {
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     constexpr int kF = TabFmt<IP>::kF;
-    __shared__ double sacc[kBlock / 32][D_NSUM];
-    int const warp = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < (kBlock / 32) * D_NSUM; k += kBlock)
-        (&sacc[0][0])[k] = 0.;
-    __syncthreads();
+    constexpr int kSlots = OBS ? D_NSUM : 1, kP2 = slots_pow2(kSlots);
+    double acc = 0.; // the block sum of this lane's slot over the warp's atom groups
     int const r = A.dblk_rep[blockIdx.x];
     Replica const *R = A.rep + r;
     int const lb = blockIdx.x - R->dblk_begin, nb = R->dblk_n;
@@ -214,8 +201,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_density_mx(AtomsView A, TablesVie
                 hv[u] = group_sum<TPA>(hv[u]);
         }
         double F = 0., d2F = 0.;
-        bool const own = valid && sub == 0;
-        if (own) {
+        if (valid) { // every lane of the atom, stored by the first
             // the embedding function in FP64 and cgs (eam.hpp:48-70)
             double const rc = rho / a3;
             if (rc > T.rhomax[ti])
@@ -225,42 +211,53 @@ __global__ void __launch_bounds__(kBlock, 8) k_density_mx(AtomsView A, TablesVie
             double dF = 0.;
             tab_eval<IP, true, true, OBS>(T.Ft + (static_cast<size_t>(ti) * T.nfi + k) * kF, t,
                                           T.inv_hf, T.inv_hf2, F, dF, d2F);
-            A.rho[i] = rc;
-            A.Fe[i] = F;
             // F' [erg cm^3] -> [eV A^3] and F'' [erg cm^6] -> [eV A^6]
-            if (OBS) {
-                A.dF2[i] = make_double2(dF, d2F);
-                A.dF2f[i] = make_float2(static_cast<float>(dF / (a3 * kEv)),
-                                        static_cast<float>(d2F / (a3 * a3 * kEv)));
-            } else {
-                A.dF2[i].x = dF;
-                A.dF2f[i].x = static_cast<float>(dF / (a3 * kEv));
+            if (sub == 0) {
+                A.rho[i] = rc;
+                A.Fe[i] = F;
+                if (OBS) {
+                    A.dF2[i] = make_double2(dF, d2F);
+                    A.dF2f[i] = make_float2(static_cast<float>(dF / (a3 * kEv)),
+                                            static_cast<float>(d2F / (a3 * a3 * kEv)));
+                } else {
+                    A.dF2[i].x = dF;
+                    A.dF2f[i].x = static_cast<float>(dF / (a3 * kEv));
+                }
             }
         }
-        warp_accumulate(F, &sacc[warp][D_FSUM]);
+        // the atom's terms of the block sums, equal in its TPA lanes (zero without an atom)
+        double v[kP2] = {};
+        v[D_FSUM] = F;
         if (OBS) {
-            // g in cm^-3 and h in cm^-4, as the cgs F'' expects; zero for lanes without an atom
+            // g in cm^-3 and h in cm^-4, as the cgs F'' expects
+            double const ia3 = 1. / a3, iha = 1. / (a3 * kAng);
             double gc[6];
 #pragma unroll
             for (int u = 0; u < 6; ++u)
-                gc[u] = own ? static_cast<double>(g[u]) / a3 : 0.;
+                gc[u] = static_cast<double>(g[u]) * ia3;
             int q = D_CB;
 #pragma unroll
             for (int u = 0; u < 6; ++u)
 #pragma unroll
-                for (int v = u; v < 6; ++v)
-                    warp_accumulate(d2F * gc[u] * gc[v], &sacc[warp][q++]);
-            double const ha = a3 * kAng;
-            double const h0 = hv[0] / ha, h1 = hv[1] / ha, h2 = hv[2] / ha;
-            warp_accumulate(own ? d2F * (h0 * h0 + h1 * h1 + h2 * h2) : 0., &sacc[warp][D_LAP]);
+                for (int w = u; w < 6; ++w)
+                    v[q++ % kP2] = d2F * gc[u] * gc[w];
+            double const h0 = hv[0] * iha, h1 = hv[1] * iha, h2 = hv[2] * iha;
+            v[D_LAP % kP2] = d2F * (h0 * h0 + h1 * h1 + h2 * h2);
         }
+        acc += warp_slots<kP2, TPA>(v);
     }
+    // the warps' slots into the block sums; unsampled steps form the embedding energy only
+    __shared__ double s_acc[kBlock / 32][kP2];
+    int const lane = threadIdx.x & 31;
+    if (lane < kP2)
+        s_acc[threadIdx.x >> 5][lane_slot<kP2>(lane)] = acc;
     __syncthreads();
-    for (int k = threadIdx.x; k < D_NSUM; k += blockDim.x) {
+    for (int k = threadIdx.x; k < D_NSUM; k += kBlock) {
         double s = 0.;
+        if (k < kSlots)
 #pragma unroll
-        for (int w = 0; w < kBlock / 32; ++w)
-            s += sacc[w][k];
+            for (int w = 0; w < kBlock / 32; ++w)
+                s += s_acc[w][k];
         A.pd[static_cast<size_t>(blockIdx.x) * D_NSUM + k] = s;
     }
 }
@@ -290,12 +287,13 @@ struct RowIn {
 };
 
 // The quintic coefficients of phi_s, rho_ti and rho_tj on interval k: from the staged
-// shared-memory copy (STAGED and k staged) or from the global pair bundle. Both hold the
-// same FP32 values, so the pair terms do not depend on where they were read.
+// shared-memory copy (STAGED and k staged) or from the global records. Both hold the same
+// FP32 values, so the pair terms do not depend on where they were read. A pair of one type
+// reads its one rho once.
 template <bool STAGED>
 __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *stab, int s,
-                                           int ti, int tj, int k, float cp[6], float ci[6],
-                                           float cj[6]) {
+                                           int ti, int tj, int k, float (&cp)[8],
+                                           float (&ci)[8], float (&cj)[8]) {
     if (STAGED) {
         unsigned const q = static_cast<unsigned>(k - T.st_lo);
         if (q < static_cast<unsigned>(T.st_n)) {
@@ -317,13 +315,14 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
             return;
         }
     }
-    constexpr int kFb = TabFmt<MDELAST_QUINTIC>::kFb;
-    const float *bundle = T.rbf + (static_cast<size_t>(s) * T.nri + k) * TabFmt<MDELAST_QUINTIC>::kB;
-    // rho_a of the bundle belongs to the smaller type of the pair
-    int const oi = (ti <= tj) ? kFb : 2 * kFb, oj = (ti < tj) ? 2 * kFb : kFb;
-    ld6f(bundle, cp);
-    ld6f(bundle + oi, ci);
-    ld6f(bundle + oj, cj);
+    constexpr int kFf = TabFmt<MDELAST_QUINTIC>::kFf;
+    ld256(T.phf + (static_cast<size_t>(s) * T.nri + k) * kFf, cp);
+    ld256(T.rrf + (static_cast<size_t>(ti) * T.nri + k) * kFf, ci);
+#pragma unroll
+    for (int u = 0; u < 6; ++u)
+        cj[u] = ci[u];
+    if (ti != tj)
+        ld256(T.rrf + (static_cast<size_t>(tj) * T.nri + k) * kFf, cj);
 }
 
 // One lane's walk over list slots [s0, s1) of an atom row (slots of partners j > i when
@@ -369,7 +368,6 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         int const s = pair_slot(ti, tj);
         float t;
         int const k = tab_locate_f(dr, T.finv_hr, T.nri, t);
-        constexpr int kFb = TabFmt<IP>::kFb;
         float V = 0.f, dV = 0.f, d2V = 0.f;
         float drho_i = 0.f, drho_j = 0.f, d2rho_i = 0.f, d2rho_j = 0.f;
         if (in_cut && dr < T.fpot_rmin[s])
@@ -378,7 +376,7 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         bool const eam_j = T.has_eam && (UC || !(dr > T.feam_rcut[tj]));
         if constexpr (IP == MDELAST_QUINTIC) {
             // the three functions' coefficients first (independent loads), then the math
-            float cp[6], ci[6], cj[6];
+            float cp[8], ci[8], cj[8];
             pair_coefs<STAGED>(T, stab, s, ti, tj, k, cp, ci, cj);
             if (UC || !(dr > T.fpot_rcut[s])) {
                 V = tabf_v(cp, t);
@@ -397,18 +395,19 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
                     d2rho_j = tabf_d2(cj, t, T.finv_hr2);
             }
         } else {
-            const float *bundle = T.rbf + (static_cast<size_t>(s) * T.nri + k) * TabFmt<IP>::kB;
+            constexpr int kFf = TabFmt<IP>::kFf;
             if (UC || !(dr > T.fpot_rcut[s]))
-                tabf_eval<IP, true, true, OBS>(bundle, t, T.finv_hr, T.finv_hr2, V, dV, d2V);
-            // rho'_{t_i} and rho'_{t_j} at r: rho_a of the bundle belongs to the smaller type
-            int const oi = (ti <= tj) ? kFb : 2 * kFb, oj = (ti < tj) ? 2 * kFb : kFb;
+                tabf_eval<IP, true, true, OBS>(T.phf + (static_cast<size_t>(s) * T.nri + k) * kFf,
+                                               t, T.finv_hr, T.finv_hr2, V, dV, d2V);
             float unused = 0.f;
             if (eam_i)
-                tabf_eval<IP, false, true, OBS>(bundle + oi, t, T.finv_hr, T.finv_hr2, unused,
-                                                drho_i, d2rho_i);
+                tabf_eval<IP, false, true, OBS>(
+                    T.rrf + (static_cast<size_t>(ti) * T.nri + k) * kFf, t, T.finv_hr,
+                    T.finv_hr2, unused, drho_i, d2rho_i);
             if (eam_j)
-                tabf_eval<IP, false, true, OBS>(bundle + oj, t, T.finv_hr, T.finv_hr2, unused,
-                                                drho_j, d2rho_j);
+                tabf_eval<IP, false, true, OBS>(
+                    T.rrf + (static_cast<size_t>(tj) * T.nri + k) * kFf, t, T.finv_hr,
+                    T.finv_hr2, unused, drho_j, d2rho_j);
         }
         float dedr = dV, X = 0.f, lap = 0.f;
         if (OBS) {
@@ -476,11 +475,14 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
 // Force pass of md_driver.cpp:300-430 (with the closing kick) in mixed precision; see
 // k_force for the roles of the terms. Each atom row is walked in two loops, partners j > i
 // (which also feed the global sums) and partners j < i, so the lanes of a warp do not
-// diverge on the global-sum work. The FP64 block accumulators live in shared memory
-// (slot-major), one set per group of TPA lanes: each atom's pair sums are combined across
-// its lanes in FP64 first, which keeps the accumulators at 36 slots per group instead of
-// per thread (5.6 KB instead of 37 KB per block at 8 lanes per atom) and leaves that
-// shared memory to the L1 that caches the tables (measured 2-4 % faster).
+// diverge on the global-sum work. The row's 22 pair sums and, after the kick, its 12 sums
+// over atoms go through warp_slots (31 and, at 4 lanes per atom, 4 exchanges) into two FP64
+// registers per lane; the virial is the trace of the Born stress.
+//
+// What bounds it: the L1 data pipe (61 % of its wavefront rate) and instruction issue
+// (53 %), at 4 blocks of 4 warps per SM. At 16 x 13,500 atoms and 4 lanes per atom 0.416 -> 0.362 ms:
+// the sums' shuffles and shared accumulators had been 19 % of the data pipe's work, the third
+// table function of one-type pairs another 20 %.
 //
 // STAGED: the block first copies the staged quintic tables (T.stf, T.st_bytes, about 180 KB
 // for a two-element alloy) into dynamic shared memory and reads every staged interval from
@@ -495,25 +497,24 @@ template <bool OBS, bool KICK, int TPA, int IP, bool STAGED, typename IX,
 __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
-    constexpr int kG = NB / TPA;
-    __shared__ double s_acc[F_NSUM * kG];
     extern __shared__ float4 s_stage[];
-    int const tid = threadIdx.x, grp = tid / TPA;
-    for (int k = tid; k < F_NSUM * kG; k += NB)
-        s_acc[k] = 0.;
+    int const tid = threadIdx.x;
     if (STAGED) {
         const float4 *src = reinterpret_cast<const float4 *>(T.stf);
         int const n16 = T.st_bytes / 16;
         for (int k = tid; k < n16; k += NB)
             s_stage[k] = __ldg(src + k);
+        __syncthreads();
     }
-    __syncthreads();
     const float *stab = reinterpret_cast<const float *>(s_stage);
     int const r = A.fblk_rep[blockIdx.x];
     Replica const *R = A.rep + r;
     int const lb = blockIdx.x - R->fblk_begin, nb = R->fblk_n;
     int const apb = NB / TPA, sub = tid % TPA;
     int const n_slots = R->n_blocks * kBlock;
+    constexpr int kPair = OBS ? F_F2 - F_SIGMA : F_CB - F_SIGMA, kP2 = slots_pow2(kPair);
+    constexpr int kKick = F_NSUM - F_F2, kK2 = slots_pow2(kKick);
+    double acc_p = 0., acc_k = 0.; // the block sums of this lane's slots
     RowIn in;
     box_f(R, in.L, in.iL);
     for (int a0 = lb * apb; a0 < n_slots; a0 += nb * apb) {
@@ -521,10 +522,7 @@ __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
         int const i = R->atom_begin + a;
         bool const valid = a < R->n_atoms;
         double fx = 0., fy = 0., fz = 0., epot = 0.;
-        double sums[F_F2]; // this atom's pair sums (virial, Born stress, tensor, Laplacian)
-#pragma unroll
-        for (int k = 0; k < F_F2; ++k)
-            sums[k] = 0.;
+        double v[kP2] = {}; // this lane's pair sums: Born stress, tensor, Laplacian
         in.ti = 0;
         if (valid) {
             in.pi = A.posf[i];
@@ -550,33 +548,26 @@ __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
             }
             if (warn_rmin)
                 status_or(A.rep + r, MDELAST_WARN_RMIN);
-            sums[F_VIRIAL] = (ps.sig_d[0] + ps.sig_d[1]) + ps.sig_d[2];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                sums[F_SIGMA + k] = ps.sig_d[k];
-                sums[F_SIGMA + 3 + k] = static_cast<double>(ps.sig_o[k]);
+                v[k] = ps.sig_d[k];
+                v[3 + k] = static_cast<double>(ps.sig_o[k]);
             }
             if (OBS) {
 #pragma unroll
                 for (int k = 0; k < 15; ++k)
-                    sums[F_CB + k] = static_cast<double>(ps.cb[k]);
-                sums[F_LAP] = static_cast<double>(ps.lap);
+                    v[(F_CB - F_SIGMA + k) % kP2] = static_cast<double>(ps.cb[k]);
+                v[(F_LAP - F_SIGMA) % kP2] = static_cast<double>(ps.lap);
             }
         }
+        acc_p += warp_slots<kP2, 1>(v);
         fx = group_sum<TPA>(fx);
         fy = group_sum<TPA>(fy);
         fz = group_sum<TPA>(fz);
         epot = group_sum<TPA>(epot);
-        constexpr int kPair = OBS ? F_F2 : F_CB; // the pair sums this step forms
-#pragma unroll
-        for (int k = 0; k < kPair; ++k)
-            sums[k] = group_sum<TPA>(sums[k]);
-        if (sub == 0) {
-#pragma unroll
-            for (int k = 0; k < kPair; ++k)
-                s_acc[k * kG + grp] += sums[k];
-        }
-        if (valid && sub == 0) {
+        double vx = 0., vy = 0., vz = 0., m = 0.;
+        double w[kK2] = {}; // the atom's terms of the sums over atoms, equal in its lanes
+        if (valid) { // every lane of the atom, stored by the first
             double const kf = kEv / kAng; // eV/A -> dyn
             fx *= kf;
             fy *= kf;
@@ -585,52 +576,72 @@ __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
             if (T.has_eam)
                 epot += A.Fe[i];
             size_t const np = A.n_pad;
-            A.frc[i] = fx;
-            A.frc[np + i] = fy;
-            A.frc[np + i + np] = fz;
-            A.epot[i] = epot;
-            double const m = T.mass[in.ti];
-            double vx = A.vel[i], vy = A.vel[np + i], vz = A.vel[2 * np + i];
+            m = T.mass[in.ti];
+            vx = A.vel[i];
+            vy = A.vel[np + i];
+            vz = A.vel[2 * np + i];
             if (KICK) {
                 double const e = R->e_kick, cdt = R->cdt_kick;
                 vx = vx * e + cdt * fx / m;
                 vy = vy * e + cdt * fy / m;
                 vz = vz * e + cdt * fz / m;
+            }
+        }
+        __syncwarp(); // the atom's lanes have read its velocity
+        if (valid && sub == 0) {
+            size_t const np = A.n_pad;
+            A.frc[i] = fx;
+            A.frc[np + i] = fy;
+            A.frc[np + i + np] = fz;
+            A.epot[i] = epot;
+            if (KICK) {
                 A.vel[i] = vx;
                 A.vel[np + i] = vy;
                 A.vel[2 * np + i] = vz;
             }
-            double *acc = s_acc + grp;
-            acc[F_F2 * kG] += fx * fx + fy * fy + fz * fz;
-            acc[F_EKIN * kG] += 0.5 * m * (vx * vx + vy * vy + vz * vz);
-            acc[(F_MVV + 0) * kG] += m * vx * vx;
-            acc[(F_MVV + 1) * kG] += m * vy * vy;
-            acc[(F_MVV + 2) * kG] += m * vz * vz;
-            acc[(F_MVV + 3) * kG] += m * vy * vz;
-            acc[(F_MVV + 4) * kG] += m * vx * vz;
-            acc[(F_MVV + 5) * kG] += m * vx * vy;
-            acc[(F_MV + 0) * kG] += vx * m;
-            acc[(F_MV + 1) * kG] += vy * m;
-            acc[(F_MV + 2) * kG] += vz * m;
-            acc[F_EPOT * kG] += epot;
         }
+        if (valid) {
+            w[F_F2 - F_F2] = fx * fx + fy * fy + fz * fz;
+            w[F_EKIN - F_F2] = 0.5 * m * (vx * vx + vy * vy + vz * vz);
+            w[F_MVV + 0 - F_F2] = m * vx * vx;
+            w[F_MVV + 1 - F_F2] = m * vy * vy;
+            w[F_MVV + 2 - F_F2] = m * vz * vz;
+            w[F_MVV + 3 - F_F2] = m * vy * vz;
+            w[F_MVV + 4 - F_F2] = m * vx * vz;
+            w[F_MVV + 5 - F_F2] = m * vx * vy;
+            w[F_MV + 0 - F_F2] = vx * m;
+            w[F_MV + 1 - F_F2] = vy * m;
+            w[F_MV + 2 - F_F2] = vz * m;
+            w[F_EPOT - F_F2] = epot;
+        }
+        acc_k += warp_slots<kK2, TPA>(w);
     }
-    // the groups' slots into the block sums; pair sums from eV (and eV/A^2 for the
-    // Laplacian) to cgs
+    // the warps' slots into the block sums; pair sums from eV (and eV/A^2 for the
+    // Laplacian) to cgs, the virial as the trace of the Born stress
+    __shared__ double s_acc[NB / 32][F_NSUM];
+    int const lane = tid & 31, warp = tid >> 5;
+    if (lane < kP2 && lane_slot<kP2>(lane) < kPair)
+        s_acc[warp][F_SIGMA + lane_slot<kP2>(lane)] = acc_p;
+    if (lane < kK2 && lane_slot<kK2>(lane) < kKick)
+        s_acc[warp][F_F2 + lane_slot<kK2>(lane)] = acc_k;
     __syncthreads();
-    double acc[F_NSUM];
+    auto block_sum = [&](int k) {
+        double s = 0.;
 #pragma unroll
-    for (int k = 0; k < F_NSUM; ++k)
-        acc[k] = tid < kG ? s_acc[k * kG + tid] : 0.;
-    acc[F_VIRIAL] *= kEv;
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-        acc[F_SIGMA + k] *= kEv;
-#pragma unroll
-    for (int k = 0; k < 15; ++k)
-        acc[F_CB + k] *= kEv;
-    acc[F_LAP] *= kEv / (kAng * kAng);
-    block_sum_store<F_NSUM, NB>(acc, A.pf + static_cast<size_t>(blockIdx.x) * F_NSUM);
+        for (int q = 0; q < NB / 32; ++q)
+            s += s_acc[q][k];
+        return s;
+    };
+    for (int k = tid; k < F_NSUM; k += NB) {
+        double s = 0.;
+        if (k == F_VIRIAL)
+            s = ((block_sum(F_SIGMA) + block_sum(F_SIGMA + 1)) + block_sum(F_SIGMA + 2)) * kEv;
+        else if (k >= F_F2)
+            s = block_sum(k);
+        else if (k - F_SIGMA < kPair)
+            s = block_sum(k) * (k == F_LAP ? kEv / (kAng * kAng) : kEv);
+        A.pf[static_cast<size_t>(blockIdx.x) * F_NSUM + k] = s;
+    }
 }
 
 namespace {
@@ -668,8 +679,7 @@ void force_mx_tpa(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesV
     else
         force_mx_tpa_ix<OBS, KICK, IP, int>(tpa, grid, s, A, T);
 }
-// the staged kernels: lanes per atom 4, 8 or 16 (one lane per atom would need 143 KB of
-// accumulators beside the tables)
+// the staged kernels: lanes per atom 4, 8 or 16
 template <bool OBS, bool KICK, typename IX>
 void force_mx_staged_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                         TablesView const &T) {

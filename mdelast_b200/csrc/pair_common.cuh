@@ -13,6 +13,14 @@ __device__ __forceinline__ void status_or(Replica *rep, unsigned bits) {
 __device__ __forceinline__ bool halted(AtomsView const &A) { return *A.halt != 0; }
 __device__ __forceinline__ void set_halt(AtomsView const &A) { *A.halt = 1; }
 
+// 32 bytes (32-byte aligned) in one 256-bit load through the read-only path.
+__device__ __forceinline__ void ld256(const float *p, float (&v)[8]) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+          "=f"(v[7])
+        : "l"(p));
+}
+
 // minimum image of pi - pj in a box of edges L (positions wrapped into [-L/2, L/2))
 __device__ __forceinline__ float min_image_f(float4 pi, float4 pj, float3 L, float3 iL,
                                              float &dx, float &dy, float &dz) {
@@ -31,38 +39,53 @@ __device__ __forceinline__ void box_f(Replica const *R, float3 &L, float3 &iL) {
     iL = make_float3(1.f / L.x, 1.f / L.y, 1.f / L.z);
 }
 
-// Sum v over the warp (fixed order) and add it to this warp's shared accumulator.
-__device__ __forceinline__ void warp_accumulate(double v, double *slot) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0)
-        *slot += v;
+// The warp's totals of N per-lane values, one total per lane: at each butterfly level a
+// lane keeps half of its values and hands the other half to its partner lane, so N values
+// take 31 exchanges instead of the 5 N of N separate warp sums, and the totals end spread over the
+// lanes, where a register per lane accumulates them from atom group to atom group. SAME:
+// lanes that differ only in the bits below SAME hold equal values that count once (the lanes
+// of an atom, after group_sum); those levels only select. Fixed order, so deterministic.
+// v holds slots_pow2(N) values, zeros past N; lane l < slots_pow2(N) ends with the total of slot
+// lane_slot<slots_pow2(N)>(l).
+constexpr __host__ __device__ int slots_pow2(int n) {
+    int p = 1;
+    while (p < n)
+        p <<= 1;
+    return p;
 }
-
-// Block-wide sum of NS per-thread values into out[0..NS), warp shuffles then shared
-// memory; deterministic for a fixed block size (NB threads).
-template <int NS, int NB = kBlock>
-__device__ __forceinline__ void block_sum_store(double (&v)[NS], double *out) {
-    __shared__ double sm[NB / 32][NS];
-    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <int CUR, int O, int SAME, int P2>
+__device__ __forceinline__ void warp_slots_level(double (&v)[P2]) {
+    int const lane = threadIdx.x & 31;
+    if constexpr (CUR > 1) {
+        constexpr int kHalf = CUR / 2;
+        bool const up = (lane & O) != 0;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        double x = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0)
-            sm[warp][k] = x;
+        for (int k = 0; k < kHalf; ++k) {
+            double const keep = up ? v[kHalf + k] : v[k];
+            if constexpr (O < SAME) {
+                v[k] = keep;
+            } else {
+                double const give = up ? v[k] : v[kHalf + k];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+            }
+        }
+    } else if constexpr (O >= SAME) {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k < NS; k += blockDim.x) {
-        double s = 0.;
+    if constexpr (O < 16)
+        warp_slots_level<(CUR > 1 ? CUR / 2 : 1), 2 * O, SAME>(v);
+}
+template <int P2, int SAME> __device__ __forceinline__ double warp_slots(double (&v)[P2]) {
+    static_assert(P2 <= 32, "one slot per lane");
+    warp_slots_level<P2, 1, SAME>(v);
+    return v[0];
+}
+template <int P2> __device__ __forceinline__ int lane_slot(int lane) {
+    int s = 0;
 #pragma unroll
-        for (int w = 0; w < NB / 32; ++w)
-            s += sm[w][k];
-        out[k] = s;
-    }
+    for (int o = 1, half = P2 / 2; half > 0; o <<= 1, half >>= 1)
+        s += (lane & o) ? half : 0;
+    return s;
 }
 
 // TPA lanes (a power of two dividing 32) share one atom: lane `sub` takes the atom's list
