@@ -111,19 +111,29 @@ double nint_host(double x) { // md_driver.hpp:48-50
     return static_cast<double>(x < 0. ? static_cast<int>(x - 0.5) : static_cast<int>(x + 0.5));
 }
 
-// Lanes per atom for the pair passes: the fewest that give about 150k threads (enough to
-// cover 148 SMs with the warps the register budget allows), at most 16. MDELAST_TPA
-// overrides it.
-int default_tpa(int n_atoms) {
+// Lanes per atom of the pair passes until a tuner or set_launch chooses otherwise: 16 lanes
+// while a pass is a wave of latency-bound warps (a few thousand atoms), then 8, and in mixed
+// precision 4 once those fill the SMs too (FP64 rows are long enough in instructions for 8 at
+// any size). One lane per atom leaves every load of a row uncoalesced. Density + force pass in
+// ms, by lanes per atom (cells of the two-element alloy):
+//   atoms     FP64 4 / 8 / 16             mixed 1 / 4 / 8 / 16
+//   5,324     0.080 / 0.053 / 0.051       0.131 / 0.051 / 0.038 / 0.040
+//   8,788     0.082 / 0.072 / 0.072       0.135 / 0.053 / 0.041 / 0.045
+//   13,500    0.094 / 0.082 / 0.090       0.139 / 0.058 / 0.058 / 0.061
+//   19,652    0.132 / 0.118 / 0.123       0.136 / 0.079 / 0.078 / 0.083
+//   32,000    0.195 / 0.175 / 0.190       0.139 / 0.098 / 0.102 / 0.116
+//   216,000   1.037 / 1.033 / 1.119       0.668 / 0.532 / 0.547 / 0.655
+//   640,000   3.03 / 3.03 / 3.27          1.83 / 1.48 / 1.58 / 1.93
+// MDELAST_TPA overrides it.
+int default_tpa(long n_atoms, bool mixed) {
     if (char const *e = std::getenv("MDELAST_TPA")) {
         int const v = std::atoi(e);
         if (valid_tpa(v))
             return v;
     }
-    for (int t : {1, 4, 8})
-        if (static_cast<long>(n_atoms) * t >= 150000)
-            return t;
-    return 16;
+    if (n_atoms < (mixed ? 5000 : 8000))
+        return 16;
+    return mixed && n_atoms >= 28000 ? 4 : 8;
 }
 
 // Deal the blocks of a pair pass out to the replicas in proportion to their atom counts:
@@ -1450,7 +1460,7 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         set_chain(x.bth, c.baro_thermo_T, c.baro_nchain, c.baro_q, c.baro_p_eta, c.baro_Nf);
         reps.push_back(&x);
     }
-    d->tpa_d = d->tpa_f = default_tpa(static_cast<int>(std::min<long>(n_total, 1L << 30)));
+    d->tpa_d = d->tpa_f = default_tpa(n_total, c0.precision == MDELAST_PRECISION_MIXED);
     std::vector<int> dmap, fmap;
     d->grid_d = deal_blocks(reps, d->tpa_d, true, dmap);
     d->grid_f = deal_blocks(reps, d->tpa_f, false, fmap);
