@@ -27,7 +27,7 @@ constexpr double kBoltz = 1.38064852e-16; // units.hpp:7
 // by Estrin's scheme, and exp(-x) = 1 - x op(x) with one FMA. For |x| <= 2 the first omitted
 // term, x^24/25!, is below 3e-18 relative; measured against long-double references over
 // [-2, 2], op is within 4 ulp and exp(-x) within 22 ulp (at x = 2, where 1 - x op = 0.135
-// loses three bits). It has no branch. Thermostat arguments are x = dt p_eta/Q: ~dt/tau
+// loses three bits). Thermostat arguments are x = dt p_eta/Q: ~dt/tau
 // at equilibrium (0.02 for tau = 50 fs, dt = 2 fs), but in the first few hundred steps from
 // a lattice start the upper links of a 13,500-atom cell's chain reach 1.24 (half of the
 // arguments above 1/16, 6 % above 1/2).
@@ -40,7 +40,15 @@ __device__ __forceinline__ void expx_exact(double x, double &expx, double &op) {
                         : 1.0 + x * (c1 + x * (c2 + x * (c3 + x * (c4 + x * c5))));
 }
 
-constexpr double kSeriesMax = 2.0;
+// In a chain sweep only op is needed: p e + hG op = p + op (hG - p x). Three forms, chosen
+// per half step: SHORT, the series to degree 13 for |x| <= 1/4 (first omitted term x^14/15!
+// below 3e-21), one level less of dependent operations; LONG, to degree 23 for |x| <= 2; EXACT,
+// LONG with the exact form per argument beyond it. A half step notes an argument beyond its
+// range and is then redone from its start in the next form (the chain in memory is written
+// only by a half step that completes). A branch per exponential, even one never taken, doubled
+// the time of a 10-link half step.
+constexpr double kShortMax = 0.25, kSeriesMax = 2.0;
+enum SeriesForm : int { SERIES_SHORT = 0, SERIES_LONG = 1, SERIES_EXACT = 2 };
 
 __device__ __forceinline__ void expx_series(double x, double &expx, double &op) {
     double const y = -x, y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
@@ -61,6 +69,17 @@ __device__ __forceinline__ void expx_series(double x, double &expx, double &op) 
     expx = fma(-x, op, 1.0);
 }
 
+__device__ __forceinline__ double op_short(double x) {
+    double const y = -x, y2 = y * y, y4 = y2 * y2, y8 = y4 * y4;
+    double const b0 = fma(y, 1.0 / 2.0, 1.0), b1 = fma(y, 1.0 / 24.0, 1.0 / 6.0),
+                 b2 = fma(y, 1.0 / 720.0, 1.0 / 120.0), b3 = fma(y, 1.0 / 40320.0, 1.0 / 5040.0),
+                 b4 = fma(y, 1.0 / 3628800.0, 1.0 / 362880.0),
+                 b5 = fma(y, 1.0 / 479001600.0, 1.0 / 39916800.0),
+                 b6 = fma(y, 1.0 / 87178291200.0, 1.0 / 6227020800.0);
+    double const t0 = fma(y2, b1, b0), t1 = fma(y2, b3, b2), t2 = fma(y2, b5, b4);
+    return fma(y8, fma(y4, b6, t2), fma(y4, t1, t0));
+}
+
 // The series outside its range falls back to the exact form.
 __device__ __forceinline__ void expx_operator(double x, double &expx, double &op) {
     expx_series(x, expx, op);
@@ -68,18 +87,28 @@ __device__ __forceinline__ void expx_operator(double x, double &expx, double &op
         expx_exact(x, expx, op);
 }
 
-// In a chain sweep: EXACT = false takes the series alone and only notes an argument beyond
-// its range in `large`; a half step that saw one is redone from its start with EXACT = true,
-// which falls back to the exact form per exponential. A branch per exponential, even one
-// never taken, doubled the time of a 10-link half step (27,600 against 13,500 cycles).
-template <bool EXACT>
-__device__ __forceinline__ void expx_sweep(double x, double &expx, double &op, bool &large) {
-    if (EXACT) {
-        expx_operator(x, expx, op);
-    } else {
-        expx_series(x, expx, op);
+// op(x) and, where the sweep uses it (EXACT), e = exp(-x) in the half step's form; `large`
+// notes an argument beyond its range
+template <int FORM>
+__device__ __forceinline__ double op_sweep(double x, double &e, bool &large) {
+    double op;
+    if (FORM == SERIES_SHORT) {
+        large |= fabs(x) > kShortMax;
+        op = op_short(x);
+    } else if (FORM == SERIES_LONG) {
         large |= fabs(x) > kSeriesMax;
+        expx_series(x, e, op);
+    } else {
+        expx_operator(x, e, op);
     }
+    return op;
+}
+
+// p e^-x + hG op(x); EXACT keeps the product with e, which the other form's 1 - x op loses
+// to cancellation at large x
+template <int FORM>
+__device__ __forceinline__ double chain_link(double p, double x, double op, double e, double hG) {
+    return FORM == SERIES_EXACT ? fma(p, e, hG * op) : fma(op, fma(-p, x, hG), p);
 }
 
 __device__ __forceinline__ double volume(const double h[3]) { return h[0] * (h[1] * h[2]); }
@@ -111,58 +140,63 @@ template <int NC> __device__ __forceinline__ void chain_store(ChainR<NC> const &
     }
 }
 
-// thermostat.cpp:40-66 (Yu et al., Chem. Phys. 370 (2010) 294, eq. 8; Allen-Tildesley
-// eqs. 3.73-3.74a): one sweep of the chain. Inward (top link first) each link needs the
-// updated link above it, so its exponential is on the critical path; outward every
-// exponential uses the not-yet-updated link above and all are formed up front.
-template <int NC, bool EXACT>
-__device__ __forceinline__ void U4_in(ChainR<NC> &c, double dt, double ec, bool &large) {
-#pragma unroll
-    for (int j = NC - 1; j >= 0; --j) {
-        double G;
-        if (j != 0)
-            G = c.p[j - 1] * c.p[j - 1] * c.iq[j - 1] - c.kT;
-        else
-            G = 2. * ec - c.Nf * c.kT;
-        if (j == NC - 1) {
-            c.p[j] += dt * G;
-        } else {
-            double e, op;
-            expx_sweep<EXACT>(dt * c.p[j + 1] * c.iq[j + 1], e, op, large);
-            c.p[j] = c.p[j] * e + dt * G * op;
-        }
-    }
-}
-
-template <int NC, bool EXACT>
-__device__ __forceinline__ void U4_out(ChainR<NC> &c, double dt, double ec, bool &large) {
-    double e[NC], op[NC];
-#pragma unroll
-    for (int j = 0; j < NC - 1; ++j)
-        expx_sweep<EXACT>(dt * c.p[j + 1] * c.iq[j + 1], e[j], op[j], large);
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-        double G;
-        if (j != 0)
-            G = c.p[j - 1] * c.p[j - 1] * c.iq[j - 1] - c.kT;
-        else
-            G = 2. * ec - c.Nf * c.kT;
-        if (j == NC - 1)
-            c.p[j] += dt * G;
-        else
-            c.p[j] = c.p[j] * e[j] + dt * G * op[j];
-    }
-}
-
-// thermostat.hpp:24-35: factor exp(-dt p_eta[0]/Q[0]) for the coupled momenta; advances
-// the chain positions
-template <int NC, bool EXACT> __device__ __forceinline__ double U3(ChainR<NC> &c, double dt,
-                                                                  bool &large) {
-    double s, op;
-    expx_sweep<EXACT>(dt * c.p[0] * c.iq[0], s, op, large);
+// One Suzuki-Yoshida sub-step of a chain: inward sweep, U3, outward sweep (thermostat.cpp:
+// 40-66, thermostat.hpp:24-35; Yu et al., Chem. Phys. 370 (2010) 294, eq. 8; Allen-Tildesley eqs.
+// 3.73-3.74a). Each link is p_j <- p_j e^-x + hG op(x) with x = h p_{j+1} / Q_{j+1}. ec0 is the
+// energy coupled to the first link before U3, after(s) the one after it, s the U3 factor.
+//
+// One thread works down a chain of dependent FP64 operations, about 16 cycles each, so the
+// sub-step's time is its number. Inward, a link waits for the updated link above it: x, the
+// series, and one FMA (p + op (hG - p x), its inner part formed beside the series). Outward,
+// a link's exponential has the very argument it had inward (the link above is not yet updated
+// again), so op is kept from there, and p_j <- a_j + b_j p_{j-1}^2 with a_j and b_j formed
+// beforehand takes two operations. A 10-link half step (7 sub-steps): 13,900 -> 9,100 cycles against a
+// series per link and direction with the products in the reference's order.
+template <int NC, int FORM, typename After>
+__device__ __forceinline__ double chain_substep(ChainR<NC> &c, double dtw, double ec0,
+                                                After &&after, bool &large) {
+    double const h = 0.5 * dtw, hkT = h * c.kT;
+    double dq[NC], x[NC], op[NC], e[NC]; // x[j], op[j], e[j]: of link j, j < NC - 1
 #pragma unroll
     for (int j = 0; j < NC; ++j)
-        c.eta[j] += dt * c.p[j] * c.iq[j];
+        dq[j] = h * c.iq[j];
+#pragma unroll
+    for (int j = NC - 1; j >= 0; --j) {
+        double const hG = j != 0 ? fma(c.p[j - 1], c.p[j - 1] * dq[j - 1], -hkT)
+                                 : h * (2. * ec0 - c.Nf * c.kT);
+        if (j == NC - 1) {
+            c.p[j] += hG;
+        } else {
+            x[j] = c.p[j + 1] * dq[j + 1];
+            op[j] = op_sweep<FORM>(x[j], e[j], large);
+            c.p[j] = chain_link<FORM>(c.p[j], x[j], op[j], e[j], hG);
+        }
+    }
+    double const x3 = 2. * (c.p[0] * dq[0]);
+    double e3 = 0.;
+    double const op3 = op_sweep<FORM>(x3, e3, large);
+    double const s = FORM == SERIES_EXACT ? e3 : fma(-x3, op3, 1.);
+#pragma unroll
+    for (int j = 0; j < NC; ++j)
+        c.eta[j] = fma(2. * dq[j], c.p[j], c.eta[j]);
+    double const ec1 = after(s);
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+        if (j == 0 && NC > 1) {
+            double const hG = h * (2. * ec1 - c.Nf * c.kT);
+            c.p[0] = chain_link<FORM>(c.p[0], x[0], op[0], e[0], hG);
+        } else if (j == 0) {
+            c.p[0] += h * (2. * ec1 - c.Nf * c.kT);
+        } else if (j < NC - 1 && FORM == SERIES_EXACT) {
+            c.p[j] = chain_link<FORM>(c.p[j], x[j], op[j], e[j],
+                                      fma(c.p[j - 1], c.p[j - 1] * dq[j - 1], -hkT));
+        } else if (j < NC - 1) {
+            double const a = fma(-op[j], fma(c.p[j], x[j], hkT), c.p[j]);
+            c.p[j] = fma(op[j] * dq[j - 1], c.p[j - 1] * c.p[j - 1], a);
+        } else {
+            c.p[j] = fma(dq[j - 1], c.p[j - 1] * c.p[j - 1], c.p[j] - hkT);
+        }
+    }
     return s;
 }
 
@@ -173,48 +207,38 @@ __device__ double chain_etot(Chain const &c) {
         e += c.eta[j];
     e *= kBoltz * c.T;
     for (int j = 0; j < c.n; ++j)
-        e += 0.5 * (c.p_eta[j] * c.p_eta[j]) / c.q[j];
+        e += 0.5 * (c.p_eta[j] * c.p_eta[j]) * c.inv_q[j];
     return e;
 }
 
-// One Suzuki-Yoshida sub-step of the particle thermostat (md_driver.cpp:539-549 with the U4
-// coupling of md_driver.cpp:512-531): returns the U3 factor; the kinetic energy follows it
-// as ekin * s^2.
-template <int NC, bool EXACT>
-__device__ __forceinline__ double thermo_substep(ChainR<NC> &c, double dtw, double &ekin,
-                                                 bool conf, bool average, double econf,
-                                                 bool &large) {
-    U4_in<NC, EXACT>(c, 0.5 * dtw, !conf ? ekin : (average ? 0.5 * (ekin + econf) : econf),
-                     large);
-    double const s = U3<NC, EXACT>(c, dtw, large);
-    ekin = ekin * s * s;
-    U4_out<NC, EXACT>(c, 0.5 * dtw, !conf ? ekin : (average ? 0.5 * (ekin + econf) : econf),
-                      large);
-    return s;
-}
-
-// The particle thermostat's half step (md_driver.cpp:539-549). The velocities are not
-// touched: the product of the seven U3 factors is returned and applied by the next atom
-// kernel. The chain in memory is written only by a half step that completes.
-template <int NC, bool EXACT>
+// The particle thermostat's half step (md_driver.cpp:539-549 with the U4 coupling of
+// md_driver.cpp:512-531). The velocities are not touched: the product of the seven U3 factors is
+// returned and applied by the next atom kernel; the kinetic energy follows it as ekin * s^2.
+template <int NC, int FORM>
 __device__ __forceinline__ double thermo_half(Chain &gc, double dt, double &ekin, bool conf,
                                               bool average, double econf, bool &large) {
     ChainR<NC> c;
     chain_load<NC>(gc, c);
+    auto coupled = [&](double e) { return !conf ? e : (average ? 0.5 * (e + econf) : econf); };
     double S = 1.;
 #pragma unroll 1
     for (int k = 0; k < 7; ++k)
-        S *= thermo_substep<NC, EXACT>(c, c_wsy7[k] * dt, ekin, conf, average, econf, large);
-    if (EXACT || !large)
+        S *= chain_substep<NC, FORM>(
+            c, c_wsy7[k] * dt, coupled(ekin),
+            [&](double s) {
+                ekin = ekin * s * s;
+                return coupled(ekin);
+            },
+            large);
+    if (FORM == SERIES_EXACT || !large)
         chain_store<NC>(c, gc);
     return S;
 }
 
-template <int NC>
-__device__ __noinline__ double thermo_half_exact(Chain &gc, double dt, double &ekin, bool conf,
-                                                 bool average, double econf) {
-    bool large = false;
-    return thermo_half<NC, true>(gc, dt, ekin, conf, average, econf, large);
+template <int NC, int FORM>
+__device__ __noinline__ double thermo_half_slow(Chain &gc, double dt, double &ekin, bool conf,
+                                                bool average, double econf, bool &large) {
+    return thermo_half<NC, FORM>(gc, dt, ekin, conf, average, econf, large);
 }
 
 template <int NC>
@@ -222,49 +246,57 @@ __device__ double nhc_thermo_n(Chain &gc, double dt, double &ekin, bool conf, bo
                                double econf) {
     double e = ekin;
     bool large = false;
-    double S = thermo_half<NC, false>(gc, dt, e, conf, average, econf, large);
+    double S = thermo_half<NC, SERIES_SHORT>(gc, dt, e, conf, average, econf, large);
     if (large) {
         e = ekin;
-        S = thermo_half_exact<NC>(gc, dt, e, conf, average, econf);
+        large = false;
+        S = thermo_half_slow<NC, SERIES_LONG>(gc, dt, e, conf, average, econf, large);
+    }
+    if (large) {
+        e = ekin;
+        S = thermo_half_slow<NC, SERIES_EXACT>(gc, dt, e, conf, average, econf, large);
     }
     ekin = e;
     return S;
 }
 
-// One sub-step of the barostat's chain (md_driver.cpp:551-561, 533-537, 507-510) acting on
-// the barostat momentum p.
-template <int NC, bool EXACT>
-__device__ __forceinline__ double baro_substep(ChainR<NC> &c, double dtw, double p, double iw,
-                                               bool &large) {
-    U4_in<NC, EXACT>(c, 0.5 * dtw, 0.5 * (p * p) * iw, large);
-    p *= U3<NC, EXACT>(c, dtw, large);
-    U4_out<NC, EXACT>(c, 0.5 * dtw, 0.5 * (p * p) * iw, large);
-    return p;
-}
-
-template <int NC, bool EXACT>
+// The barostat chain's half step (md_driver.cpp:551-561, 533-537, 507-510) acting on the
+// barostat momentum p.
+template <int NC, int FORM>
 __device__ __forceinline__ double baro_half(Chain &gc, double dt, double p, double iw,
                                             bool &large) {
     ChainR<NC> c;
     chain_load<NC>(gc, c);
 #pragma unroll 1
     for (int k = 0; k < 7; ++k)
-        p = baro_substep<NC, EXACT>(c, c_wsy7[k] * dt, p, iw, large);
-    if (EXACT || !large)
+        chain_substep<NC, FORM>(
+            c, c_wsy7[k] * dt, 0.5 * (p * p) * iw,
+            [&](double s) {
+                p *= s;
+                return 0.5 * (p * p) * iw;
+            },
+            large);
+    if (FORM == SERIES_EXACT || !large)
         chain_store<NC>(c, gc);
     return p;
 }
 
-template <int NC>
-__device__ __noinline__ double baro_half_exact(Chain &gc, double dt, double p, double iw) {
-    bool large = false;
-    return baro_half<NC, true>(gc, dt, p, iw, large);
+template <int NC, int FORM>
+__device__ __noinline__ double baro_half_slow(Chain &gc, double dt, double p, double iw,
+                                              bool &large) {
+    return baro_half<NC, FORM>(gc, dt, p, iw, large);
 }
 
 template <int NC> __device__ double nhc_baro_n(Chain &gc, double dt, double p, double iw) {
     bool large = false;
-    double const q = baro_half<NC, false>(gc, dt, p, iw, large);
-    return large ? baro_half_exact<NC>(gc, dt, p, iw) : q;
+    double q = baro_half<NC, SERIES_SHORT>(gc, dt, p, iw, large);
+    if (large) {
+        large = false;
+        q = baro_half_slow<NC, SERIES_LONG>(gc, dt, p, iw, large);
+    }
+    if (large)
+        q = baro_half_slow<NC, SERIES_EXACT>(gc, dt, p, iw, large);
+    return q;
 }
 
 #define MDELAST_CHAIN_CASES(F)                                                                \
@@ -288,9 +320,8 @@ __device__ double nhc_thermo(Replica *R, Chain &gc, double dt, double &ekin) {
     }
 }
 
-__device__ void nhc_baro(Replica *R, Chain &gc, double dt) {
+__device__ double nhc_baro(Replica *R, Chain &gc, double dt, double p) {
     double const iw = 1. / R->baro_w;
-    double p = R->p_eps;
     switch (gc.n) {
 #define F(N)                                                                                  \
     case N:                                                                                   \
@@ -301,31 +332,21 @@ __device__ void nhc_baro(Replica *R, Chain &gc, double dt) {
     default:
         break;
     }
-    R->p_eps = p;
+    return p;
 }
 
-// md_driver.cpp:454-459 (Yu et al. eq. 31)
-__device__ void U2p(Replica *R, double dt, double ekin, double virial) {
-    double const pv = R->baro_P * volume(R->h);
-    R->p_eps += (2. * R->alpha * ekin + 3. * virial - 3. * pv) * dt;
+// md_driver.cpp:454-459 (Yu et al. eq. 31): the barostat momentum after U2p
+__device__ __forceinline__ double U2p(double p_eps, double alpha, double pv, double dt, double ekin,
+                                      double virial) {
+    return p_eps + (2. * alpha * ekin + 3. * virial - 3. * pv) * dt;
 }
 
-__device__ int monomial_index(int iv, int ivp) {
-    constexpr int VA[6] = {0, 1, 2, 1, 0, 0}, VB[6] = {0, 1, 2, 2, 2, 1};
-    // exponents (x, y, z) of the monomials in the order the force kernel accumulates them
-    constexpr int EX[15][3] = {{4, 0, 0}, {0, 4, 0}, {0, 0, 4}, {3, 1, 0}, {3, 0, 1},
-                               {1, 3, 0}, {0, 3, 1}, {1, 0, 3}, {0, 1, 3}, {2, 2, 0},
-                               {2, 0, 2}, {0, 2, 2}, {2, 1, 1}, {1, 2, 1}, {1, 1, 2}};
-    int e[3] = {0, 0, 0};
-    e[VA[iv]]++;
-    e[VB[iv]]++;
-    e[VA[ivp]]++;
-    e[VB[ivp]]++;
-    for (int m = 0; m < 15; ++m)
-        if (EX[m][0] == e[0] && EX[m][1] == e[1] && EX[m][2] == e[2])
-            return m;
-    return 0;
-}
+// Monomial (in the order the force kernel accumulates them: x4 y4 z4 x3y x3z xy3 y3z xz3 yz3
+// x2y2 x2z2 y2z2 x2yz xy2z xyz2) of entry (a, b), a <= b, of the Born tensor in Voigt order
+// (xx, yy, zz, yz, xz, xy); the lower triangle is not read.
+__constant__ signed char c_monomial[36] = {0,  9,  10, 12, 4,  3,  -1, 1,  11, 6,  13, 5,
+                                           -1, -1, 2,  8,  7,  14, -1, -1, -1, 11, 14, 13,
+                                           -1, -1, -1, -1, 10, 12, -1, -1, -1, -1, -1, 9};
 
 // The replica state in shared memory for k_post: one thread works through a long chain of
 // dependent updates of it (the thermodynamics), and reading and writing it in global
@@ -354,59 +375,65 @@ __device__ __forceinline__ void replica_store(Replica const *s, Replica *g) {
 
 // Opening scalar work of integrate() (md_driver.cpp:567-581): barostat and particle NHC
 // half steps, U2p, and the coefficients of the opening kick and of the drift, with the
-// NPT box update of U1 (md_driver.cpp:488-498).
+// NPT box update of U1 (md_driver.cpp:488-498). The two chains run on two warps; the
+// coefficients of the kick (thread 0) and of the drift with the box (thread 32) follow side by
+// side from the same barostat momentum. Everything read from the replica is read before the
+// chains, so that no round trip to memory sits behind them.
 __global__ void k_pre(AtomsView A) {
     if (*A.halt) // a list build ran out of capacity: nothing until the host regrows
         return;
     Replica *R = A.rep + blockIdx.x;
-    __shared__ double s_S, s_ekin;
+    __shared__ double s_ekin, s_p;
+    int const t = threadIdx.x;
     int const ens = R->ensemble;
-    double const dt = R->dt;
-    if (threadIdx.x == 0) {
+    bool const npt = ens == MDELAST_NPT;
+    double const dt = R->dt, virial = R->obs.virial, alpha = R->alpha, w = R->baro_w;
+    double const h[3] = {R->h[0], R->h[1], R->h[2]}, h0[3] = {R->h0[0], R->h0[1], R->h0[2]};
+    double const vscale = R->vscale, vol = volume(h), pv = R->baro_P * vol;
+    double const eps0 = R->eps;
+    double S = 1.;
+    if (t == 0) {
         R->sub_d2 = 0.; // k_kick_drift takes this step's largest displacement
         double ekin = R->obs.ekin_tot;
-        double S = 1.;
-        if (ens == MDELAST_NVT || ens == MDELAST_NPT) {
+        if (ens == MDELAST_NVT || npt)
             S = nhc_thermo(R, R->th, 0.5 * dt, ekin);
-        }
-        s_S = S;
         s_ekin = ekin;
-    } else if (threadIdx.x == 32 && ens == MDELAST_NPT) {
-        nhc_baro(R, R->bth, 0.5 * dt);
+    } else if (t == 32) {
+        double const p = R->p_eps;
+        s_p = npt ? nhc_baro(R, R->bth, 0.5 * dt, p) : p;
     }
     __syncthreads();
-    if (threadIdx.x != 0)
-        return;
     double const ekin = s_ekin;
-    R->obs.ekin_tot = ekin;
-    double e = 1., c = 1.;
-    if (ens == MDELAST_NPT) {
-        U2p(R, 0.5 * dt, ekin, R->obs.virial);
-        double const x = R->alpha * (0.5 * dt) * R->p_eps / R->baro_w;
-        expx_operator(x, e, c);
-    }
-    R->s_kick = R->vscale * s_S;
-    R->vscale = 1.;
-    R->e_kick = e;
-    R->cdt_kick = c * (0.5 * dt);
-    // U1 (md_driver.cpp:464-470, 488-498)
-    double cf = 1.;
-    if (ens == MDELAST_NPT) {
-        double const x = dt * R->p_eps / R->baro_w;
-        R->eps += x;
-        double ee;
-        expx_operator(x, ee, cf);
-    }
-    R->cfdt = cf * dt;
-    for (int a = 0; a < 3; ++a)
-        R->h_pos[a] = R->h[a];
-    if (ens == MDELAST_NPT) {
-        double const expe = exp(R->eps);
-        double const vol_old = volume(R->h);
+    double const p_eps = npt ? U2p(s_p, alpha, pv, 0.5 * dt, ekin, virial) : s_p;
+    if (t == 0) {
+        R->obs.ekin_tot = ekin;
+        double e = 1., c = 1.;
+        if (npt)
+            expx_operator(alpha * (0.5 * dt) * p_eps / w, e, c);
+        R->s_kick = vscale * S;
+        R->vscale = 1.;
+        R->e_kick = e;
+        R->cdt_kick = c * (0.5 * dt);
+    } else if (t == 32) {
+        // U1 (md_driver.cpp:464-470, 488-498)
+        double cf = 1.;
         for (int a = 0; a < 3; ++a)
-            R->h[a] = R->h0[a] * expe;
-        if (fabs(volume(R->h) / vol_old - 1.) > 0.05)
-            atomicOr(&R->obs.status, MDELAST_FATAL_VOLUME);
+            R->h_pos[a] = h[a];
+        if (npt) {
+            double const x = dt * p_eps / w, eps = eps0 + x;
+            double ee, hn[3];
+            expx_operator(x, ee, cf);
+            R->p_eps = p_eps;
+            R->eps = eps;
+            double const expe = exp(eps);
+            for (int a = 0; a < 3; ++a) {
+                hn[a] = h0[a] * expe;
+                R->h[a] = hn[a];
+            }
+            if (fabs(volume(hn) / vol - 1.) > 0.05)
+                atomicOr(&R->obs.status, MDELAST_FATAL_VOLUME);
+        }
+        R->cfdt = cf * dt;
     }
 }
 
@@ -555,8 +582,7 @@ __global__ void k_samples_reset(AtomsView A, int what) {
     }
 }
 
-__device__ void thermodynamics(Replica *R, int mode, int obs, const double *sf, const double *sd,
-                               double S, double ekin, double virial);
+__device__ void thermodynamics(Replica *R, int mode, int obs, double etot_th, double etot_npt);
 
 __global__ void k_post(AtomsView A, int mode, int obs) {
     if (*A.halt) // a list build ran out of capacity: nothing until the host regrows
@@ -564,7 +590,7 @@ __global__ void k_post(AtomsView A, int mode, int obs) {
     __shared__ Replica sR;
     __shared__ double sf[F_NSUM], sd[D_NSUM];
     __shared__ double s_part[4][F_NSUM + D_NSUM];
-    __shared__ double s_S, s_ekin, s_virial;
+    __shared__ double s_S, s_ekin;
     replica_load(A.rep + blockIdx.x, &sR);
     Replica *R = &sR;
     int const t = threadIdx.x;
@@ -598,58 +624,92 @@ __global__ void k_post(AtomsView A, int mode, int obs) {
         }
     }
     __syncthreads();
+    // One thread of each warp takes an independent part: the two chains (warps 0 and 1) are the
+    // long ones, the rest of calculate_forces and of the tail of U2 runs beside them. On one
+    // thread before and after the chains those parts had taken 6,600 of the kernel's 24,600
+    // cycles (13,500 atoms, NVT).
     int const ens = R->ensemble;
+    bool const npt = ens == MDELAST_NPT, nhc = npt || ens == MDELAST_NVT;
     double const dt = R->dt;
     mdelast_observables &o = R->obs;
     // The box does not change in k_post: the volume of the thermodynamics (md_driver.cpp:
     // 648-730), which divides the Born tensor, one entry per thread (zeros below the
     // diagonal, as the reference stores it).
     double const V = volume(R->h);
-    if (obs && t < 36) {
-        int const a = t / 6, b = t % 6;
-        o.born_elasticity_tensor[t] =
-            b < a ? 0. : (sf[F_CB + monomial_index(a, b)] + sd[D_CB + a * (11 - a) / 2 + b]) / V;
+    double const virial = sf[F_VIRIAL] / -3.;
+    double const f2 = sf[F_F2], lap = sf[F_LAP] + sd[D_LAP];
+    // the configurational temperature of this step, which a coupled chain reads (R->obs holds it
+    // after the barrier)
+    double const tci = (f2 != 0. && lap != 0.) ? kBoltz * lap / f2 : 0.;
+    bool const coupled = R->coupling != MDELAST_THERMOSTAT_KINETIC;
+    if (mode == POST_STEP && obs && coupled) {
+        if (t == 0)
+            o.temperature_conf_inverse = tci;
+        __syncthreads();
     }
     if (t == 0) {
-        double const virial = sf[F_VIRIAL] / -3.;
-        s_virial = virial;
+        double ekin = sf[F_EKIN], S = 1.;
+        if (mode == POST_STEP && nhc)
+            S = nhc_thermo(R, R->th, 0.5 * dt, ekin);
+        s_S = S;
+        s_ekin = ekin;
+    } else if (t == 32) {
+        if (mode == POST_STEP && npt) {
+            double const p = U2p(R->p_eps, R->alpha, R->baro_P * V, 0.5 * dt, sf[F_EKIN], virial);
+            R->p_eps = nhc_baro(R, R->bth, 0.5 * dt, p);
+        }
+    } else if (t == 64) {
         o.virial = virial;
         double const vir_trace = -(sf[F_SIGMA] + sf[F_SIGMA + 1] + sf[F_SIGMA + 2]);
         if (fabs(virial / (vir_trace / 3.) - 1.) > 1e-7)
             atomicOr(&o.status, MDELAST_WARN_VIRIAL);
-        if (obs)
-            o.total_laplacian = sf[F_LAP] + sd[D_LAP];
-        double ekin = sf[F_EKIN];
-        if (mode == POST_STEP) {
-            if (obs) {
-                double const f2 = sf[F_F2];
-                o.total_force2 = f2;
-                o.temperature_conf_inverse =
-                    (f2 != 0. && o.total_laplacian != 0.) ? kBoltz * o.total_laplacian / f2 : 0.;
-            }
-            if (ens == MDELAST_NPT)
-                U2p(R, 0.5 * dt, ekin, virial);
+        if (obs) {
+            o.total_laplacian = lap;
+            o.total_force2 = f2;
+            if (!(mode == POST_STEP && coupled))
+                o.temperature_conf_inverse = tci;
         }
-        s_ekin = ekin;
+        o.epot_atom = sf[F_EPOT] / R->n_atoms;
+        o.epot_eam_atom = sd[D_FSUM] / R->n_atoms;
+    } else if (t >= 96 && t < 102) {
+        o.born_stress_tensor[t - 96] = sf[F_SIGMA + t - 96] / V;
+    } else if (t >= 128 && t < 164 && obs) {
+        int const q = t - 128, a = q / 6, b = q % 6;
+        o.born_elasticity_tensor[q] =
+            b < a ? 0. : (sf[F_CB + c_monomial[q]] + sd[D_CB + a * (11 - a) / 2 + b]) / V;
     }
     __syncthreads();
-    if (mode == POST_STEP) {
-        if (t == 0) {
-            double ekin = s_ekin, S = 1.;
-            if (ens == MDELAST_NVT || ens == MDELAST_NPT) {
-                S = nhc_thermo(R, R->th, 0.5 * dt, ekin);
-            }
-            s_S = S;
-            s_ekin = ekin;
-        } else if (t == 32 && ens == MDELAST_NPT) {
-            nhc_baro(R, R->bth, 0.5 * dt);
+    // ... and of the thermodynamics: the chains' energies, the stresses, what follows from the
+    // kinetic energy after the chains
+    __shared__ double s_etot[2];
+    double const S = s_S, ekin = s_ekin;
+    if (t == 0) {
+        R->vscale = S;
+        o.ekin_tot = ekin;
+        o.ekin_atom = ekin / R->n_atoms;
+        o.temperature_kin = 2. * ekin / (kBoltz * R->Nf);
+    } else if (t == 32) {
+        s_etot[1] = npt ? V * R->baro_P + (0.5 * (R->p_eps * R->p_eps) / R->baro_w + chain_etot(R->bth))
+                        : 0.;
+    } else if (t == 64) {
+        s_etot[0] = nhc ? chain_etot(R->th) : 0.;
+    } else if (t == 96) {
+        double mom2 = 0.;
+        for (int a = 0; a < 3; ++a) {
+            o.momentum_tot[a] = S * sf[F_MV + a];
+            mom2 += o.momentum_tot[a] * o.momentum_tot[a];
         }
-    } else if (t == 0) {
-        s_S = 1.;
+        if (mom2 / (2. * R->mass0 * ekin) > 1e-14)
+            atomicOr(&o.status, MDELAST_FATAL_MOMENTUM);
+    } else if (t >= 128 && t < 134) {
+        int const k = t - 128;
+        o.stress_tensor[k] = (-sf[F_SIGMA + k] + S * S * sf[F_MVV + k]) / V;
+    } else if (t == 160) {
+        o.pressure = (ekin * 2. / 3. + virial) / V;
     }
     __syncthreads();
     if (t == 0)
-        thermodynamics(R, mode, obs, sf, sd, s_S, s_ekin, s_virial);
+        thermodynamics(R, mode, obs, s_etot[0], s_etot[1]);
     if (mode == POST_STEP && obs) {
         __syncthreads();
         record_sample(A, static_cast<int>(blockIdx.x), R, V);
@@ -657,53 +717,23 @@ __global__ void k_post(AtomsView A, int mode, int obs) {
     replica_store(&sR, A.rep + blockIdx.x);
 }
 
-// calculate_thermodynamics (md_driver.cpp:648-730) on the replica's shared copy, one thread;
-// k_post spreads the Born tensor's division by the volume and the sample record over the
-// block.
-__device__ void thermodynamics(Replica *R, int mode, int obs,
-                               const double *sf, const double *sd, double S, double ekin,
-                               double virial) {
+// The rest of calculate_thermodynamics (md_driver.cpp:648-730) on the replica's shared copy, one
+// thread: the conserved energy from its parts (etot_th of the thermostat chain, etot_npt of the
+// barostat), the remaining fatal checks, the clock, the box.
+__device__ void thermodynamics(Replica *R, int mode, int obs, double etot_th, double etot_npt) {
     mdelast_observables &o = R->obs;
-    double const dt = R->dt;
     int const ens = R->ensemble;
-    int const N = R->n_atoms;
-    R->vscale = S;
-    o.ekin_tot = ekin;
-    o.ekin_atom = ekin / N;
-    double mom2 = 0.;
-    for (int a = 0; a < 3; ++a) {
-        o.momentum_tot[a] = S * sf[F_MV + a];
-        mom2 += o.momentum_tot[a] * o.momentum_tot[a];
-    }
-    if (mom2 / (2. * R->mass0 * ekin) > 1e-14)
-        atomicOr(&o.status, MDELAST_FATAL_MOMENTUM);
-    o.epot_atom = sf[F_EPOT] / N;
-    o.epot_eam_atom = sd[D_FSUM] / N;
     o.etot_atom = o.ekin_atom + o.epot_atom;
     double const old = o.etot_cons;
-    double etot = o.etot_atom * N;
+    double etot = o.etot_atom * R->n_atoms;
     if (ens == MDELAST_NVT || ens == MDELAST_NPT)
-        etot += chain_etot(R->th);
-    double const V = volume(R->h);
+        etot += etot_th;
     if (ens == MDELAST_NPT)
-        etot += V * R->baro_P + (0.5 * (R->p_eps * R->p_eps) / R->baro_w + chain_etot(R->bth));
+        etot += etot_npt;
     o.etot_cons = etot;
     double const e0 = mode == POST_INIT ? 0. : R->etot_cons_initial;
     o.etot_cons_err = fabs(etot / e0 - 1.);
     double const err_current = fabs(etot / old - 1.);
-    o.temperature_kin = 2. * ekin / (kBoltz * R->Nf);
-    if (obs) {
-        double const f2 = sf[F_F2];
-        o.total_force2 = f2;
-        o.temperature_conf_inverse =
-            (f2 != 0. && o.total_laplacian != 0.) ? kBoltz * o.total_laplacian / f2 : 0.;
-    }
-    o.pressure = (ekin * 2. / 3. + virial) / V;
-    double const S2 = S * S;
-    for (int k = 0; k < 6; ++k) {
-        o.stress_tensor[k] = (-sf[F_SIGMA + k] + S2 * sf[F_MVV + k]) / V;
-        o.born_stress_tensor[k] = sf[F_SIGMA + k] / V;
-    }
     double const p_trace = o.stress_tensor[0] + o.stress_tensor[1] + o.stress_tensor[2];
     if (fabs(o.pressure / (p_trace / 3.) - 1.) > 1e-5)
         atomicOr(&o.status, MDELAST_FATAL_PRESSURE);
@@ -711,11 +741,10 @@ __device__ void thermodynamics(Replica *R, int mode, int obs,
         R->cycle > 0.)
         atomicOr(&o.status, MDELAST_FATAL_CONSERVATION);
     if (mode == POST_STEP) {
-        R->time += dt;
+        R->time += R->dt;
         R->cycle += 1.;
     } else {
         R->etot_cons_initial = etot;
-        o.etot_cons_initial = etot;
     }
     o.etot_cons_initial = R->etot_cons_initial;
     o.time = R->time;
