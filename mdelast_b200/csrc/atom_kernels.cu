@@ -80,6 +80,7 @@ __global__ void k_cell_bin(AtomsView A) {
 // and everything summed over it are deterministic. One warp per half cell (about 8 atoms),
 // blockDim.x / 32 cells per block.
 __global__ void k_cell_sort(AtomsView A) {
+    chain_begin();
     extern __shared__ int s_mem[];
     __shared__ int s_max; // the block's largest cell count: one global atomic per block
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -171,6 +172,7 @@ __device__ __forceinline__ float cell_gap(int d, float f) {
 }
 
 __global__ void __launch_bounds__(kWarpsH * 32, 3) k_nbr_cells(AtomsView A) {
+    chain_begin();
     extern __shared__ unsigned char s_raw[];
     float4 *s_w = reinterpret_cast<float4 *>(s_raw); // wrapped scaled, FP32
     int *s_j = reinterpret_cast<int *>(s_w + kStageH);
@@ -508,6 +510,7 @@ __device__ __forceinline__ void nbr_build_atom(AtomsView const &A, int i, unsign
 // Grid-striding warps over the atoms of the replicas k_nbr_cells left (all when
 // !cells_done); the padding slots keep the zero counts of their allocation.
 __global__ void k_nbr_build(AtomsView A, int cells_done) {
+    chain_begin();
     unsigned const lane = threadIdx.x & 31u;
     int const w0 = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int const n_warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
@@ -534,6 +537,7 @@ __global__ void k_nbr_build(AtomsView A, int cells_done) {
 // per atom).
 template <bool OBS, int TPA, int IP, typename IX>
 __global__ void __launch_bounds__(kBlock) k_density(AtomsView A, TablesView T) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     constexpr int kF = TabFmt<IP>::kF;
@@ -799,6 +803,7 @@ __device__ __forceinline__ void force_row(AtomsView const &A, TablesView const &
 
 template <bool OBS, bool KICK, int TPA, int IP, typename IX>
 __global__ void __launch_bounds__(kBlock) k_force(AtomsView A, TablesView T) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     int const tid = threadIdx.x;
@@ -933,6 +938,7 @@ __global__ void __launch_bounds__(kBlock) k_force(AtomsView A, TablesView T) {
 // c += (cf dt) v / h with the box before this step's barostat update.
 
 __global__ void __launch_bounds__(kBlock) k_kick_drift(AtomsView A, TablesView T) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     // the grid covers the n_pad slots exactly; a warp never spans two replicas (their
@@ -1158,6 +1164,7 @@ __host__ __device__ size_t sublist_smem(int maxn) {
 
 // 5 blocks of 256 threads per SM (the launch is 5 blocks per SM): at most 48 registers
 __global__ void __launch_bounds__(256, 5) k_sublist(AtomsView A) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     extern __shared__ int s_sub[];
@@ -1179,6 +1186,7 @@ __global__ void __launch_bounds__(256, 5) k_sublist(AtomsView A) {
 }
 
 __global__ void k_sub_invalidate(AtomsView A) {
+    chain_begin();
     for (int r = threadIdx.x; r < A.n_rep; r += blockDim.x)
         A.rep[r].sub_force = 1;
 }
@@ -1277,6 +1285,11 @@ __global__ void k_half_list_fill(AtomsView A, int r, const int *point, int *out)
     }
 }
 
+__global__ void k_clear_counts(AtomsView A) {
+    if (threadIdx.x < 2)
+        A.max_count[threadIdx.x] = 0;
+}
+
 __global__ void k_status_and(AtomsView A, unsigned mask) {
     for (int r = threadIdx.x; r < A.n_rep; r += blockDim.x)
         atomicAnd(&A.rep[r].obs.status, mask);
@@ -1335,10 +1348,10 @@ namespace {
 template <bool OBS, int IP, typename IX>
 void density_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesView const &T) {
     switch (tpa) {
-    case 1: k_density<OBS, 1, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 4: k_density<OBS, 4, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 8: k_density<OBS, 8, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    default: k_density<OBS, 16, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
+    case 1: launch_chain(k_density<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_chain(k_density<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_chain(k_density<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_density<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -1351,10 +1364,10 @@ void density_tpa(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesVi
 template <bool OBS, bool KICK, int IP, typename IX>
 void force_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesView const &T) {
     switch (tpa) {
-    case 1: k_force<OBS, KICK, 1, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 4: k_force<OBS, KICK, 4, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 8: k_force<OBS, KICK, 8, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    default: k_force<OBS, KICK, 16, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
+    case 1: launch_chain(k_force<OBS, KICK, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_chain(k_force<OBS, KICK, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_chain(k_force<OBS, KICK, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_force<OBS, KICK, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>

@@ -1,8 +1,9 @@
 // Host orchestration of the B200 path: the mdelast_driver_* entry points of
 // include/mdelast.h. A driver owns its device buffers and one stream; integrate() is one
-// CUDA-graph launch per step (the two graphs differ in whether the step samples the Born
-// tensor and the Laplacian). Results come back lazily: the graph's last node copies the
-// scalar observables into pinned host memory and the first read after a step waits for it.
+// CUDA-graph launch per step (the graphs differ in whether the step rebuilds the list, samples
+// the Born tensor and the Laplacian, and ends a launch). Results come back lazily: the closing
+// kernel of a launch's last step writes the scalar observables into pinned host memory and the
+// first read after it waits for that.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -261,15 +262,16 @@ struct mdelast_driver_s {
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(k_sublist, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem));
-            k_sublist<<<std::min(n_pad / 8, kSublistBlocks), 256, smem, s>>>(A);
+            launch_chain(k_sublist, std::min(n_pad / 8, kSublistBlocks), 256, smem, s, A);
         }
     }
     double *d_pd = nullptr, *d_pf = nullptr, *d_red = nullptr;
     size_t cap_dmap = 0, cap_fmap = 0, cap_pd = 0, cap_pf = 0, cap_red = 0; // elements
     // closing scalar work: fold the block sums, then the per-replica kernel
-    void post(int mode, int obs, cudaStream_t s) {
-        k_reduce<<<dim3(A.max_chunks, n_rep), 256, 0, s>>>(A);
-        k_post<<<n_rep, 256, 0, s>>>(A, mode, obs);
+    // (which writes the observables to h_obs when to_host)
+    void post(int mode, int obs, bool to_host, cudaStream_t s) {
+        launch_chain(k_reduce, dim3(A.max_chunks, n_rep), 256, 0, s, A);
+        launch_chain(k_post, n_rep, 256, 0, s, A, mode, obs, to_host ? h_obs : nullptr);
     }
     int *d_cell_count = nullptr, *d_cell_atoms = nullptr, *d_max_count = nullptr;
     int *d_halt = nullptr; // AtomsView::halt
@@ -305,7 +307,7 @@ struct mdelast_driver_s {
     TablesView T{};
     mdelast_observables *h_obs = nullptr; // pinned, n_rep entries
     cudaEvent_t ev_step = nullptr;
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr}; // [2 * rebuild + obs]
+    cudaGraphExec_t graph[8] = {}; // [4 * last + 2 * rebuild + obs]
     unsigned long long host_cycle = 0; // steps launched (the reference's cycle counter)
     int list_regrowths = 0;            // launches resumed after a list overflow
     bool all_pairs = false; // every replica lists by all-pairs search
@@ -321,10 +323,10 @@ struct mdelast_driver_s {
     std::vector<long> pos0_off;            // offset of each replica in d_pos0
     int enqueue_rebuild();
     int build_list_checked();
-    int enqueue_step(int obs, int rebuild, cudaEvent_t const *ev = nullptr);
+    int enqueue_step(int obs, int rebuild, int last, cudaEvent_t const *ev = nullptr);
     int time_steps(int n, int rebuild_every, double *ms_d, double *ms_f);
     int tune_on_steps(int n, int rebuild_every, int *choice, double *ms);
-    int step_graph(int obs, int rebuild, cudaGraphExec_t *out);
+    int step_graph(int obs, int rebuild, int last, cudaGraphExec_t *out);
     int launch_steps(int n_steps, int rebuild_every, int sample_every);
     int wait_step();
     int check_status();
@@ -582,7 +584,7 @@ int mdelast_driver_s::time_steps(int n, int rebuild_every, double *ms_d, double 
         last_launch.n = 1;
         last_launch.rebuild_every = rebuild_every;
         last_launch.sample_every = 1;
-        rc = enqueue_step(1, rebuild, ev);
+        rc = enqueue_step(1, rebuild, 1, ev);
         if (rc)
             break;
         ++host_cycle;
@@ -789,8 +791,9 @@ std::vector<double> mdelast_driver_s::current_boxes() const {
     return b;
 }
 
+// The largest counts (d_max_count) are read only by build_list_checked, which clears them first (with a
+// kernel: what a chained launch follows is a kernel throughout).
 int mdelast_driver_s::enqueue_rebuild() {
-    CK(cudaMemsetAsync(d_max_count, 0, 2 * sizeof(int), stream));
     int const grid = n_pad / kBlock;
     if (!all_pairs && A.n_cells > 0) {
         CK(cudaMemsetAsync(d_cell_count, 0, sizeof(int) * A.n_cells, stream));
@@ -807,7 +810,7 @@ int mdelast_driver_s::enqueue_rebuild() {
         if (sort_smem > 48 * 1024)
             CK(cudaFuncSetAttribute(k_cell_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(sort_smem)));
-        k_cell_sort<<<(A.n_cells + wpb - 1) / wpb, 32 * wpb, sort_smem, stream>>>(A);
+        launch_chain(k_cell_sort, (A.n_cells + wpb - 1) / wpb, 32 * wpb, sort_smem, stream, A);
     }
     int cells_done = 0;
     size_t const smem = nbr_cells_smem(A.cell_cap);
@@ -817,13 +820,13 @@ int mdelast_driver_s::enqueue_rebuild() {
         // the dynamic part alone may stay below 48 KB while static + dynamic exceed it
         CK(cudaFuncSetAttribute(k_nbr_cells, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
-        k_nbr_cells<<<A.n_cells / 8, kNbrCellsThreads, smem, stream>>>(A);
+        launch_chain(k_nbr_cells, A.n_cells / 8, kNbrCellsThreads, smem, stream, A);
         cells_done = 1;
     }
     // all-pairs replicas, and cell replicas k_nbr_cells left (narrow or too crowded cells)
-    k_nbr_build<<<std::min(n_pad / 8, 148 * 8), 256, 0, stream>>>(A, cells_done);
+    launch_chain(k_nbr_build, std::min(n_pad / 8, 148 * 8), 256, 0, stream, A, cells_done);
     if (A.crd_ref)
-        k_sub_invalidate<<<1, 128, 0, stream>>>(A);
+        launch_chain(k_sub_invalidate, 1, 128, 0, stream, A);
     CK(cudaGetLastError());
     return MDELAST_OK;
 }
@@ -842,6 +845,7 @@ double list_headroom() {
 // Build the list now and grow the neighbour or cell capacity until it fits.
 int mdelast_driver_s::build_list_checked() {
     for (int attempt = 0; attempt < 6; ++attempt) {
+        k_clear_counts<<<1, 32, 0, stream>>>(A);
         if (int rc = enqueue_rebuild())
             return rc;
         int mc[2];
@@ -871,13 +875,14 @@ int mdelast_driver_s::build_list_checked() {
     return fail(MDELAST_ERR_CAPACITY, "neighbour list did not fit after repeated growth");
 }
 
-int mdelast_driver_s::enqueue_step(int obs, int rebuild, cudaEvent_t const *ev) {
+// last: the step's observables go to the host (the last step of a launch)
+int mdelast_driver_s::enqueue_step(int obs, int rebuild, int last, cudaEvent_t const *ev) {
     int const grid = n_pad / kBlock;
     if (rebuild && neighbors) // calculate_neighbors() before integrate() (md.py:1245-1251)
         if (int rc = enqueue_rebuild())
             return rc;
-    k_pre<<<n_rep, 64, 0, stream>>>(A);
-    k_kick_drift<<<grid, kBlock, 0, stream>>>(A, T);
+    launch_chain(k_pre, n_rep, 64, 0, stream, A);
+    launch_chain(k_kick_drift, grid, kBlock, 0, stream, A, T);
     if (!neighbors)
         if (int rc = enqueue_rebuild())
             return rc;
@@ -890,21 +895,18 @@ int mdelast_driver_s::enqueue_step(int obs, int rebuild, cudaEvent_t const *ev) 
     pass_force(obs != 0, true, stream);
     if (ev)
         CK(cudaEventRecord(ev[2], stream));
-    post(POST_STEP, obs, stream);
+    post(POST_STEP, obs, last != 0, stream);
     CK(cudaGetLastError());
-    CK(cudaMemcpy2DAsync(h_obs, sizeof(mdelast_observables),
-                         reinterpret_cast<char *>(d_rep) + offsetof(Replica, obs), sizeof(Replica),
-                         sizeof(mdelast_observables), n_rep, cudaMemcpyDeviceToHost, stream));
     return MDELAST_OK;
 }
 
 // The instantiated graph of one step, captured on first use.
-int mdelast_driver_s::step_graph(int obs, int rebuild, cudaGraphExec_t *out) {
-    cudaGraphExec_t &ge = graph[2 * (rebuild ? 1 : 0) + (obs ? 1 : 0)];
+int mdelast_driver_s::step_graph(int obs, int rebuild, int last, cudaGraphExec_t *out) {
+    cudaGraphExec_t &ge = graph[4 * (last ? 1 : 0) + 2 * (rebuild ? 1 : 0) + (obs ? 1 : 0)];
     if (!ge) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        int rc = enqueue_step(obs, rebuild);
+        int rc = enqueue_step(obs, rebuild, last);
         cudaError_t e = cudaStreamEndCapture(stream, &g);
         if (rc)
             return rc;
@@ -933,7 +935,7 @@ int mdelast_driver_s::launch_steps(int n_steps, int rebuild_every, int sample_ev
                                          : (sample_every > 0 &&
                                             (c + 1) % static_cast<unsigned>(sample_every) == 0);
         cudaGraphExec_t g;
-        if (int rc = step_graph(obs, rebuild, &g))
+        if (int rc = step_graph(obs, rebuild, s == n_steps - 1, &g))
             return rc;
         CK(cudaGraphLaunch(g, stream));
         ++host_cycle;
@@ -1581,14 +1583,10 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
     }
     d->pass_density(true, d->stream);
     d->pass_force(true, false, d->stream);
-    d->post(POST_INIT, 1, d->stream);
+    d->post(POST_INIT, 1, true, d->stream);
     if (cudaGetLastError() != cudaSuccess)
         return bail(fail(MDELAST_ERR_CUDA, "kernel launch failed"));
-    if (cudaMemcpy2DAsync(d->h_obs, sizeof(mdelast_observables),
-                          reinterpret_cast<char *>(d->d_rep) + offsetof(Replica, obs),
-                          sizeof(Replica), sizeof(mdelast_observables), d->n_rep,
-                          cudaMemcpyDeviceToHost, d->stream) ||
-        cudaStreamSynchronize(d->stream))
+    if (cudaStreamSynchronize(d->stream))
         return bail(fail(MDELAST_ERR_CUDA, "constructor force call failed: %s",
                          cudaGetErrorString(cudaGetLastError())));
     d->obs_valid = true;
@@ -1669,9 +1667,9 @@ int mdelast_driver_kernel_times(mdelast_driver *d, int32_t n_steps, double *ms_o
         if (d->neighbors || step == 0)
             rc = d->enqueue_rebuild();
         cudaEventRecord(ev[1], s);
-        k_pre<<<d->n_rep, 64, 0, s>>>(d->A);
+        launch_chain(k_pre, d->n_rep, 64, 0, s, d->A);
         cudaEventRecord(ev[2], s);
-        k_kick_drift<<<grid, kBlock, 0, s>>>(d->A, d->T);
+        launch_chain(k_kick_drift, grid, kBlock, 0, s, d->A, d->T);
         cudaEventRecord(ev[3], s);
         d->refresh_pair_list(s);
         cudaEventRecord(ev[7], s);
@@ -1679,7 +1677,7 @@ int mdelast_driver_kernel_times(mdelast_driver *d, int32_t n_steps, double *ms_o
         cudaEventRecord(ev[4], s);
         d->pass_force(true, true, s);
         cudaEventRecord(ev[5], s);
-        d->post(POST_STEP, 1, s);
+        d->post(POST_STEP, 1, false, s);
         cudaEventRecord(ev[6], s);
         cudaError_t e = cudaEventSynchronize(ev[6]);
         if (e != cudaSuccess) {

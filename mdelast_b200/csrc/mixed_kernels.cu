@@ -159,6 +159,7 @@ __device__ __forceinline__ void dens_loop(AtomsView const &A, TablesView const &
 // 4 lanes per atom 0.195 -> 0.162 ms with the 32-byte records and warp_slots.
 template <bool OBS, int TPA, int IP, typename IX>
 __global__ void __launch_bounds__(kBlock, 8) k_density_mx(AtomsView A, TablesView T) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     constexpr int kF = TabFmt<IP>::kF;
@@ -495,6 +496,7 @@ constexpr int kBlockStaged = kStagedBlock;
 template <bool OBS, bool KICK, int TPA, int IP, bool STAGED, typename IX,
           int NB = STAGED ? kBlockStaged : kBlock>
 __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
+    chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     extern __shared__ float4 s_stage[];
@@ -649,10 +651,10 @@ template <bool OBS, int IP, typename IX>
 void density_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                        TablesView const &T) {
     switch (tpa) {
-    case 1: k_density_mx<OBS, 1, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 4: k_density_mx<OBS, 4, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 8: k_density_mx<OBS, 8, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    default: k_density_mx<OBS, 16, IP, IX><<<grid, kBlock, 0, s>>>(A, T); break;
+    case 1: launch_chain(k_density_mx<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_chain(k_density_mx<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_chain(k_density_mx<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_density_mx<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -666,10 +668,10 @@ template <bool OBS, bool KICK, int IP, typename IX>
 void force_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                      TablesView const &T) {
     switch (tpa) {
-    case 1: k_force_mx<OBS, KICK, 1, IP, false, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 4: k_force_mx<OBS, KICK, 4, IP, false, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    case 8: k_force_mx<OBS, KICK, 8, IP, false, IX><<<grid, kBlock, 0, s>>>(A, T); break;
-    default: k_force_mx<OBS, KICK, 16, IP, false, IX><<<grid, kBlock, 0, s>>>(A, T); break;
+    case 1: launch_chain(k_force_mx<OBS, KICK, 1, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_chain(k_force_mx<OBS, KICK, 4, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_chain(k_force_mx<OBS, KICK, 8, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_force_mx<OBS, KICK, 16, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>
@@ -686,10 +688,10 @@ void force_mx_staged_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
     size_t const smem = static_cast<size_t>(T.st_bytes);
     constexpr int Q = MDELAST_QUINTIC;
     switch (tpa) {
-    case 4: k_force_mx<OBS, KICK, 4, Q, true, IX><<<grid, kBlockStaged, smem, s>>>(A, T); break;
-    case 8: k_force_mx<OBS, KICK, 8, Q, true, IX><<<grid, kBlockStaged, smem, s>>>(A, T); break;
+    case 4: launch_chain(k_force_mx<OBS, KICK, 4, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    case 8: launch_chain(k_force_mx<OBS, KICK, 8, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
     default:
-        k_force_mx<OBS, KICK, 16, Q, true, IX><<<grid, kBlockStaged, smem, s>>>(A, T);
+        launch_chain(k_force_mx<OBS, KICK, 16, Q, true, IX>, grid, kBlockStaged, smem, s, A, T);
         break;
     }
 }

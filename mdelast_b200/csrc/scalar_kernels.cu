@@ -380,6 +380,7 @@ __device__ __forceinline__ void replica_store(Replica const *s, Replica *g) {
 // side from the same barostat momentum. Everything read from the replica is read before the
 // chains, so that no round trip to memory sits behind them.
 __global__ void k_pre(AtomsView A) {
+    chain_begin();
     if (*A.halt) // a list build ran out of capacity: nothing until the host regrows
         return;
     Replica *R = A.rep + blockIdx.x;
@@ -446,6 +447,7 @@ __global__ void k_pre(AtomsView A) {
 // (c, r) adds blocks [c kChunk, (c+1) kChunk) of replica r for every slot, in a fixed
 // order, spreading the reduction over many SMs (k_post then adds the chunk sums).
 __global__ void k_reduce(AtomsView A) {
+    chain_begin();
     if (*A.halt) // a list build ran out of capacity: nothing until the host regrows
         return;
     Replica const *R = A.rep + blockIdx.y;
@@ -584,9 +586,24 @@ __global__ void k_samples_reset(AtomsView A, int what) {
 
 __device__ void thermodynamics(Replica *R, int mode, int obs, double etot_th, double etot_npt);
 
-__global__ void k_post(AtomsView A, int mode, int obs) {
-    if (*A.halt) // a list build ran out of capacity: nothing until the host regrows
+// host: pinned memory that takes the replicas' observables (null: not on this step). A halted
+// step hands them over too: the host reads the overflow and the last completed cycle from them.
+__device__ __forceinline__ void to_host(mdelast_observables const &o, mdelast_observables *host) {
+    static_assert(sizeof(mdelast_observables) % sizeof(double) == 0, "copied as doubles");
+    const double *src = reinterpret_cast<const double *>(&o);
+    double *dst = reinterpret_cast<double *>(host + blockIdx.x);
+    for (int k = threadIdx.x; k < static_cast<int>(sizeof(mdelast_observables) / sizeof(double));
+         k += blockDim.x)
+        dst[k] = src[k];
+}
+
+__global__ void k_post(AtomsView A, int mode, int obs, mdelast_observables *host) {
+    chain_begin();
+    if (*A.halt) { // a list build ran out of capacity: nothing until the host regrows
+        if (host)
+            to_host(A.rep[blockIdx.x].obs, host);
         return;
+    }
     __shared__ Replica sR;
     __shared__ double sf[F_NSUM], sd[D_NSUM];
     __shared__ double s_part[4][F_NSUM + D_NSUM];
@@ -715,6 +732,8 @@ __global__ void k_post(AtomsView A, int mode, int obs) {
         record_sample(A, static_cast<int>(blockIdx.x), R, V);
     }
     replica_store(&sR, A.rep + blockIdx.x);
+    if (host)
+        to_host(sR.obs, host);
 }
 
 // The rest of calculate_thermodynamics (md_driver.cpp:648-730) on the replica's shared copy, one
