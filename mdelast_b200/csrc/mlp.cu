@@ -3,10 +3,12 @@
 // Adam kernels. It maps (composition, temperature) to the zero-pressure lattice constant
 // and initial C11, C12, C44, so that a production run can start near equilibrium.
 //
-// Sizes are small (inputs and widths of tens, a few thousand samples), so every kernel is a
-// plain FP32 FMA loop with one thread per output element and sums in a fixed order: no
-// atomics, training is bit-for-bit repeatable. A training step (forward, loss, backward,
-// Adam) is captured once as a CUDA graph and replayed.
+// Sizes are small (inputs and widths of tens, a few thousand samples), so every kernel is
+// FP32 FMA work with sums in a fixed order: no atomics, training is bit-for-bit repeatable.
+// A network whose parameters, gradients and activations of 16 samples fit a block's shared
+// memory (every network this package trains) takes a training step in two kernels, k_step_grad and
+// k_step_update; larger ones run layer by layer, the step captured once as a CUDA graph and
+// replayed.
 //
 // Parameter layout (also of gradients and of the host copies): for each layer l in order,
 // W_l as in_l x out_l row-major (W[i * out + o]), then b_l (out_l).
@@ -19,6 +21,7 @@
 #include <vector>
 
 #include "host_tables.h"
+#include "kernels.cuh"
 #include "mdelast.h"
 
 using mdelast::clear_error;
@@ -113,25 +116,292 @@ __global__ void k_bwd_dw(const float *X, const float *dZ, float *dW, float *db, 
 
 // Adam (Kingma & Ba 2015) with bias correction; the step count lives on the device so that
 // a captured graph can be replayed
-__global__ void k_adam(float *p, const float *g, float *m1, float *m2, int np, float lr,
-                       const int *t) {
-    int const k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np)
-        return;
+__device__ __forceinline__ void adam(float *p, float *m1, float *m2, int k, float gk, float lr,
+                                     float step) {
     float const b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    float const step = static_cast<float>(*t + 1);
     float const c1 = 1.f - powf(b1, step), c2 = 1.f - powf(b2, step);
-    float const gk = g[k];
     float const a = b1 * m1[k] + (1.f - b1) * gk;
     float const v = b2 * m2[k] + (1.f - b2) * gk * gk;
     m1[k] = a;
     m2[k] = v;
     p[k] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
 }
+__global__ void k_adam(float *p, const float *g, float *m1, float *m2, int np, float lr,
+                       const int *t) {
+    int const k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < np)
+        adam(p, m1, m2, k, g[k], lr, static_cast<float>(*t + 1));
+}
 
 __global__ void k_step_inc(int *t) {
     if (threadIdx.x == 0 && blockIdx.x == 0)
         *t += 1;
+}
+
+// ------------------------------------------------------------------------------------
+// A training step of a network that fits shared memory. Layer by layer, a step was 17
+// launches whose weight-gradient kernel ran one thread per weight down a serial chain over
+// all samples (2,048 samples: 0.55 of the step's 0.57 ms on a few blocks). Here each block takes tiles of
+// kTile16 samples through forward, loss and backward out of shared memory, with the weight
+// gradients of its tiles summed there in sample order; k_step_update adds the blocks' sums in block
+// order and applies Adam. 2,048 samples fill 128 of the 148 SMs once. 2-64-64-64-4 network,
+// 2,048 samples: 570 -> 22 us per training step; what bounds it now is latency inside one block
+// per SM (16 warps, dot products of 64 out of shared memory between barriers).
+constexpr int kTile16 = 16;      // samples per tile
+constexpr int kTileP = 20;       // floats per activation row: 16-byte rows whose starts 8 lanes
+                                 // apart fall on different banks
+constexpr int kStepThreads = 512;
+constexpr int kStepBlocks = 148; // one block per SM; more samples loop over tiles
+constexpr size_t kStepSmemMax = 200 * 1024;
+
+struct NetView {
+    int L, np, n, wsum; // layers, parameters, samples, sum of all widths
+    int w[MDELAST_MLP_MAX_LAYERS + 1], off_w[MDELAST_MLP_MAX_LAYERS];
+};
+
+// The step's own copy of the parameters and its gradients are laid out as they lie in shared
+// memory: per layer w_l + 1 rows (the weights' and the bias) of w_{l+1} floats padded by one, so
+// that lanes along either index read different banks, the whole rounded to 16 bytes. The blocks copy
+// it in and their sums out with 16-byte accesses (copied element by element with the
+// layout's arithmetic, that was 17,000 of k_step_grad's 41,000 cycles).
+__host__ __device__ inline int padded_params(NetView const &v) {
+    int k = 0;
+    for (int l = 0; l < v.L; ++l)
+        k += (v.w[l] + 1) * (v.w[l + 1] + 1);
+    return (k + 3) / 4 * 4;
+}
+// index in the parameters' layout of padded entry k, -1 for a pad
+__device__ __forceinline__ int unpadded(NetView const &v, int k) {
+    for (int l = 0; l < v.L; ++l) {
+        int const out = v.w[l + 1], row = out + 1, rows = (v.w[l] + 1) * row;
+        if (k < rows) {
+            int const i = k / row, o = k - i * row;
+            return o < out ? v.off_w[l] + i * out + o : -1;
+        }
+        k -= rows;
+    }
+    return -1;
+}
+__host__ inline size_t step_smem(NetView const &v) {
+    int wmax = 0;
+    for (int l = 0; l <= v.L; ++l)
+        wmax = std::max(wmax, v.w[l]);
+    return sizeof(float) * (2 * static_cast<size_t>(padded_params(v)) +
+                            2 * static_cast<size_t>(kTileP) * (v.wsum + wmax));
+}
+
+// the padded copy of the parameters
+__global__ void k_step_params(NetView v, const float *p, float *pp) {
+    int const k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < padded_params(v)) {
+        int const u = unpadded(v, k);
+        pp[k] = u >= 0 ? p[u] : 0.f;
+    }
+}
+
+// Gradients of the mean-squared error summed over this block's tiles, to part[block] (in the
+// padded layout) and its loss sum to part_loss[block]. count: the training step counter
+// to advance (null outside training).
+__global__ void __launch_bounds__(kStepThreads)
+    k_step_grad(NetView v, const float *X, const float *Y, const float *pp, float *part,
+                float *part_loss, int *count) {
+    mdelast::chain_begin();
+    extern __shared__ float4 s_net[];
+    int const tid = threadIdx.x, T = kStepThreads, L = v.L;
+    float *sW = reinterpret_cast<float *>(s_net); // layer l: (w_l + 1) rows of w_{l+1} + 1
+    int const nW = padded_params(v);
+    float *sG = sW + nW;            // gradients in the same layout
+    float *sA = sG + nW;            // activations of layer l: rows of kTileP samples
+    float *sD = sA + kTileP * v.wsum; // gelu'(z) of layer l
+    int wmax = 0;
+    for (int l = 0; l <= L; ++l)
+        wmax = max(wmax, v.w[l]);
+    float *sP = sD + kTileP * v.wsum; // dA or dZ of the layer above, and of the one below
+    float *sQ = sP + kTileP * wmax;
+    __shared__ float s_loss[kStepThreads];
+    if (count && blockIdx.x == 0 && tid == 0)
+        *count += 1;
+#pragma unroll 8
+    for (int k = tid; k < nW / 4; k += T) {
+        reinterpret_cast<float4 *>(sW)[k] = reinterpret_cast<const float4 *>(pp)[k];
+        reinterpret_cast<float4 *>(sG)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float const inv = 1.f / static_cast<float>(v.n * v.w[L]);
+    float loss = 0.f;
+    int const tiles = (v.n + kTile16 - 1) / kTile16;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        int const s0 = t * kTile16;
+        __syncthreads(); // weights in place; the previous tile is done with
+        for (int k = tid; k < kTile16 * v.w[0]; k += T) {
+            int const s = k / v.w[0], i = k % v.w[0];
+            sA[i * kTileP + s] = s0 + s < v.n ? X[static_cast<size_t>(s0 + s) * v.w[0] + i] : 0.f;
+        }
+        __syncthreads();
+        // forward: a thread forms 2 samples of one output
+        int a0 = 0, o0 = 0;
+        for (int l = 0; l < L; ++l) {
+            int const in = v.w[l], out = v.w[l + 1], row = out + 1;
+            const float *x = sA + kTileP * a0;
+            float *A = sA + kTileP * (a0 + in), *D = sD + kTileP * (a0 + in);
+            for (int k = tid; k < out * (kTile16 / 2); k += T) {
+                int const o = k % out, q = 2 * (k / out);
+                const float *W = sW + o0 + o;
+                float2 z = make_float2(W[in * row], W[in * row]);
+#pragma unroll 8
+                for (int i = 0; i < in; ++i) {
+                    float const w = W[i * row];
+                    float2 const a = *reinterpret_cast<const float2 *>(x + i * kTileP + q);
+                    z.x = fmaf(a.x, w, z.x);
+                    z.y = fmaf(a.y, w, z.y);
+                }
+                if (l + 1 < L) {
+                    *reinterpret_cast<float2 *>(D + o * kTileP + q) =
+                        make_float2(gelu_d(z.x), gelu_d(z.y));
+                    z = make_float2(gelu(z.x), gelu(z.y));
+                }
+                *reinterpret_cast<float2 *>(A + o * kTileP + q) = z;
+            }
+            a0 += in;
+            o0 += (in + 1) * row;
+            __syncthreads();
+        }
+        // loss and its derivative
+        for (int k = tid; k < kTile16 * v.w[L]; k += T) {
+            int const s = k / v.w[L], o = k % v.w[L];
+            float d = 0.f;
+            if (s0 + s < v.n) {
+                d = sA[(a0 + o) * kTileP + s] - Y[static_cast<size_t>(s0 + s) * v.w[L] + o];
+                loss = fmaf(d, d, loss);
+            }
+            sP[o * kTileP + s] = 2.f * d * inv;
+        }
+        __syncthreads();
+        // backward: sP holds dZ of layer l + 1
+        for (int l = L - 1; l >= 0; --l) {
+            int const in = v.w[l], out = v.w[l + 1], row = out + 1;
+            a0 -= in;
+            o0 -= (in + 1) * row;
+            // weight gradients: lanes along the outputs, a thread every (T / out)-th input
+            // (or, wider than the block, several outputs); the bias is the row after the inputs
+            const float *x = sA + kTileP * a0;
+            int const groups = max(1, T / out);
+            for (int o = tid % out; o < out && tid < groups * out; o += T) {
+                float dz[kTile16];
+#pragma unroll
+                for (int q = 0; q < kTile16; q += 4) {
+                    float4 const d = *reinterpret_cast<const float4 *>(sP + o * kTileP + q);
+                    dz[q] = d.x;
+                    dz[q + 1] = d.y;
+                    dz[q + 2] = d.z;
+                    dz[q + 3] = d.w;
+                }
+                // two inputs at a time: two independent chains of FMAs in sample order
+                for (int i = tid / out; i < in; i += 2 * groups) {
+                    int const i1 = min(i + groups, in - 1);
+                    float g = sG[o0 + i * row + o], g1 = sG[o0 + i1 * row + o];
+#pragma unroll
+                    for (int q = 0; q < kTile16; q += 4) {
+                        float4 const a = *reinterpret_cast<const float4 *>(x + i * kTileP + q),
+                                     b = *reinterpret_cast<const float4 *>(x + i1 * kTileP + q);
+                        g = fmaf(a.x, dz[q], g);
+                        g1 = fmaf(b.x, dz[q], g1);
+                        g = fmaf(a.y, dz[q + 1], g);
+                        g1 = fmaf(b.y, dz[q + 1], g1);
+                        g = fmaf(a.z, dz[q + 2], g);
+                        g1 = fmaf(b.z, dz[q + 2], g1);
+                        g = fmaf(a.w, dz[q + 3], g);
+                        g1 = fmaf(b.w, dz[q + 3], g1);
+                    }
+                    sG[o0 + i * row + o] = g;
+                    if (i + groups < in)
+                        sG[o0 + i1 * row + o] = g1;
+                }
+                if (tid < out || out > T) {
+                    float g = sG[o0 + in * row + o];
+#pragma unroll
+                    for (int q = 0; q < kTile16; ++q)
+                        g += dz[q];
+                    sG[o0 + in * row + o] = g;
+                }
+            }
+            // dZ of layer l = dA gelu'(z)
+            if (l > 0) {
+                const float *D = sD + kTileP * a0;
+                for (int k = tid; k < in * (kTile16 / 2); k += T) {
+                    int const i = k % in, q = 2 * (k / in);
+                    const float *W = sW + o0 + i * row;
+                    float2 a = make_float2(0.f, 0.f);
+#pragma unroll 8
+                    for (int o = 0; o < out; ++o) {
+                        float const w = W[o];
+                        float2 const d = *reinterpret_cast<const float2 *>(sP + o * kTileP + q);
+                        a.x = fmaf(d.x, w, a.x);
+                        a.y = fmaf(d.y, w, a.y);
+                    }
+                    float2 const g = *reinterpret_cast<const float2 *>(D + i * kTileP + q);
+                    *reinterpret_cast<float2 *>(sQ + i * kTileP + q) =
+                        make_float2(a.x * g.x, a.y * g.y);
+                }
+                __syncthreads();
+                float *const u = sP;
+                sP = sQ;
+                sQ = u;
+            }
+        }
+    }
+    s_loss[tid] = loss;
+    __syncthreads();
+    for (int w = T / 2; w > 0; w >>= 1) {
+        if (tid < w)
+            s_loss[tid] += s_loss[tid + w];
+        __syncthreads();
+    }
+    if (tid == 0)
+        part_loss[blockIdx.x] = s_loss[0];
+    float4 *out_p = reinterpret_cast<float4 *>(part + static_cast<size_t>(blockIdx.x) * nW);
+    for (int k = tid; k < nW / 4; k += T)
+        out_p[k] = reinterpret_cast<float4 *>(sG)[k];
+}
+
+// The blocks' gradients added in block order (4 threads of a parameter take every fourth block,
+// their sums are added in order), then Adam (lr > 0) with the step counter k_step_grad advanced.
+// Block 0 adds the loss sums.
+constexpr int kUpdateThreads = 256;
+__global__ void __launch_bounds__(kUpdateThreads)
+    k_step_update(NetView v, const float *part, const float *part_loss, int n_part, float inv_m,
+                  float *g, float *loss, float *p, float *pp, float *m1, float *m2, float lr,
+                  const int *t) {
+    mdelast::chain_begin();
+    __shared__ float s_g[3][64];
+    int const c = threadIdx.x & 63, q = threadIdx.x >> 6, np = padded_params(v);
+    int const k = blockIdx.x * 64 + c;
+    float a = 0.f;
+    if (k < np)
+#pragma unroll 16
+        for (int b = q; b < n_part; b += 4)
+            a += part[static_cast<size_t>(b) * np + k];
+    if (q > 0)
+        s_g[q - 1][c] = a;
+    __syncthreads();
+    int const u = q == 0 && k < np ? unpadded(v, k) : -1;
+    if (u >= 0) {
+        float const gk = ((a + s_g[0][c]) + s_g[1][c]) + s_g[2][c];
+        g[u] = gk;
+        if (lr > 0.f) {
+            adam(p, m1, m2, u, gk, lr, static_cast<float>(*t));
+            pp[k] = p[u];
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x >= kUpdateThreads - 32) {
+        float sum = 0.f;
+        for (int b = threadIdx.x & 31; b < n_part; b += 32)
+            sum += part_loss[b];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0)
+            *loss = sum * inv_m;
+    }
 }
 
 unsigned blocks(long m) { return static_cast<unsigned>((m + kT - 1) / kT); }
@@ -158,6 +428,40 @@ struct mdelast_mlp_s {
     int cap = 0;
     std::vector<float *> Z, A, dA;
     float *Yt = nullptr, *dZ = nullptr, *loss = nullptr;
+    // the two-kernel step: per-block gradients and loss sums (kStepBlocks of them)
+    bool fused = false;
+    size_t fused_smem = 0;
+    float *part = nullptr, *part_loss = nullptr, *pp = nullptr; // pp: the padded parameters
+    NetView view(int n) const {
+        NetView v{};
+        v.L = L;
+        v.np = static_cast<int>(np);
+        v.n = n;
+        for (int l = 0; l <= L; ++l) {
+            v.w[l] = w[l];
+            v.wsum += w[l];
+            if (l < L)
+                v.off_w[l] = static_cast<int>(off_w[l]);
+        }
+        return v;
+    }
+    // the padded copy of the current parameters, which the steps then keep
+    void begin_fused() {
+        NetView const v = view(1);
+        k_step_params<<<(padded_params(v) + 255) / 256, 256, 0, stream>>>(v, p, pp);
+    }
+    // gradients into g and the loss; an Adam step when lr > 0
+    int step_fused(int n, float lr) {
+        int const nb = std::min((n + kTile16 - 1) / kTile16, kStepBlocks);
+        NetView const v = view(n);
+        MCK(mdelast::launch_chain(k_step_grad, nb, kStepThreads, fused_smem, stream, v, A[0], Yt,
+                                  pp, part, part_loss, lr > 0.f ? t : nullptr));
+        MCK(mdelast::launch_chain(k_step_update, (padded_params(v) + 63) / 64, kUpdateThreads, 0,
+                                  stream, v, part, part_loss, nb,
+                                  1.f / static_cast<float>(n * w[L]), g, loss, p, pp, m1, m2, lr,
+                                  t));
+        return MDELAST_OK;
+    }
     cudaGraphExec_t graph = nullptr;
     int graph_n = -1;
     float graph_lr = 0.f;
@@ -166,9 +470,8 @@ struct mdelast_mlp_s {
         cudaSetDevice(device);
         if (graph)
             cudaGraphExecDestroy(graph);
-        for (float *q : {p, g, m1, m2, Yt, dZ, loss})
+        for (float *q : {p, Yt, dZ}) // p: the slab of all that is sized by the parameters
             cudaFree(q);
-        cudaFree(t);
         for (auto *v : {&Z, &A, &dA})
             for (float *q : *v)
                 cudaFree(q);
@@ -283,23 +586,30 @@ int mdelast_mlp_create(int32_t n_layers, const int32_t *widths, uint64_t seed, i
     }
     size_t const bytes = sizeof(float) * static_cast<size_t>(m->np);
     cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    for (float **q : {&m->p, &m->g, &m->m1, &m->m2})
-        if (e == cudaSuccess)
-            e = cudaMalloc(q, bytes);
+    // one allocation: p, g, m1, m2 (zero but p), the step counter, the loss, and the two-kernel
+    // step's per-block sums
+    m->fused_smem = step_smem(m->view(1));
+    m->fused = m->fused_smem <= kStepSmemMax;
+    size_t const np = (static_cast<size_t>(m->np) + 63) / 64 * 64,
+                 npp = static_cast<size_t>(padded_params(m->view(1))),
+                 extra = m->fused ? npp * (kStepBlocks + 1) + kStepBlocks : 0;
     if (e == cudaSuccess)
-        e = cudaMalloc(&m->t, sizeof(int));
+        e = cudaMalloc(&m->p, sizeof(float) * (4 * np + 64 + extra));
     if (e == cudaSuccess)
-        e = cudaMalloc(&m->loss, sizeof(float));
+        e = cudaMemset(m->p, 0, sizeof(float) * (4 * np + 64));
+    m->g = m->p + np;
+    m->m1 = m->p + 2 * np;
+    m->m2 = m->p + 3 * np;
+    m->t = reinterpret_cast<int *>(m->p + 4 * np);
+    m->loss = m->p + 4 * np + 32;
+    m->pp = m->p + 4 * np + 64;
+    m->part = m->pp + npp;
+    m->part_loss = m->part + npp * kStepBlocks;
+    if (e == cudaSuccess && m->fused)
+        e = cudaFuncSetAttribute(k_step_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kStepSmemMax));
     if (e == cudaSuccess)
         e = cudaMemcpy(m->p, h.data(), bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemset(m->m1, 0, bytes);
-    if (e == cudaSuccess)
-        e = cudaMemset(m->m2, 0, bytes);
-    if (e == cudaSuccess)
-        e = cudaMemset(m->g, 0, bytes);
-    if (e == cudaSuccess)
-        e = cudaMemset(m->t, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete m;
         return fail(MDELAST_ERR_CUDA, "MLP set-up: %s", cudaGetErrorString(e));
@@ -366,8 +676,14 @@ int mdelast_mlp_gradients(mdelast_mlp *m, const float *x, const float *y, int32_
     MCK(cudaSetDevice(m->device));
     if (int rc = m->upload(x, y, n))
         return rc;
-    m->forward(n, m->stream);
-    m->backward(n, m->stream);
+    if (m->fused) {
+        m->begin_fused();
+        if (int rc = m->step_fused(n, 0.f))
+            return rc;
+    } else {
+        m->forward(n, m->stream);
+        m->backward(n, m->stream);
+    }
     MCK(cudaGetLastError());
     if (loss)
         MCK(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -386,7 +702,12 @@ int mdelast_mlp_train(mdelast_mlp *m, const float *x, const float *y, int32_t n,
     MCK(cudaSetDevice(m->device));
     if (int rc = m->upload(x, y, n))
         return rc;
-    if (!m->graph || m->graph_n != n || m->graph_lr != lr) {
+    if (m->fused)
+        m->begin_fused();
+    for (int k = 0; m->fused && k < steps; ++k)
+        if (int rc = m->step_fused(n, lr))
+            return rc;
+    if (!m->fused && (!m->graph || m->graph_n != n || m->graph_lr != lr)) {
         if (m->graph) {
             cudaGraphExecDestroy(m->graph);
             m->graph = nullptr;
@@ -410,12 +731,17 @@ int mdelast_mlp_train(mdelast_mlp *m, const float *x, const float *y, int32_t n,
         m->graph_n = n;
         m->graph_lr = lr;
     }
-    for (int k = 0; k < steps; ++k)
+    for (int k = 0; !m->fused && k < steps; ++k)
         MCK(cudaGraphLaunch(m->graph, m->stream));
     if (loss) {
         // the loss of the parameters after the last step
-        m->forward(n, m->stream);
-        m->backward(n, m->stream);
+        if (m->fused) {
+            if (int rc = m->step_fused(n, 0.f))
+                return rc;
+        } else {
+            m->forward(n, m->stream);
+            m->backward(n, m->stream);
+        }
         MCK(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
     }
     MCK(cudaStreamSynchronize(m->stream));
