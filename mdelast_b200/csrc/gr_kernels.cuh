@@ -24,7 +24,7 @@ struct GrArgs {
 __host__ __device__ inline size_t gr_count_slots(int n_rg, int ntypes) {
     return static_cast<size_t>(1 + ntypes * (ntypes + 1) / 2) * static_cast<size_t>(n_rg);
 }
-// Thread blocks of the pair count for n atoms: one per pair of 128-atom tiles (I <= J).
+// Units of the pair count for n atoms: one per pair of 128-atom tiles (I <= J); the static variant launches a block each.
 // A launch takes at most 2^31 - 1 blocks, so callers reject n beyond gr_max_atoms().
 constexpr long kGrTileAtoms = 128;
 __host__ inline long gr_count_blocks(long n) {
