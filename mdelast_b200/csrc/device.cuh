@@ -188,7 +188,8 @@ __device__ __forceinline__ double min_image_r2(double4 ci, double4 cj, double hx
 }
 
 // Row i of the pair list in either entry width: at(k) is the atom slot of list slot k
-// (partners j > i from slot 0 up, j < i from slot pmaxn - 1 down). IX = int: slots as stored;
+// (its upper half from slot 0 up, its lower half from slot pmaxn - 1 down; of a pair's two rows
+// one holds it in the upper half). IX = int: slots as stored;
 // IX = uint16_t: offsets from the replica's first slot `base`. Loads stream (evict first):
 // each row is read once per pass.
 template <typename IX> struct PairRow {

@@ -326,9 +326,9 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
         ld256(T.rrf + (static_cast<size_t>(tj) * T.nri + k) * kFf, cj);
 }
 
-// One lane's walk over list slots [s0, s1) of an atom row (slots of partners j > i when
-// UPPER, else of partners j < i, addressed from the end of the row); every pair adds its
-// force and half its energy to the atom, and pairs j > i also add to the global sums.
+// One lane's walk over list slots [s0, s1) of an atom row (slots of the upper half when
+// UPPER, else of the lower half, addressed from the end of the row); every pair adds its
+// force and half its energy to the atom, and the upper half also adds to the global sums.
 // STAGED: quintic tables read from the staged shared-memory copy `stab` where staged.
 template <bool OBS, bool UPPER, int TPA, int IP, bool STAGED, typename IX, bool UC>
 __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView const &T,
@@ -474,8 +474,8 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
 }
 
 // Force pass of md_driver.cpp:300-430 (with the closing kick) in mixed precision; see
-// k_force for the roles of the terms. Each atom row is walked in two loops, partners j > i
-// (which also feed the global sums) and partners j < i, so the lanes of a warp do not
+// k_force for the roles of the terms. Each atom row is walked in two loops, its upper
+// half (which also feeds the global sums) and its lower half, so the lanes of a warp do not
 // diverge on the global-sum work. The row's 22 pair sums and, after the kick, its 12 sums
 // over atoms go through warp_slots (31 and, at 4 lanes per atom, 4 exchanges) into two FP64
 // registers per lane; the virial is the trace of the Born stress.

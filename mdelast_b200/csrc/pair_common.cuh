@@ -98,7 +98,7 @@ template <int TPA, typename V> __device__ __forceinline__ V group_sum(V x) {
     return x;
 }
 
-// list entry kk of an atom row: partners j > i at slots 0.., j < i at slots maxn-1 down
+// list entry kk of an atom row: the upper half at slots 0.., the lower half at slots maxn-1 down
 __device__ __forceinline__ int list_slot(int kk, int nu, int maxn) {
     return kk < nu ? kk : maxn - 1 - (kk - nu);
 }
