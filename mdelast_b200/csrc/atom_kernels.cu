@@ -972,11 +972,8 @@ __global__ void __launch_bounds__(kBlock) k_kick_drift(AtomsView A, TablesView T
                      dz = c.z * R->h[2] - c0.z;
         d2 = dx * dx + dy * dy + dz * dz;
     }
-    if (A.posf) // mixed precision: wrapped FP32 positions in the box after this drift
-        A.posf[i] = make_float4(static_cast<float>((c.x - nint_ref(c.x)) * R->h[0] / kAng),
-                                static_cast<float>((c.y - nint_ref(c.y)) * R->h[1] / kAng),
-                                static_cast<float>((c.z - nint_ref(c.z)) * R->h[2] / kAng),
-                                static_cast<float>(c.w));
+    if (A.posf)
+        A.posf[i] = position_f(c, R);
     }
     if (A.crd_ref) {
         // the replica's largest displacement: warp maximum, then one atomic per warp
@@ -1062,21 +1059,17 @@ __device__ __forceinline__ void sublist_row(AtomsView const &A, int i, int lane,
             out[slot] = j;
     };
     unsigned const lt = (1u << lane) - 1u;
-    // Mixed precision: the keep test runs in FP32 on the wrapped positions the pair passes
-    // read, with the minimum image they use (the same on both atoms of a pair, so the list
-    // stays symmetric), against the radius widened by 1e-5: every pair within it in exact
-    // arithmetic is kept, a few just beyond it too, which add zeros. FP64: the reference's
-    // min image and the exact radius.
-    // (the box edges in A by a product, not the pair passes' quotient: the list needs the
-    // same image on both atoms of a pair, not the pair passes' last bit)
+    // Mixed precision: the keep test runs in FP32 on the positions the pair passes read, with
+    // the minimum image they use (the same on both atoms of a pair, so the list stays
+    // symmetric), against the radius widened by 1e-5: every pair within it in exact arithmetic is
+    // kept, a few just beyond it too, which add zeros. FP64: the reference's min image and the
+    // exact radius.
     bool const f32 = A.posf != nullptr;
     float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
     float3 L = make_float3(0.f, 0.f, 0.f), iL = L;
     if (f32) {
         pi = A.posf[i];
-        L = make_float3(static_cast<float>(hx * 1e8), static_cast<float>(hy * 1e8),
-                        static_cast<float>(hz * 1e8));
-        iL = make_float3(__frcp_rn(L.x), __frcp_rn(L.y), __frcp_rn(L.z));
+        box_f(R, L, iL);
     }
     float const sub_r2f = sc.r2f, ish = f32 ? sc.inv_shell_a : sc.inv_shell;
     if (sorted) {

@@ -101,18 +101,20 @@ struct TablesView {
     double mass[kMaxTypes];
     // mixed precision: the r tables in FP32 with lengths in angstrom and values in eV
     // (phi) or angstrom^-3 (rho), one record of TabFmt<IP>::kFf floats per function and
-    // interval: phf phi_ab of every type pair (a <= b), rrf rho of every type. Cutoffs in
-    // angstrom.
-    const float *phf, *rrf;
-    float finv_hr, finv_hr2, fr_cut_sq, fpad;
+    // interval: phf phi_ab of every type pair (a <= b), rrf rho of every type (quintic records
+    // hold c0..c5, 3 c3, 5 c5); rdf, quintic only, rho for the force pass, which needs its
+    // derivatives alone: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5. Cutoffs in angstrom.
+    const float *phf, *rrf, *rdf;
+    float finv_hr, finv_hr2, fr_cut_sq, frmin_max; // frmin_max: the largest fpot_rmin
+    uint2 slots[kMaxTypes]; // byte b of slots[a]: pair_slot(a, b)
     // Staged copy for the shared-memory force pass (quintic only): the intervals
     // [st_lo, st_lo + st_n) of every phi_ab (slot s at s * st_n) followed by every rho_a
     // (type a at (npot + a) * st_n), 6 floats each, de-duplicated (each rho once, not once
     // per type pair). st_n == 0: no staged copy. st_bytes: its size (a multiple of 16).
     const float *stf;
     int st_lo, st_n, st_bytes;
-    // fuc: every function's FP32 cutoff is at least the pair cutoff, so no per-function
-    // cutoff applies to a pair within it; the mixed passes then skip those tests. uc64: the
+    // fuc: there is EAM and every function's FP32 cutoff is at least the pair cutoff, so no
+    // per-function test applies to a pair within it; the mixed passes then skip them. uc64: the
     // same in FP64, exactly: every cutoff is at least sqrt(r_cut_sq), the largest distance
     // the FP64 passes compute for a pair with r^2 <= r_cut_sq (sqrt is correctly rounded)
     int fuc, uc64;
@@ -133,7 +135,7 @@ struct AtomsView {
     double *vel, *frc; // [3][n_pad]
     double *rho, *Fe, *epot;
     double2 *dF2;
-    float4 *posf; // mixed precision: wrapped positions [angstrom], type in .w (or null)
+    float4 *posf; // mixed precision (or null): wrapped positions [angstrom], .w the type's bits
     float2 *dF2f; // mixed precision: F' [eV A^3], F'' [eV A^6]
     int *nbr, *n_up, *n_dn;
     int maxn;
@@ -260,8 +262,8 @@ __device__ __forceinline__ void ld6(const double *p, double c[6]) {
 // a pair-table bundle holds three functions (phi_ab, rho_a, rho_b).
 template <int IP> struct TabFmt {
     static constexpr int kF = IP == MDELAST_BSPLINE ? 12 : 6;
-    // FP32 records of the mixed-precision tables: a quintic's 6 coefficients and two pads in
-    // 32 bytes (one 256-bit load), a bspline's 12 in 48. The pair passes are bound by the L1's
+    // FP32 records of the mixed-precision tables: a quintic's 6 coefficients and two products
+    // of them in 32 bytes (one 256-bit load), a bspline's 12 coefficients in 48. The pair passes are bound by the L1's
     // data pipe, which serves about 32 scattered bytes per cycle however they are asked for
     // (force pass, wavefronts per gather of 32 lanes: 8 bytes 9, 16 bytes 16, 32 bytes 27), so
     // one record per function, read once per pair of one type, replaced a 72-byte bundle of

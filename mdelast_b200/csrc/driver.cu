@@ -222,7 +222,7 @@ struct mdelast_driver_s {
     int precision = MDELAST_PRECISION_FP64;
     float4 *d_posf = nullptr;
     float2 *d_dF2f = nullptr;
-    float *d_phf = nullptr, *d_rrf = nullptr;
+    float *d_phf = nullptr, *d_rrf = nullptr, *d_rdf = nullptr;
     void pass_density(bool obs, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED)
             launch_density_mx(obs, tpa_d, grid_d, s, A, T);
@@ -359,6 +359,7 @@ mdelast_driver_s::~mdelast_driver_s() {
     dfree(d_dF2f);
     dfree(d_phf);
     dfree(d_rrf);
+    dfree(d_rdf);
     dfree(d_stf);
     dfree(d_nbr);
     dfree(d_nup);
@@ -1341,6 +1342,26 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
             for (int k = 0; k < nri; ++k)
                 pack(fun(c0.eam[t]->rho, k), a3,
                      rrf.data() + (static_cast<size_t>(t) * nri + k) * kFf);
+        if (!bsp) { // the products of the records, rounded as the kernels round them
+            std::vector<float> rdf(rrf.size());
+            for (std::vector<float> *v : {&phf, &rrf})
+                for (size_t q = 0; q < v->size(); q += kFf) {
+                    float *c = v->data() + q;
+                    c[6] = 3.f * c[3];
+                    c[7] = 5.f * c[5];
+                }
+            for (size_t q = 0; q < rrf.size(); q += kFf) {
+                float const *c = rrf.data() + q;
+                float const d[8] = {c[1],       2.f * c[2], c[6],        4.f * c[4],
+                                    c[7],       6.f * c[3], 12.f * c[4], 20.f * c[5]};
+                std::copy(d, d + 8, rdf.data() + q);
+            }
+            TRY(dalloc(&d->d_rdf, rdf.size()));
+            if (cudaMemcpy(d->d_rdf, rdf.data(), sizeof(float) * rdf.size(),
+                           cudaMemcpyHostToDevice))
+                return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
+            T.rdf = d->d_rdf;
+        }
         TRY(dalloc(&d->d_phf, phf.size()));
         TRY(dalloc(&d->d_rrf, rrf.size()));
         if (cudaMemcpy(d->d_phf, phf.data(), sizeof(float) * phf.size(), cudaMemcpyHostToDevice) ||
@@ -1397,8 +1418,17 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         }
         for (int t = 0; t < nt; ++t)
             T.feam_rcut[t] = static_cast<float>(T.eam_rcut[t] / kAng);
+        T.frmin_max = 0.f;
+        for (int s = 0; s < npot; ++s)
+            T.frmin_max = std::max(T.frmin_max, T.fpot_rmin[s]);
+        for (int a = 0; a < nt; ++a) {
+            unsigned char b[kMaxTypes] = {};
+            for (int q = 0; q < nt; ++q)
+                b[q] = static_cast<unsigned char>(pair_slot(a, q));
+            std::memcpy(&T.slots[a], b, sizeof(b));
+        }
         float const rcf = static_cast<float>(rcut / kAng);
-        T.fuc = 1;
+        T.fuc = T.has_eam;
         for (int s = 0; s < npot; ++s)
             T.fuc &= T.fpot_rcut[s] >= rcf;
         if (T.has_eam)

@@ -18,33 +18,49 @@ namespace mdelast {
 
 namespace {
 
+// interval index, at most n - 1, and local coordinate; x >= 0
 __device__ __forceinline__ int tab_locate_f(float x, float inv_h, int n, float &t) {
     float const u = __fmul_rn(x, inv_h);
-    int i = 0;
-    if (u >= static_cast<float>(n))
-        i = n - 1;
-    else if (u > 0.f)
-        i = static_cast<int>(u);
-    t = __fsub_rn(u, static_cast<float>(i));
+    int const i = min(__float2int_rz(u), n - 1);
+    t = __fsub_rn(u, __int2float_rn(i));
     return i;
 }
 
-// The pair force is evaluated from both of its atoms, in different code paths of the
-// force pass; its arithmetic is written with explicit rounding (no contraction left to
-// the compiler) so that both evaluations give the same bits.
+// Quintic records (8 floats, TablesView::phf and rrf: c0..c5, 3 c3, 5 c5) and derivative records
+// (rdf: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5). The pair force is evaluated from
+// both of its atoms, in different code paths of the force pass; its arithmetic is written with
+// explicit rounding (no contraction left to the compiler) so that both evaluations, and those
+// from the staged tables, give the same bits.
+__device__ __forceinline__ float horner4(float t, float a, float b, float c, float d) {
+    return __fmaf_rn(t, __fmaf_rn(t, __fmaf_rn(t, d, c), b), a);
+}
 __device__ __forceinline__ float tabf_v(const float *c, float t) {
-    return c[0] + t * (c[1] + t * (c[2] + t * (c[3] + t * (c[4] + t * c[5]))));
+    return __fmaf_rn(t, __fmaf_rn(t, horner4(t, c[2], c[3], c[4], c[5]), c[1]), c[0]);
 }
 __device__ __forceinline__ float tabf_d1(const float *c, float t, float inv_h) {
-    float p = __fmul_rn(5.f, c[5]);
-    p = __fmaf_rn(t, p, __fmul_rn(4.f, c[4]));
-    p = __fmaf_rn(t, p, __fmul_rn(3.f, c[3]));
-    p = __fmaf_rn(t, p, __fmul_rn(2.f, c[2]));
-    p = __fmaf_rn(t, p, c[1]);
-    return __fmul_rn(p, inv_h);
+    return __fmul_rn(__fmaf_rn(t, horner4(t, __fmul_rn(2.f, c[2]), c[6], __fmul_rn(4.f, c[4]), c[7]),
+                               c[1]), inv_h);
 }
 __device__ __forceinline__ float tabf_d2(const float *c, float t, float inv_h2) {
-    return (2.f * c[2] + t * (6.f * c[3] + t * (12.f * c[4] + t * 20.f * c[5]))) * inv_h2;
+    return __fmul_rn(horner4(t, __fmul_rn(2.f, c[2]), __fmul_rn(2.f, c[6]), __fmul_rn(12.f, c[4]),
+                             __fmul_rn(4.f, c[7])), inv_h2);
+}
+__device__ __forceinline__ float tabd_d1(const float *d, float t, float inv_h) {
+    return __fmul_rn(__fmaf_rn(t, horner4(t, d[1], d[2], d[3], d[4]), d[0]), inv_h);
+}
+__device__ __forceinline__ float tabd_d2(const float *d, float t, float inv_h2) {
+    return __fmul_rn(horner4(t, d[1], d[5], d[6], d[7]), inv_h2);
+}
+// the derivative record of the coefficients c0..c5, as the host rounds it
+__device__ __forceinline__ void derivative_record(const float *c, float (&d)[8]) {
+    d[0] = c[1];
+    d[1] = __fmul_rn(2.f, c[2]);
+    d[2] = __fmul_rn(3.f, c[3]);
+    d[3] = __fmul_rn(4.f, c[4]);
+    d[4] = __fmul_rn(5.f, c[5]);
+    d[5] = __fmul_rn(6.f, c[3]);
+    d[6] = __fmul_rn(12.f, c[4]);
+    d[7] = __fmul_rn(20.f, c[5]);
 }
 
 // FP32 counterpart of tab_eval (device.cuh): QUINTIC interval data are the 6 quintic
@@ -66,7 +82,7 @@ __device__ __forceinline__ void tabf_eval(const float *p, float t, float inv_h, 
         if (ND2)
             d2 = cubicf_at(p + 8, t);
     } else {
-        float c[8]; // 6 coefficients, 2 pads
+        float c[8];
         ld256(p, c);
         if (NV)
             v = tabf_v(c, t);
@@ -85,29 +101,22 @@ __global__ void k_posf(AtomsView A) {
     if (i >= A.n_pad)
         return;
     int const r = A.rep_of[i];
-    if (r < 0)
-        return;
-    Replica const *R = A.rep + r;
-    double4 const c = A.crd[i];
-    A.posf[i] = make_float4(static_cast<float>((c.x - nint_ref(c.x)) * R->h[0] / kAng),
-                            static_cast<float>((c.y - nint_ref(c.y)) * R->h[1] / kAng),
-                            static_cast<float>((c.z - nint_ref(c.z)) * R->h[2] / kAng),
-                            static_cast<float>(c.w));
+    if (r >= 0)
+        A.posf[i] = position_f(A.crd[i], A.rep + r);
 }
 
-// One lane's share of an atom row in the density pass: branch-free body, two entries per
-// unrolled pass, as in the force pass; an entry beyond the cutoff adds zeros. UC: every
+// One lane's share of an atom row in the density pass: branch-free body, three entries per
+// unrolled pass (two spilled at 8 blocks per SM: 0.187 against 0.167 ms at 16 x 13,500 atoms); an entry beyond the cutoff adds zeros. UC: every
 // density cutoff is at least the pair cutoff (no per-type test).
 template <bool OBS, int TPA, int IP, typename IX, bool UC>
 __device__ __forceinline__ void dens_loop(AtomsView const &A, TablesView const &T, float4 pi,
                                           float3 L, float3 iL, PairRow<IX> const &row, int nu,
-                                          int ntot, int sub, double &rho, float (&g)[6],
-                                          float (&hv)[3]) {
+                                          int ntot, int sub, double &rho, float (&g)[6], float (&hv)[3]) {
     // the next partner's record and the list entry after it are loaded ahead, so the
     // entry's load does not delay the record's
     float4 pn = A.posf[sub < ntot ? row.at(list_slot(sub, nu, A.pmaxn)) : row.base];
     int jn = sub < ntot ? row.at(list_slot(min(sub + TPA, ntot - 1), nu, A.pmaxn)) : row.base;
-#pragma unroll 2
+#pragma unroll 3
     for (int kk = sub; kk < ntot; kk += TPA) {
         float4 const pj = pn;
         pn = A.posf[jn];
@@ -116,13 +125,13 @@ __device__ __forceinline__ void dens_loop(AtomsView const &A, TablesView const &
         float const r2 = min_image_f(pi, pj, L, iL, dx, dy, dz);
         float const idr = rsqrtf(r2);
         float const dr = __fmul_rn(r2, idr);
-        int const tj = static_cast<int>(pj.w);
+        int const tj = __float_as_int(pj.w);
         bool const in_cut = !(r2 > T.fr_cut_sq) && (UC || !(dr > T.feam_rcut[tj]));
         float t;
         int const k = tab_locate_f(dr, T.finv_hr, T.nri, t);
         float v = 0.f, d1 = 0.f, d2 = 0.f;
         tabf_eval<IP, true, OBS, false>(
-            T.rrf + (static_cast<size_t>(tj) * T.nri + k) * TabFmt<IP>::kFf, t, T.finv_hr,
+            T.rrf + static_cast<unsigned>(tj * T.nri + k) * TabFmt<IP>::kFf, t, T.finv_hr,
             T.finv_hr2, v, d1, d2);
         if (!in_cut) {
             v = 0.f;
@@ -182,15 +191,16 @@ __global__ void __launch_bounds__(kBlock, 8) k_density_mx(AtomsView A, TablesVie
         int ti = 0;
         if (valid) {
             float4 const pi = A.posf[i];
-            ti = static_cast<int>(pi.w);
+            ti = __float_as_int(pi.w);
             int const nu = A.pn_up[i], ntot = nu + A.pn_dn[i];
             PairRow<IX> const row = pair_row<IX>(A, i, R->atom_begin);
             // uniform cutoffs (every setfl potential): no per-function cutoff test
             if (T.fuc)
-                dens_loop<OBS, TPA, IP, IX, true>(A, T, pi, L, iL, row, nu, ntot, sub, rho, g, hv);
+                dens_loop<OBS, TPA, IP, IX, true>(A, T, pi, L, iL, row, nu, ntot, sub, rho, g,
+                                                  hv);
             else
                 dens_loop<OBS, TPA, IP, IX, false>(A, T, pi, L, iL, row, nu, ntot, sub, rho, g,
-                                                   hv);
+                                                  hv);
         }
         rho = group_sum<TPA>(rho);
         if (OBS) {
@@ -284,17 +294,19 @@ struct RowIn {
     float4 pi;
     float dFi, d2Fi;
     int ti;
+    uint2 slots; // byte b: the pair slot with type b
     float3 L, iL;
 };
 
-// The quintic coefficients of phi_s, rho_ti and rho_tj on interval k: from the staged
-// shared-memory copy (STAGED and k staged) or from the global records. Both hold the same
-// FP32 values, so the pair terms do not depend on where they were read. A pair of one type
-// reads its one rho once.
+// The quintic record of phi_s and the derivative records of rho_ti and rho_tj on interval k:
+// from the staged shared-memory copy (STAGED and k staged; c0..c5 alone, the products formed
+// here) or from the global records. Both give the same FP32 values, so the pair terms do not
+// depend on where they were read. A pair of one type reads its one rho once: dj is left
+// undefined and the caller takes the terms of di.
 template <bool STAGED>
 __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *stab, int s,
                                            int ti, int tj, int k, float (&cp)[8],
-                                           float (&ci)[8], float (&cj)[8]) {
+                                           float (&di)[8], float (&dj)[8]) {
     if (STAGED) {
         unsigned const q = static_cast<unsigned>(k - T.st_lo);
         if (q < static_cast<unsigned>(T.st_n)) {
@@ -303,6 +315,7 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
             const float2 *pp = reinterpret_cast<const float2 *>(b + s * n6);
             const float2 *pi = reinterpret_cast<const float2 *>(b + (T.npot + ti) * n6);
             const float2 *pj = reinterpret_cast<const float2 *>(b + (T.npot + tj) * n6);
+            float ci[6], cj[6];
 #pragma unroll
             for (int u = 0; u < 3; ++u) {
                 float2 const a = pp[u], c = pi[u], d = pj[u];
@@ -313,17 +326,17 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
                 cj[2 * u] = d.x;
                 cj[2 * u + 1] = d.y;
             }
+            cp[6] = __fmul_rn(3.f, cp[3]);
+            cp[7] = __fmul_rn(5.f, cp[5]);
+            derivative_record(ci, di);
+            derivative_record(cj, dj);
             return;
         }
     }
     constexpr int kFf = TabFmt<MDELAST_QUINTIC>::kFf;
-    ld256(T.phf + (static_cast<size_t>(s) * T.nri + k) * kFf, cp);
-    ld256(T.rrf + (static_cast<size_t>(ti) * T.nri + k) * kFf, ci);
-#pragma unroll
-    for (int u = 0; u < 6; ++u)
-        cj[u] = ci[u];
-    if (ti != tj)
-        ld256(T.rrf + (static_cast<size_t>(tj) * T.nri + k) * kFf, cj);
+    ld256(T.phf + static_cast<unsigned>(s * T.nri + k) * kFf, cp);
+    ld256(T.rdf + static_cast<unsigned>(ti * T.nri + k) * kFf, di);
+    ld256_if(ti != tj, T.rdf + static_cast<unsigned>(tj * T.nri + k) * kFf, dj);
 }
 
 // One lane's walk over list slots [s0, s1) of an atom row (slots of the upper half when
@@ -335,7 +348,7 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
                                              RowIn const &in, PairRow<IX> const &row, int n,
                                              int sub,
                                              double &fx, double &fy, double &fz, double &epot,
-                                             PairSums<OBS> &ps, bool &warn_rmin,
+                                             PairSums<OBS> &ps, float &dr_min,
                                              const float *stab = nullptr) {
     if (sub >= n)
         return;
@@ -348,11 +361,11 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
     float2 fn = A.dF2f[jn];
     jn = row.at(slot(min(sub + TPA, n - 1)));
     // The body has no branch: a pair beyond the cutoff is evaluated and its terms are
-    // replaced by zeros (the sums then gain +0 or -0, which changes no sum), and the next
-    // partner is always prefetched (the last one again at the end of the row). Two
-    // iterations then form one block of straight-line code, in which the second pair's
-    // gathers and table loads overlap the first pair's arithmetic.
-#pragma unroll 2
+    // replaced by zeros (the sums then gain +0 or -0, which changes no sum), the second rho of
+    // a two-type pair is a predicated load, and the next partner is always prefetched (the
+    // last one again at the end of the row). Not unrolled: one body fills the 128 registers of
+    // 4 blocks per SM, two spill (0.346 instead of 0.312 ms at 16 x 13,500 atoms).
+#pragma unroll 1
     for (int kk = sub; kk < n; kk += TPA) {
         float4 const pj = pn;
         float2 const dFj2 = fn;
@@ -364,50 +377,51 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         bool const in_cut = !(r2 > T.fr_cut_sq);
         float const idr = rsqrtf(r2);
         float const dr = __fmul_rn(r2, idr);
-        int const tj = static_cast<int>(pj.w);
-        int const ti = in.ti;
-        int const s = pair_slot(ti, tj);
+        dr_min = fminf(dr_min, dr);
+        int const ti = in.ti, tj = __float_as_int(pj.w);
+        int const s = __byte_perm(in.slots.x, in.slots.y, tj) & 0xff;
         float t;
         int const k = tab_locate_f(dr, T.finv_hr, T.nri, t);
         float V = 0.f, dV = 0.f, d2V = 0.f;
         float drho_i = 0.f, drho_j = 0.f, d2rho_i = 0.f, d2rho_j = 0.f;
-        if (in_cut && dr < T.fpot_rmin[s])
-            warn_rmin = true;
-        bool const eam_i = T.has_eam && (UC || !(dr > T.feam_rcut[ti]));
-        bool const eam_j = T.has_eam && (UC || !(dr > T.feam_rcut[tj]));
+        bool const eam_i = UC || (T.has_eam && !(dr > T.feam_rcut[ti]));
+        bool const eam_j = UC || (T.has_eam && !(dr > T.feam_rcut[tj]));
         if constexpr (IP == MDELAST_QUINTIC) {
             // the three functions' coefficients first (independent loads), then the math
-            float cp[8], ci[8], cj[8];
-            pair_coefs<STAGED>(T, stab, s, ti, tj, k, cp, ci, cj);
+            float cp[8], di[8], dj[8];
+            pair_coefs<STAGED>(T, stab, s, ti, tj, k, cp, di, dj);
             if (UC || !(dr > T.fpot_rcut[s])) {
                 V = tabf_v(cp, t);
                 dV = tabf_d1(cp, t, T.finv_hr);
                 if (OBS)
                     d2V = tabf_d2(cp, t, T.finv_hr2);
             }
-            if (eam_i) {
-                drho_i = tabf_d1(ci, t, T.finv_hr);
-                if (OBS)
-                    d2rho_i = tabf_d2(ci, t, T.finv_hr2);
+            bool const one = ti == tj;
+            drho_i = tabd_d1(di, t, T.finv_hr);
+            drho_j = tabd_d1(dj, t, T.finv_hr);
+            drho_j = one ? drho_i : drho_j;
+            if (OBS) {
+                d2rho_i = tabd_d2(di, t, T.finv_hr2);
+                d2rho_j = tabd_d2(dj, t, T.finv_hr2);
+                d2rho_j = one ? d2rho_i : d2rho_j;
             }
-            if (eam_j) {
-                drho_j = tabf_d1(cj, t, T.finv_hr);
-                if (OBS)
-                    d2rho_j = tabf_d2(cj, t, T.finv_hr2);
-            }
+            if (!eam_i)
+                drho_i = d2rho_i = 0.f;
+            if (!eam_j)
+                drho_j = d2rho_j = 0.f;
         } else {
             constexpr int kFf = TabFmt<IP>::kFf;
             if (UC || !(dr > T.fpot_rcut[s]))
-                tabf_eval<IP, true, true, OBS>(T.phf + (static_cast<size_t>(s) * T.nri + k) * kFf,
+                tabf_eval<IP, true, true, OBS>(T.phf + static_cast<unsigned>(s * T.nri + k) * kFf,
                                                t, T.finv_hr, T.finv_hr2, V, dV, d2V);
             float unused = 0.f;
             if (eam_i)
                 tabf_eval<IP, false, true, OBS>(
-                    T.rrf + (static_cast<size_t>(ti) * T.nri + k) * kFf, t, T.finv_hr,
+                    T.rrf + static_cast<unsigned>(ti * T.nri + k) * kFf, t, T.finv_hr,
                     T.finv_hr2, unused, drho_i, d2rho_i);
             if (eam_j)
                 tabf_eval<IP, false, true, OBS>(
-                    T.rrf + (static_cast<size_t>(tj) * T.nri + k) * kFf, t, T.finv_hr,
+                    T.rrf + static_cast<unsigned>(tj * T.nri + k) * kFf, t, T.finv_hr,
                     T.finv_hr2, unused, drho_j, d2rho_j);
         }
         float dedr = dV, X = 0.f, lap = 0.f;
@@ -415,7 +429,7 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
             X = d2V - dV * idr;
             lap = 2.f * (d2V + 2.f * dV * idr);
         }
-        if (T.has_eam) {
+        if (UC || T.has_eam) {
             float const dFj = dFj2.x, dFi = in.dFi;
             // the two cross terms rounded separately and added commutatively: the pair
             // force is the same, bit for bit, seen from either atom
@@ -438,17 +452,16 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         fx += static_cast<double>(__fmul_rn(sc, dx));
         fy += static_cast<double>(__fmul_rn(sc, dy));
         fz += static_cast<double>(__fmul_rn(sc, dz));
-        epot += static_cast<double>(0.5f * V);
+        epot += static_cast<double>(V); // halved at the end of the row
         if (UPPER) {
             float const xx = dx * dx, yy = dy * dy, zz = dz * dz;
             float const yz = dy * dz, xz = dx * dz, xy = dx * dy;
-            float const w = dedr * idr;
-            ps.sig_d[0] += static_cast<double>(w * xx);
-            ps.sig_d[1] += static_cast<double>(w * yy);
-            ps.sig_d[2] += static_cast<double>(w * zz);
-            ps.sig_o[0] += w * yz;
-            ps.sig_o[1] += w * xz;
-            ps.sig_o[2] += w * xy;
+            ps.sig_d[0] -= static_cast<double>(sc * xx); // sc = -dE/dr / r
+            ps.sig_d[1] -= static_cast<double>(sc * yy);
+            ps.sig_d[2] -= static_cast<double>(sc * zz);
+            ps.sig_o[0] -= sc * yz;
+            ps.sig_o[1] -= sc * xz;
+            ps.sig_o[2] -= sc * xy;
             if (OBS) {
                 X *= idr * idr;
                 float const Xxx = X * xx, Xyy = X * yy, Xzz = X * zz;
@@ -473,6 +486,24 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
     }
 }
 
+// whether one of this lane's pairs lies within the cutoff and below its r_min (potential.hpp:
+// 92-104 warns); walked only when the smallest distance of the row asks for it
+template <int TPA, typename IX>
+__device__ __forceinline__ bool below_rmin(AtomsView const &A, TablesView const &T,
+                                           RowIn const &in, PairRow<IX> const &row, int nu,
+                                           int nd, int sub) {
+    bool warn = false;
+    for (int half = 0; half < 2; ++half)
+        for (int k = sub; k < (half ? nd : nu); k += TPA) {
+            float4 const pj = A.posf[row.at(half ? A.pmaxn - 1 - k : k)];
+            float dx, dy, dz;
+            float const r2 = min_image_f(in.pi, pj, in.L, in.iL, dx, dy, dz);
+            float const dr = __fmul_rn(r2, rsqrtf(r2));
+            warn |= !(r2 > T.fr_cut_sq) && dr < T.fpot_rmin[pair_slot(in.ti, __float_as_int(pj.w))];
+        }
+    return warn;
+}
+
 // Force pass of md_driver.cpp:300-430 (with the closing kick) in mixed precision; see
 // k_force for the roles of the terms. Each atom row is walked in two loops, its upper
 // half (which also feeds the global sums) and its lower half, so the lanes of a warp do not
@@ -480,10 +511,12 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
 // over atoms go through warp_slots (31 and, at 4 lanes per atom, 4 exchanges) into two FP64
 // registers per lane; the virial is the trace of the Born stress.
 //
-// What bounds it: the L1 data pipe (61 % of its wavefront rate) and instruction issue
-// (53 %), at 4 blocks of 4 warps per SM. At 16 x 13,500 atoms and 4 lanes per atom 0.416 -> 0.362 ms:
-// the sums' shuffles and shared accumulators had been 19 % of the data pipe's work, the third
-// table function of one-type pairs another 20 %.
+// What bounds it: the L1 data pipe (about two thirds of its wavefront rate) with instruction
+// issue (about half) behind it, at 4 blocks of 4 warps per SM. At 16 x 13,500 atoms and 4 lanes per
+// atom: 0.416 ms when the sums' shuffles and shared accumulators were 19 % of the data pipe's
+// work and the third table function of one-type pairs another 20 %, 0.362 ms without them, 0.345 with
+// even row halves, 0.312 with the products of the coefficients in the table records, the r_min test
+// once per row, pair slots from a byte table and no unrolling.
 //
 // STAGED: the block first copies the staged quintic tables (T.stf, T.st_bytes, about 180 KB
 // for a two-element alloy) into dynamic shared memory and reads every staged interval from
@@ -495,7 +528,7 @@ constexpr int kBlockStaged = kStagedBlock;
 
 template <bool OBS, bool KICK, int TPA, int IP, bool STAGED, typename IX,
           int NB = STAGED ? kBlockStaged : kBlock>
-__global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
+__global__ void __launch_bounds__(NB, STAGED ? 1 : 4) k_force_mx(AtomsView A, TablesView T) {
     chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
@@ -528,27 +561,29 @@ __global__ void __launch_bounds__(NB) k_force_mx(AtomsView A, TablesView T) {
         in.ti = 0;
         if (valid) {
             in.pi = A.posf[i];
-            in.ti = static_cast<int>(in.pi.w);
+            in.ti = __float_as_int(in.pi.w);
+            in.slots = T.slots[in.ti];
             float2 const dFi2 = T.has_eam ? A.dF2f[i] : make_float2(0.f, 0.f);
             in.dFi = dFi2.x;
             in.d2Fi = OBS ? dFi2.y : 0.f;
             int const nu = A.pn_up[i], nd = A.pn_dn[i];
             PairRow<IX> const row = pair_row<IX>(A, i, R->atom_begin);
-            bool warn_rmin = false;
+            float dr_min = 3.4e38f; // of this lane's pairs
             PairSums<OBS> ps;
             // uniform cutoffs (every setfl potential): no per-function cutoff tests
             if (T.fuc) {
                 force_row_mx<OBS, true, TPA, IP, STAGED, IX, true>(
-                    A, T, in, row, nu, sub, fx, fy, fz, epot, ps, warn_rmin, stab);
+                    A, T, in, row, nu, sub, fx, fy, fz, epot, ps, dr_min, stab);
                 force_row_mx<OBS, false, TPA, IP, STAGED, IX, true>(
-                    A, T, in, row, nd, sub, fx, fy, fz, epot, ps, warn_rmin, stab);
+                    A, T, in, row, nd, sub, fx, fy, fz, epot, ps, dr_min, stab);
             } else {
                 force_row_mx<OBS, true, TPA, IP, STAGED, IX, false>(
-                    A, T, in, row, nu, sub, fx, fy, fz, epot, ps, warn_rmin, stab);
+                    A, T, in, row, nu, sub, fx, fy, fz, epot, ps, dr_min, stab);
                 force_row_mx<OBS, false, TPA, IP, STAGED, IX, false>(
-                    A, T, in, row, nd, sub, fx, fy, fz, epot, ps, warn_rmin, stab);
+                    A, T, in, row, nd, sub, fx, fy, fz, epot, ps, dr_min, stab);
             }
-            if (warn_rmin)
+            epot *= 0.5;
+            if (dr_min < T.frmin_max && below_rmin<TPA>(A, T, in, row, nu, nd, sub))
                 status_or(A.rep + r, MDELAST_WARN_RMIN);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {

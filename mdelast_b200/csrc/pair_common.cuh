@@ -21,22 +21,49 @@ __device__ __forceinline__ void ld256(const float *p, float (&v)[8]) {
         : "l"(p));
 }
 
-// minimum image of pi - pj in a box of edges L (positions wrapped into [-L/2, L/2))
+// The same where `on`; elsewhere v is left undefined.
+__device__ __forceinline__ void ld256_if(bool on, const float *p, float (&v)[8]) {
+    asm("{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %9, 0;\n\t"
+        "@q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+        "}"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+          "=f"(v[7])
+        : "l"(p), "r"(static_cast<int>(on)));
+}
+
+// Positions of the mixed passes (AtomsView::posf) from the FP64 scaled coordinates and the box:
+// wrapped, in angstrom, the type's bits in .w.
+__device__ __forceinline__ float4 position_f(double4 c, Replica const *R) {
+    double const u = 1e8; // cm -> angstrom
+    return make_float4(static_cast<float>((c.x - nint_ref(c.x)) * R->h[0] * u),
+                       static_cast<float>((c.y - nint_ref(c.y)) * R->h[1] * u),
+                       static_cast<float>((c.z - nint_ref(c.z)) * R->h[2] * u),
+                       __int_as_float(static_cast<int>(c.w)));
+}
+// rint(x) for |x| < 2^22 by adding 1.5 * 2^23: two FP32 additions instead of a conversion on the
+// narrow unit that also takes the square roots and the conversions to FP64
+__device__ __forceinline__ float round_small(float x) {
+    return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f);
+}
+// minimum image of pi - pj in a box of edges L (positions wrapped into [-L/2, L/2)) and its
+// square. Every operation is an odd function: the image seen from j is the negative, bit for bit.
 __device__ __forceinline__ float min_image_f(float4 pi, float4 pj, float3 L, float3 iL,
                                              float &dx, float &dy, float &dz) {
     dx = __fsub_rn(pi.x, pj.x);
     dy = __fsub_rn(pi.y, pj.y);
     dz = __fsub_rn(pi.z, pj.z);
-    dx = __fmaf_rn(-L.x, rintf(__fmul_rn(dx, iL.x)), dx);
-    dy = __fmaf_rn(-L.y, rintf(__fmul_rn(dy, iL.y)), dy);
-    dz = __fmaf_rn(-L.z, rintf(__fmul_rn(dz, iL.z)), dz);
+    dx = __fmaf_rn(-L.x, round_small(__fmul_rn(dx, iL.x)), dx);
+    dy = __fmaf_rn(-L.y, round_small(__fmul_rn(dy, iL.y)), dy);
+    dz = __fmaf_rn(-L.z, round_small(__fmul_rn(dz, iL.z)), dz);
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
 __device__ __forceinline__ void box_f(Replica const *R, float3 &L, float3 &iL) {
-    L = make_float3(static_cast<float>(R->h[0] / kAng), static_cast<float>(R->h[1] / kAng),
-                    static_cast<float>(R->h[2] / kAng));
-    iL = make_float3(1.f / L.x, 1.f / L.y, 1.f / L.z);
+    L = make_float3(static_cast<float>(R->h[0] * 1e8), static_cast<float>(R->h[1] * 1e8),
+                    static_cast<float>(R->h[2] * 1e8));
+    iL = make_float3(__frcp_rn(L.x), __frcp_rn(L.y), __frcp_rn(L.z));
 }
 
 // The warp's totals of N per-lane values, one total per lane: at each butterfly level a

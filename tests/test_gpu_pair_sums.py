@@ -52,3 +52,14 @@ def test_mixed(types, edges, vacancies, tpa):
         g.integrate()
         o.integrate()
     _check(g, o, 2e-5, 1e-6, 1e-4)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("rmin_ang,warns", [(1.0, False), (2.45, True)])
+def test_rmin_warning(precision, rmin_ang, warns):
+    """The r_min warning, which the mixed pass decides from each row's smallest distance."""
+    t = generic_tables(2)
+    t.rmin_fatal = rmin_ang * 1e-8
+    c = generic_case(t, (5, 5, 5), 7)
+    g, o = gpu(c, precision=precision), oracle(c)
+    assert g.status == o.status() and (g.status != 0) == warns
