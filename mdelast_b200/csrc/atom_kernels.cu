@@ -1200,64 +1200,60 @@ __global__ void k_sub_invalidate(AtomsView A) {
 
 // ------------------------------------------------------------------------------------
 // Readout of one per-atom field in the C-ABI layout (x, y, z interleaved per atom) for
-// replica r, applying the deferred velocity factor.
+// replica r, applying the deferred velocity factor. One value per thread: `out` is pinned host memory,
+// and a warp's stores are contiguous.
 
 __global__ void k_readout(AtomsView A, TablesView T, int r, int field, double *out,
                           const double *pos0, int stepped) {
     Replica const *R = A.rep + r;
-    int const n = R->n_atoms;
-    int const a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n)
+    int const e = blockIdx.x * blockDim.x + threadIdx.x;
+    bool const vec = field <= MDELAST_ATOM_FORCES;
+    int const a = vec ? e / 3 : e, k = vec ? e - 3 * a : 0;
+    if (a >= R->n_atoms)
         return;
     int const i = R->atom_begin + a;
-    size_t const np = A.n_pad;
+    size_t const at = static_cast<size_t>(k) * A.n_pad + i; // component k of an SoA field
+    auto coord = [&]() {
+        double4 const c = A.crd[i];
+        return k == 0 ? c.x : (k == 1 ? c.y : c.z);
+    };
+    double v = 0.;
     switch (field) {
-    case MDELAST_ATOM_POSITIONS: {
+    case MDELAST_ATOM_POSITIONS:
         if (!stepped) {
-            out[3 * a] = pos0[3 * a];
-            out[3 * a + 1] = pos0[3 * a + 1];
-            out[3 * a + 2] = pos0[3 * a + 2];
+            v = pos0[e];
         } else {
-            double4 const c = A.crd[i];
-            out[3 * a] = __dmul_rn(__dadd_rn(c.x, -nint_ref(c.x)), R->h_pos[0]);
-            out[3 * a + 1] = __dmul_rn(__dadd_rn(c.y, -nint_ref(c.y)), R->h_pos[1]);
-            out[3 * a + 2] = __dmul_rn(__dadd_rn(c.z, -nint_ref(c.z)), R->h_pos[2]);
+            double const c = coord();
+            v = __dmul_rn(__dadd_rn(c, -nint_ref(c)), R->h_pos[k]);
         }
         break;
-    }
-    case MDELAST_ATOM_COORDINATES: {
-        double4 const c = A.crd[i];
-        out[3 * a] = c.x;
-        out[3 * a + 1] = c.y;
-        out[3 * a + 2] = c.z;
+    case MDELAST_ATOM_COORDINATES:
+        v = coord();
         break;
-    }
     case MDELAST_ATOM_VELOCITIES:
-        out[3 * a] = A.vel[i] * R->vscale;
-        out[3 * a + 1] = A.vel[np + i] * R->vscale;
-        out[3 * a + 2] = A.vel[2 * np + i] * R->vscale;
+        v = A.vel[at] * R->vscale;
         break;
     case MDELAST_ATOM_FORCES:
-        out[3 * a] = A.frc[i];
-        out[3 * a + 1] = A.frc[np + i];
-        out[3 * a + 2] = A.frc[2 * np + i];
+        v = A.frc[at];
         break;
     case MDELAST_ATOM_RHO:
-        out[a] = A.rho[i];
+        v = A.rho[i];
         break;
     case MDELAST_ATOM_EPOT:
-        out[a] = A.epot[i];
+        v = A.epot[i];
         break;
     case MDELAST_ATOM_EKIN: {
+        size_t const np = A.n_pad;
         double const m = T.mass[static_cast<int>(A.crd[i].w)];
         double const vx = A.vel[i] * R->vscale, vy = A.vel[np + i] * R->vscale,
                      vz = A.vel[2 * np + i] * R->vscale;
-        out[a] = 0.5 * m * (vx * vx + vy * vy + vz * vz);
+        v = 0.5 * m * (vx * vx + vy * vy + vz * vz);
         break;
     }
     default:
-        break;
+        return;
     }
+    out[e] = v;
 }
 
 // The reference-format half list of replica r: for each atom its partners j > i, in

@@ -60,9 +60,14 @@ int own_pool(int dev, cudaMemPool_t *out) {
     return MDELAST_OK;
 }
 
-// Allocated, zeroed and complete on return (the driver's own stream does not order against
-// the legacy stream the pool is used on).
-template <typename T> int dalloc(T **p, size_t n) {
+// Allocated and zeroed in the order of the legacy stream, which the pool is used on. The driver's
+// own stream does not order against it: allocs_done() comes before that stream's first use of the
+// buffers (a creation makes some forty; a wait for each took 0.5 ms).
+int allocs_done() {
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
+    return MDELAST_OK;
+}
+template <typename T> int dalloc_later(T **p, size_t n) {
     size_t const bytes = sizeof(T) * (n > 0 ? n : 1);
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -71,17 +76,75 @@ template <typename T> int dalloc(T **p, size_t n) {
         return rc;
     CK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, pool, cudaStreamLegacy));
     CK(cudaMemsetAsync(*p, 0, bytes, cudaStreamLegacy));
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
     return MDELAST_OK;
 }
+// ... complete on return
+template <typename T> int dalloc(T **p, size_t n) {
+    if (int rc = dalloc_later(p, n))
+        return rc;
+    return allocs_done();
+}
 
-// Returned to the pool once all work on the device has finished, as cudaFree would wait.
-template <typename T> void dfree(T *&p) {
-    if (p) {
-        cudaDeviceSynchronize();
+// Returned to the pool; the caller has waited for all work on the device, as cudaFree would.
+template <typename T> void dfree_idle(T *&p) {
+    if (p)
         cudaFreeAsync(p, cudaStreamLegacy);
-    }
     p = nullptr;
+}
+// ... waiting here
+template <typename T> void dfree(T *&p) {
+    if (p)
+        cudaDeviceSynchronize();
+    dfree_idle(p);
+}
+
+// Pinned host blocks of drivers (observables, atom readouts), kept for the next driver: pinning
+// and unpinning pages takes a fraction of a millisecond each. At most kPinnedKeep blocks and
+// kPinnedKeepBytes are kept, each used by one driver at a time; mdelast_release_cached_memory()
+// frees them.
+struct PinnedBlock {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+constexpr size_t kPinnedKeep = 16, kPinnedKeepBytes = 64u << 20;
+std::mutex g_pinned_mutex;
+std::vector<PinnedBlock> g_pinned;
+
+int pinned_take(PinnedBlock &b, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mutex);
+        size_t best = g_pinned.size();
+        for (size_t k = 0; k < g_pinned.size(); ++k)
+            if (g_pinned[k].bytes >= bytes && g_pinned[k].bytes <= 4 * bytes + 65536 &&
+                (best == g_pinned.size() || g_pinned[k].bytes < g_pinned[best].bytes))
+                best = k;
+        if (best < g_pinned.size()) {
+            b = g_pinned[best];
+            g_pinned.erase(g_pinned.begin() + static_cast<long>(best));
+            return MDELAST_OK;
+        }
+    }
+    CK(cudaHostAlloc(&b.p, bytes, cudaHostAllocPortable));
+    b.bytes = bytes;
+    return MDELAST_OK;
+}
+// call with no device work left that uses the block
+void pinned_give(PinnedBlock &b) {
+    if (!b.p)
+        return;
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mutex);
+        size_t kept = 0;
+        for (PinnedBlock const &q : g_pinned)
+            kept += q.bytes;
+        if (g_pinned.size() < kPinnedKeep && kept + b.bytes <= kPinnedKeepBytes) {
+            g_pinned.push_back(b);
+            b = PinnedBlock{};
+            return;
+        }
+    }
+    cudaFreeHost(b.p);
+    b = PinnedBlock{};
 }
 
 // Host staging of a creation's atom uploads: pinned, kept from one creation to the next (a
@@ -286,7 +349,7 @@ struct mdelast_driver_s {
     int *d_cell_rep = nullptr;
     std::vector<int> cell_rep_host; // replica of each cell, as uploaded
     double *d_rb = nullptr, *d_Ft = nullptr;
-    double *d_pos0 = nullptr, *d_out = nullptr;
+    double *d_pos0 = nullptr;
     int *d_tmp_i = nullptr;
     size_t tmp_i_cap = 0;
 
@@ -305,7 +368,9 @@ struct mdelast_driver_s {
 
     AtomsView A{};
     TablesView T{};
-    mdelast_observables *h_obs = nullptr; // pinned, n_rep entries
+    mdelast_observables *h_obs = nullptr; // pinned, n_rep entries (obs_block)
+    // pinned: the observables, and one replica's field of an atom readout (taken at the first one)
+    PinnedBlock obs_block, out_block;
     cudaEvent_t ev_step = nullptr;
     cudaGraphExec_t graph[8] = {}; // [4 * last + 2 * rebuild + obs]
     unsigned long long host_cycle = 0; // steps launched (the reference's cycle counter)
@@ -344,52 +409,52 @@ mdelast_driver_s::~mdelast_driver_s() {
             cudaGraphExecDestroy(g);
     if (ev_step)
         cudaEventDestroy(ev_step);
-    if (h_obs)
-        cudaFreeHost(h_obs);
-    dfree(d_rep);
-    dfree(d_rep_of);
-    dfree(d_crd);
-    dfree(d_vel);
-    dfree(d_frc);
-    dfree(d_rho);
-    dfree(d_Fe);
-    dfree(d_epot);
-    dfree(d_dF2);
-    dfree(d_posf);
-    dfree(d_dF2f);
-    dfree(d_phf);
-    dfree(d_rrf);
-    dfree(d_rdf);
-    dfree(d_stf);
-    dfree(d_nbr);
-    dfree(d_nup);
-    dfree(d_ndn);
-    dfree(d_pnbr);
-    dfree(d_pnbr16);
-    dfree(d_pnup);
-    dfree(d_pndn);
-    dfree(d_crd_ref);
-    dfree(d_pd);
-    dfree(d_pf);
-    dfree(d_red);
-    dfree(d_cell_count);
-    dfree(d_cell_atoms);
-    dfree(d_cell_rep);
-    dfree(d_max_count);
-    dfree(d_halt);
-    dfree(d_rb);
-    dfree(d_Ft);
-    dfree(d_pos0);
-    dfree(d_out);
-    dfree(d_tmp_i);
-    dfree(d_dblk_rep);
-    dfree(d_fblk_rep);
-    dfree(d_ring);
-    dfree(d_rg);
-    dfree(d_gr);
-    dfree(d_grp);
-    dfree(d_gr_counts);
-    dfree(d_gr_ntype);
+    cudaDeviceSynchronize(); // once for all buffers
+    pinned_give(obs_block);
+    pinned_give(out_block);
+    dfree_idle(d_rep);
+    dfree_idle(d_rep_of);
+    dfree_idle(d_crd);
+    dfree_idle(d_vel);
+    dfree_idle(d_frc);
+    dfree_idle(d_rho);
+    dfree_idle(d_Fe);
+    dfree_idle(d_epot);
+    dfree_idle(d_dF2);
+    dfree_idle(d_posf);
+    dfree_idle(d_dF2f);
+    dfree_idle(d_phf);
+    dfree_idle(d_rrf);
+    dfree_idle(d_rdf);
+    dfree_idle(d_stf);
+    dfree_idle(d_nbr);
+    dfree_idle(d_nup);
+    dfree_idle(d_ndn);
+    dfree_idle(d_pnbr);
+    dfree_idle(d_pnbr16);
+    dfree_idle(d_pnup);
+    dfree_idle(d_pndn);
+    dfree_idle(d_crd_ref);
+    dfree_idle(d_pd);
+    dfree_idle(d_pf);
+    dfree_idle(d_red);
+    dfree_idle(d_cell_count);
+    dfree_idle(d_cell_atoms);
+    dfree_idle(d_cell_rep);
+    dfree_idle(d_max_count);
+    dfree_idle(d_halt);
+    dfree_idle(d_rb);
+    dfree_idle(d_Ft);
+    dfree_idle(d_pos0);
+    dfree_idle(d_tmp_i);
+    dfree_idle(d_dblk_rep);
+    dfree_idle(d_fblk_rep);
+    dfree_idle(d_ring);
+    dfree_idle(d_rg);
+    dfree_idle(d_gr);
+    dfree_idle(d_grp);
+    dfree_idle(d_gr_counts);
+    dfree_idle(d_gr_ntype);
     if (stream)
         cudaStreamDestroy(stream);
 }
@@ -1034,6 +1099,12 @@ int mdelast_release_cached_memory(int32_t device) {
         g_stage = nullptr;
         g_stage_bytes = 0;
     }
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mutex);
+        for (PinnedBlock const &b : g_pinned)
+            cudaFreeHost(b.p);
+        g_pinned.clear();
+    }
     return MDELAST_OK;
 }
 
@@ -1279,8 +1350,8 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         for (int k = 0; k < nfi; ++k)
             std::memcpy(Ft.data() + (static_cast<size_t>(t) * nfi + k) * kF,
                         fun(c0.eam[t]->F, k), sizeof(double) * kF);
-    TRY(dalloc(&d->d_rb, rb.size()));
-    TRY(dalloc(&d->d_Ft, Ft.size()));
+    TRY(dalloc_later(&d->d_rb, rb.size()));
+    TRY(dalloc_later(&d->d_Ft, Ft.size()));
     if (cudaMemcpy(d->d_rb, rb.data(), sizeof(double) * rb.size(), cudaMemcpyHostToDevice) ||
         cudaMemcpy(d->d_Ft, Ft.data(), sizeof(double) * Ft.size(), cudaMemcpyHostToDevice))
         return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
@@ -1356,14 +1427,14 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
                                     c[7],       6.f * c[3], 12.f * c[4], 20.f * c[5]};
                 std::copy(d, d + 8, rdf.data() + q);
             }
-            TRY(dalloc(&d->d_rdf, rdf.size()));
+            TRY(dalloc_later(&d->d_rdf, rdf.size()));
             if (cudaMemcpy(d->d_rdf, rdf.data(), sizeof(float) * rdf.size(),
                            cudaMemcpyHostToDevice))
                 return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
             T.rdf = d->d_rdf;
         }
-        TRY(dalloc(&d->d_phf, phf.size()));
-        TRY(dalloc(&d->d_rrf, rrf.size()));
+        TRY(dalloc_later(&d->d_phf, phf.size()));
+        TRY(dalloc_later(&d->d_rrf, rrf.size()));
         if (cudaMemcpy(d->d_phf, phf.data(), sizeof(float) * phf.size(), cudaMemcpyHostToDevice) ||
             cudaMemcpy(d->d_rrf, rrf.data(), sizeof(float) * rrf.size(), cudaMemcpyHostToDevice))
             return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
@@ -1395,7 +1466,7 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
                         else
                             pack(fun(c0.eam[q - npot]->rho, static_cast<int>(lo + k)), a3, o);
                     }
-                TRY(dalloc(&d->d_stf, stf.size()));
+                TRY(dalloc_later(&d->d_stf, stf.size()));
                 if (cudaMemcpy(d->d_stf, stf.data(), sizeof(float) * stf.size(),
                                cudaMemcpyHostToDevice))
                     return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
@@ -1452,11 +1523,11 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
             off += c.n_rg;
             max_slots = std::max(max_slots, gr_count_slots(c.n_rg, nt));
         }
-        TRY(dalloc(&d->d_rg, rg_all.size()));
-        TRY(dalloc(&d->d_gr, rg_all.size()));
-        TRY(dalloc(&d->d_grp, rg_all.size() * static_cast<size_t>(npot)));
-        TRY(dalloc(&d->d_gr_counts, max_slots));
-        TRY(dalloc(&d->d_gr_ntype, static_cast<size_t>(nt)));
+        TRY(dalloc_later(&d->d_rg, rg_all.size()));
+        TRY(dalloc_later(&d->d_gr, rg_all.size()));
+        TRY(dalloc_later(&d->d_grp, rg_all.size() * static_cast<size_t>(npot)));
+        TRY(dalloc_later(&d->d_gr_counts, max_slots));
+        TRY(dalloc_later(&d->d_gr_ntype, static_cast<size_t>(nt)));
         if (cudaMemcpy(d->d_rg, rg_all.data(), sizeof(double) * rg_all.size(),
                        cudaMemcpyHostToDevice))
             return bail(fail(MDELAST_ERR_CUDA, "rg upload failed"));
@@ -1496,50 +1567,47 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
     std::vector<int> dmap, fmap;
     d->grid_d = deal_blocks(reps, d->tpa_d, true, dmap);
     d->grid_f = deal_blocks(reps, d->tpa_f, false, fmap);
-    TRY(dalloc(&d->d_dblk_rep, dmap.size()));
-    TRY(dalloc(&d->d_fblk_rep, fmap.size()));
+    TRY(dalloc_later(&d->d_dblk_rep, dmap.size()));
+    TRY(dalloc_later(&d->d_fblk_rep, fmap.size()));
     d->cap_dmap = dmap.size();
     d->cap_fmap = fmap.size();
-    TRY(dalloc(&d->d_rep, static_cast<size_t>(n_rep)));
+    TRY(dalloc_later(&d->d_rep, static_cast<size_t>(n_rep)));
     if (cudaMemcpy(d->d_rep, R.data(), sizeof(Replica) * n_rep, cudaMemcpyHostToDevice) ||
         cudaMemcpy(d->d_dblk_rep, dmap.data(), sizeof(int) * dmap.size(), cudaMemcpyHostToDevice) ||
         cudaMemcpy(d->d_fblk_rep, fmap.data(), sizeof(int) * fmap.size(), cudaMemcpyHostToDevice))
         return bail(fail(MDELAST_ERR_CUDA, "state upload failed"));
 
     // ---- atoms
-    TRY(dalloc(&d->d_rep_of, np));
-    TRY(dalloc(&d->d_crd, np));
-    TRY(dalloc(&d->d_vel, 3 * static_cast<size_t>(np)));
-    TRY(dalloc(&d->d_frc, 3 * static_cast<size_t>(np)));
-    TRY(dalloc(&d->d_rho, np));
-    TRY(dalloc(&d->d_Fe, np));
-    TRY(dalloc(&d->d_epot, np));
-    TRY(dalloc(&d->d_dF2, np));
+    TRY(dalloc_later(&d->d_rep_of, np));
+    TRY(dalloc_later(&d->d_crd, np));
+    TRY(dalloc_later(&d->d_vel, 3 * static_cast<size_t>(np)));
+    TRY(dalloc_later(&d->d_frc, 3 * static_cast<size_t>(np)));
+    TRY(dalloc_later(&d->d_rho, np));
+    TRY(dalloc_later(&d->d_Fe, np));
+    TRY(dalloc_later(&d->d_epot, np));
+    TRY(dalloc_later(&d->d_dF2, np));
     if (c0.precision == MDELAST_PRECISION_MIXED) {
-        TRY(dalloc(&d->d_posf, np));
-        TRY(dalloc(&d->d_dF2f, np));
+        TRY(dalloc_later(&d->d_posf, np));
+        TRY(dalloc_later(&d->d_dF2f, np));
     }
-    TRY(dalloc(&d->d_nup, np));
-    TRY(dalloc(&d->d_ndn, np));
-    TRY(dalloc(&d->d_pd, static_cast<size_t>(d->grid_d) * D_NSUM));
-    TRY(dalloc(&d->d_pf, static_cast<size_t>(d->grid_f) * F_NSUM));
+    TRY(dalloc_later(&d->d_nup, np));
+    TRY(dalloc_later(&d->d_ndn, np));
+    TRY(dalloc_later(&d->d_pd, static_cast<size_t>(d->grid_d) * D_NSUM));
+    TRY(dalloc_later(&d->d_pf, static_cast<size_t>(d->grid_f) * F_NSUM));
     d->cap_pd = static_cast<size_t>(d->grid_d) * D_NSUM;
     d->cap_pf = static_cast<size_t>(d->grid_f) * F_NSUM;
     int max_chunks = 1;
     for (Replica const *x : reps)
         max_chunks = std::max(max_chunks, (std::max(x->dblk_n, x->fblk_n) + kChunk - 1) / kChunk);
-    TRY(dalloc(&d->d_red, static_cast<size_t>(n_rep) * max_chunks * 64));
+    TRY(dalloc_later(&d->d_red, static_cast<size_t>(n_rep) * max_chunks * 64));
     d->cap_red = static_cast<size_t>(n_rep) * max_chunks * 64;
-    TRY(dalloc(&d->d_max_count, 2));
-    TRY(dalloc(&d->d_halt, 1));
-    TRY(dalloc(&d->d_pos0, 3 * static_cast<size_t>(n_total)));
-    int max_n = 0;
-    for (int r = 0; r < n_rep; ++r)
-        max_n = std::max(max_n, count[r]);
-    TRY(dalloc(&d->d_out, 3 * static_cast<size_t>(max_n)));
+    TRY(dalloc_later(&d->d_max_count, 2));
+    TRY(dalloc_later(&d->d_halt, 1));
+    TRY(dalloc_later(&d->d_pos0, 3 * static_cast<size_t>(n_total)));
     d->pos0_off.assign(static_cast<size_t>(n_rep), 0);
     for (int r = 1; r < n_rep; ++r)
         d->pos0_off[r] = d->pos0_off[r - 1] + 3L * count[r - 1];
+    TRY(allocs_done());
     if (cudaMemcpyAsync(d->d_rep_of, rep_of, b_rep, cudaMemcpyHostToDevice, d->stream) ||
         cudaMemcpyAsync(d->d_crd, crd, b_crd, cudaMemcpyHostToDevice, d->stream) ||
         cudaMemcpyAsync(d->d_vel, vel, b_vel, cudaMemcpyHostToDevice, d->stream) ||
@@ -1547,9 +1615,11 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         cudaStreamSynchronize(d->stream))
         return bail(fail(MDELAST_ERR_CUDA, "atom upload failed"));
     stage_lock.unlock(); // the staging is free for the next creation
-    if (cudaMallocHost(&d->h_obs, sizeof(mdelast_observables) * n_rep) ||
-        cudaEventCreateWithFlags(&d->ev_step, cudaEventDisableTiming))
-        return bail(fail(MDELAST_ERR_CUDA, "host staging allocation failed"));
+    TRY(pinned_take(d->obs_block, sizeof(mdelast_observables) * n_rep));
+    d->h_obs = static_cast<mdelast_observables *>(d->obs_block.p);
+    std::memset(static_cast<void *>(d->h_obs), 0, sizeof(mdelast_observables) * n_rep);
+    if (cudaEventCreateWithFlags(&d->ev_step, cudaEventDisableTiming))
+        return bail(fail(MDELAST_ERR_CUDA, "event creation failed"));
 
     AtomsView &A = d->A;
     A.n_pad = np;
@@ -1801,14 +1871,22 @@ static int get_atoms_r(mdelast_driver *d, int r, int32_t field, double *out) {
     CK(cudaSetDevice(d->device));
     if (int rc = d->wait_step())
         return rc;
+    // the kernel writes the field straight into pinned memory
     int const N = d->rep_count[r];
-    k_readout<<<(N + 255) / 256, 256, 0, d->stream>>>(d->A, d->T, r, field, d->d_out,
-                                                      d->d_pos0 + d->pos0_off[r],
-                                                      d->stepped ? 1 : 0);
-    CK(cudaGetLastError());
     size_t const n = field <= MDELAST_ATOM_FORCES ? 3 * static_cast<size_t>(N) : N;
-    CK(cudaMemcpyAsync(out, d->d_out, sizeof(double) * n, cudaMemcpyDeviceToHost, d->stream));
+    if (!d->out_block.p) {
+        size_t most = 0;
+        for (int c : d->rep_count)
+            most = std::max(most, static_cast<size_t>(c));
+        if (int rc = pinned_take(d->out_block, 3 * sizeof(double) * most))
+            return rc;
+    }
+    double *const host = static_cast<double *>(d->out_block.p);
+    k_readout<<<static_cast<unsigned>((n + 255) / 256), 256, 0, d->stream>>>(
+        d->A, d->T, r, field, host, d->d_pos0 + d->pos0_off[r], d->stepped ? 1 : 0);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(d->stream));
+    std::memcpy(out, host, sizeof(double) * n);
     return MDELAST_OK;
 }
 
