@@ -530,13 +530,30 @@ __global__ void k_nbr_build(AtomsView A, int cells_done) {
 // so those per-atom Born and Laplacian terms (md_driver.cpp:410-419) are formed here and
 // g, h are never stored.
 
+// r and 1/r from r^2. UC (one cutoff for every function): both from one reciprocal square root (1
+// ulp; r is then within 2 ulp), about 20 FP64 operations less than a square root and a division;
+// else r correctly rounded, as the per-function cutoffs compare it. Two atoms in one place:
+// r = 0, 1/r infinite.
+template <bool UC>
+__device__ __forceinline__ void pair_distance(double r2, double &dr, double &idr) {
+    if (UC) {
+        idr = rsqrt(r2);
+        dr = r2 == 0. ? 0. : r2 * idr;
+    } else {
+        dr = sqrt(r2);
+        idr = 1. / dr;
+    }
+}
+
 // The atom's terms of the block's FP64 sums (embedding energy, the per-atom Born term
 // F''_i g_i g_i^T and the Laplacian term) are formed in every lane of the atom and spread
 // over the lanes by warp_slots, one running sum per lane; with 23 warp sums per atom group
 // into shared accumulators the pass took 0.0397 instead of 0.0306 ms on 13,500 atoms (16 lanes
-// per atom).
+// per atom; 0.0266 ms with 8 lanes and pair_distance). Bound by the L1 data pipe (75 % of its
+// wavefront rate, FP64 pipe 39 %). 6 blocks per SM: 5 and 7 are slower by 3 and 5 % on 108,000
+// atoms.
 template <bool OBS, int TPA, int IP, typename IX>
-__global__ void __launch_bounds__(kBlock) k_density(AtomsView A, TablesView T) {
+__global__ void __launch_bounds__(kBlock, 6) k_density(AtomsView A, TablesView T) {
     chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
@@ -559,7 +576,6 @@ __global__ void __launch_bounds__(kBlock) k_density(AtomsView A, TablesView T) {
         double4 ci = make_double4(0., 0., 0., 0.);
         if (valid) {
             ci = A.crd[i];
-            int const ti = static_cast<int>(ci.w);
             int const nu = A.pn_up[i], ntot = nu + A.pn_dn[i];
             PairRow<IX> const row = pair_row<IX>(A, i, R->atom_begin);
             // the next partner's record is loaded one iteration ahead, its list entry two
@@ -575,21 +591,22 @@ __global__ void __launch_bounds__(kBlock) k_density(AtomsView A, TablesView T) {
                 double const r2 = min_image_r2(ci, cj, hx, hy, hz, px, py, pz);
                 if (r2 > T.r_cut_sq)
                     continue;
-                double const dr = sqrt(r2);
+                double dr, idr;
+                if (uc)
+                    pair_distance<true>(r2, dr, idr);
+                else
+                    pair_distance<false>(r2, dr, idr);
                 int const tj = static_cast<int>(cj.w);
                 if (!uc && dr > T.eam_rcut[tj])
                     continue;
                 double t;
                 int const k = tab_locate(dr, T.inv_hr, T.nri, t);
-                int const s = pair_slot(ti, tj);
-                int const off = (tj == (ti < tj ? ti : tj)) ? kF : 2 * kF;
                 double v = 0., d1 = 0., d2 = 0.;
-                tab_eval<IP, true, OBS, false>(
-                    T.rb + (static_cast<size_t>(s) * T.nri + k) * 3 * kF + off, t, T.inv_hr,
-                    T.inv_hr2, v, d1, d2);
+                tab_eval<IP, true, OBS, false>(T.rr + static_cast<unsigned>(tj * T.nri + k) * kF, t,
+                                               T.inv_hr, T.inv_hr2, v, d1, d2);
                 rho += v;
                 if (OBS) {
-                    double const ar = d1 / dr;
+                    double const ar = d1 * idr;
                     double const ap[3] = {ar * px, ar * py, ar * pz};
                     g[0] += ap[0] * px;
                     g[1] += ap[1] * py;
@@ -675,8 +692,12 @@ __global__ void __launch_bounds__(kBlock) k_density(AtomsView A, TablesView T) {
 // row's global sums are summed in FP64 registers along the row; warp_slots then spreads the
 // warp's 23 pair sums and 12 sums over atoms over its lanes, two running sums per lane. The
 // loops keep 23 FP64 sums live instead of all 35 of the block, so three 128-thread blocks of
-// the observable-step variant fit an SM instead of two. 13,500 atoms, 16 lanes per atom: 0.0717
-// -> 0.0580 ms against a shuffle reduction per atom into shared accumulators.
+// the observable-step variant fit an SM instead of two (4 blocks, 128 registers, spill). 13,500
+// atoms: 0.0717 -> 0.0580 ms against a shuffle reduction per atom into shared accumulators (16
+// lanes per atom), 0.0513 with 8 lanes and even row halves, 0.0481 with one rho read per one-type
+// pair instead of a bundle of three functions (L1 wavefronts 38.4 -> 30.5 M at 54,000 atoms, 75 ->
+// 63 % of the rate), 0.0469 with pair_distance. Bound by the latency of the L1 gathers at 12 warps per
+// SM.
 
 template <bool OBS> struct RowSums64 {
     double virial = 0.;
@@ -720,19 +741,20 @@ __device__ __forceinline__ void force_row(AtomsView const &A, TablesView const &
         double const r2 = min_image_r2(in.ci, cj, in.hx, in.hy, in.hz, px, py, pz);
         if (r2 > T.r_cut_sq)
             continue;
-        double const dr = sqrt(r2);
-        double const idr = 1. / dr;
+        double dr, idr;
+        pair_distance<UC>(r2, dr, idr);
         int const tj = static_cast<int>(cj.w);
         int const s = pair_slot(ti, tj);
         double t;
         int const k = tab_locate(dr, T.inv_hr, T.nri, t);
-        const double *bundle = T.rb + (static_cast<size_t>(s) * T.nri + k) * 3 * kF;
         // TablePotential::calculate (potential.hpp:92-104)
         double V = 0., dV = 0., d2V = 0.;
         if (dr < T.pot_rmin[s])
             warn_rmin = true;
         if (UC || !(dr > T.pot_rcut[s]))
-            tab_eval<IP, true, true, OBS && UPPER>(bundle, t, T.inv_hr, T.inv_hr2, V, dV, d2V);
+            tab_eval<IP, true, true, OBS && UPPER>(
+                T.rb + static_cast<unsigned>(s * T.nri + k) * kF, t, T.inv_hr, T.inv_hr2, V, dV,
+                d2V);
         double dedr = dV;
         double X = 0., lap = 0.;
         if (OBS && UPPER) {
@@ -740,15 +762,20 @@ __device__ __forceinline__ void force_row(AtomsView const &A, TablesView const &
             lap = 2. * (d2V + 2. * dV * idr);
         }
         if (T.has_eam) {
-            // rho of the lower type at bundle offset kF, of the higher type at 2 kF
-            int const oi = (ti <= tj) ? kF : 2 * kF, oj = (ti < tj) ? 2 * kF : kF;
+            // a pair of one type reads and evaluates its one rho once
             double drho_i = 0., drho_j = 0., d2rho_i = 0., d2rho_j = 0., unused = 0.;
             if (UC || !(dr > T.eam_rcut[ti]))
-                tab_eval<IP, false, true, OBS && UPPER>(bundle + oi, t, T.inv_hr, T.inv_hr2,
-                                                        unused, drho_i, d2rho_i);
-            if (UC || !(dr > T.eam_rcut[tj]))
-                tab_eval<IP, false, true, OBS && UPPER>(bundle + oj, t, T.inv_hr, T.inv_hr2,
-                                                        unused, drho_j, d2rho_j);
+                tab_eval<IP, false, true, OBS && UPPER>(
+                    T.rr + static_cast<unsigned>(ti * T.nri + k) * kF, t, T.inv_hr, T.inv_hr2,
+                    unused, drho_i, d2rho_i);
+            if (ti == tj) {
+                drho_j = drho_i;
+                d2rho_j = d2rho_i;
+            } else if (UC || !(dr > T.eam_rcut[tj])) {
+                tab_eval<IP, false, true, OBS && UPPER>(
+                    T.rr + static_cast<unsigned>(tj * T.nri + k) * kF, t, T.inv_hr, T.inv_hr2,
+                    unused, drho_j, d2rho_j);
+            }
             double const dFj = dFj2.x;
             // the two cross terms are rounded separately and added (commutative), so
             // the i- and j-side evaluations of dE/dr are bitwise equal
@@ -802,7 +829,7 @@ __device__ __forceinline__ void force_row(AtomsView const &A, TablesView const &
 }
 
 template <bool OBS, bool KICK, int TPA, int IP, typename IX>
-__global__ void __launch_bounds__(kBlock) k_force(AtomsView A, TablesView T) {
+__global__ void __launch_bounds__(kBlock, 3) k_force(AtomsView A, TablesView T) {
     chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
@@ -1321,19 +1348,9 @@ __global__ void k_table_eval(TablesView T, int which, int s, const double *x, in
                                                         v[2]);
     } else {
         int const k = tab_locate(xv, T.inv_hr, T.nri, t);
-        int slot, off;
-        double rc;
-        if (which == 0) {
-            slot = s;
-            off = 0;
-            rc = T.pot_rcut[s];
-        } else {
-            slot = pair_slot(s, s);
-            off = kF;
-            rc = T.eam_rcut[s];
-        }
+        double const rc = which == 0 ? T.pot_rcut[s] : T.eam_rcut[s];
         if (!(xv > rc)) {
-            const double *p = T.rb + (static_cast<size_t>(slot) * T.nri + k) * 3 * kF + off;
+            const double *p = (which == 0 ? T.rb : T.rr) + (static_cast<size_t>(s) * T.nri + k) * kF;
             if (bs)
                 tab_eval<MDELAST_BSPLINE, true, true, true>(p, t, T.inv_hr, T.inv_hr2, v[0],
                                                             v[1], v[2]);

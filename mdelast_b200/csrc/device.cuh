@@ -11,8 +11,8 @@
 //   nbr   int[n_pad][maxn] full neighbour list, atom-major (one contiguous row per atom,
 //                          read by the atom's TPA lanes together): partners j > i from
 //                          slot 0 up (n_up), j < i from slot maxn-1 down (n_dn)
-//   rb    double[npot][nri][18] r-table bundle of each type pair (a <= b):
-//                          phi_ab | rho_a | rho_b quintic coefficients of one interval
+//   rb    double[npot][nri][6] phi_ab and rr double[ntypes][nri][6] rho_a: quintic
+//                          coefficients of one interval
 //   Ft    double[ntypes][nfi][6] embedding-function coefficients
 #pragma once
 
@@ -86,7 +86,9 @@ struct Replica {
 };
 
 struct TablesView {
-    const double *rb; // [npot][nri][18]
+    // FP64 r tables, kF coefficients per interval: phi of every type pair (a <= b), [npot][nri],
+    // and rho of every type, [ntypes][nri]
+    const double *rb, *rr;
     int nri, npot;
     double inv_hr, inv_hr2;
     const double *Ft; // [ntypes][nfi][6]
@@ -258,8 +260,8 @@ __device__ __forceinline__ void ld6(const double *p, double c[6]) {
 // (poly_table.hpp:137-176): QUINTIC, the 6 coefficients of the quintic in t from which
 // value and derivatives all come (poly_table.hpp:71-97); BSPLINE, 12 = three cubics in t,
 // the pieces of the three independent cubic B-splines through the node values of f, f'
-// and f'' (poly_table.hpp:117-135), evaluated as values. kF is the per-function stride;
-// a pair-table bundle holds three functions (phi_ab, rho_a, rho_b).
+// and f'' (poly_table.hpp:117-135), evaluated as values. kF is the
+// stride of an interval.
 template <int IP> struct TabFmt {
     static constexpr int kF = IP == MDELAST_BSPLINE ? 12 : 6;
     // FP32 records of the mixed-precision tables: a quintic's 6 coefficients and two products

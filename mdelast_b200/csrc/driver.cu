@@ -1322,7 +1322,7 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
     double const rcut = p0->rcut;
     d->r_list = d->neighbors ? rcut * c0.r_skin : rcut;
 
-    // ---- tables: r-table bundles and embedding tables. Per interval and function, the 6
+    // ---- tables: r tables and embedding tables. Per interval and function, the 6
     // quintic coefficients, or for "bspline" the 12 coefficients of the three cubics
     int const interp = p0->interpolation;
     bool const bsp = interp == MDELAST_BSPLINE;
@@ -1331,19 +1331,15 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         return (bsp ? q.cub.data() : q.coef.data()) + kF * static_cast<size_t>(k);
     };
     int const nri = p0->table.n;
-    std::vector<double> rb(static_cast<size_t>(npot) * nri * 3 * kF, 0.);
-    for (int b = 0; b < nt; ++b)
-        for (int a = 0; a <= b; ++a) {
-            int const s = b * (b + 1) / 2 + a;
-            for (int k = 0; k < nri; ++k) {
-                double *o = rb.data() + (static_cast<size_t>(s) * nri + k) * 3 * kF;
-                std::memcpy(o, fun(c0.pair[s]->table, k), kF * sizeof(double));
-                if (c0.n_eam) {
-                    std::memcpy(o + kF, fun(c0.eam[a]->rho, k), kF * sizeof(double));
-                    std::memcpy(o + 2 * kF, fun(c0.eam[b]->rho, k), kF * sizeof(double));
-                }
-            }
-        }
+    // phi of every pair slot, then rho of every type (zeros without EAM)
+    size_t const n_phi = static_cast<size_t>(npot) * nri * kF;
+    std::vector<double> rb(n_phi + static_cast<size_t>(nt) * nri * kF, 0.);
+    for (int q = 0; q < npot; ++q)
+        std::memcpy(rb.data() + static_cast<size_t>(q) * nri * kF, fun(c0.pair[q]->table, 0),
+                    static_cast<size_t>(nri) * kF * sizeof(double));
+    for (int t = 0; t < c0.n_eam; ++t)
+        std::memcpy(rb.data() + n_phi + static_cast<size_t>(t) * nri * kF, fun(c0.eam[t]->rho, 0),
+                    static_cast<size_t>(nri) * kF * sizeof(double));
     int const nfi = c0.n_eam ? c0.eam[0]->F.n : 1;
     std::vector<double> Ft(static_cast<size_t>(nt) * nfi * kF, 0.);
     for (int t = 0; t < c0.n_eam; ++t)
@@ -1357,6 +1353,7 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
     TablesView &T = d->T;
     T.rb = d->d_rb;
+    T.rr = d->d_rb + n_phi;
     T.nri = nri;
     T.npot = npot;
     T.inv_hr = p0->table.inv_h;
@@ -2362,16 +2359,13 @@ int mdelast_table_eval_device(const mdelast_pair *p, const mdelast_eam *e, int w
     T.interp = bsp ? MDELAST_BSPLINE : MDELAST_QUINTIC;
     if (which == 2) {
         Ft.assign(src.begin(), src.end());
-        rb.assign(3 * kF, 0.);
+        rb.assign(kF, 0.);
         T.nfi = nint;
         T.inv_hf = tab.inv_h;
         T.inv_hf2 = tab.inv_h2;
         T.nri = 1;
     } else {
-        rb.assign(static_cast<size_t>(nint) * 3 * kF, 0.);
-        for (int k = 0; k < nint; ++k)
-            std::memcpy(rb.data() + static_cast<size_t>(k) * 3 * kF + (which == 0 ? 0 : kF),
-                        src.data() + kF * static_cast<size_t>(k), kF * sizeof(double));
+        rb.assign(src.begin(), src.end());
         Ft.assign(kF, 0.);
         T.nri = nint;
         T.inv_hr = tab.inv_h;
@@ -2392,7 +2386,7 @@ int mdelast_table_eval_device(const mdelast_pair *p, const mdelast_eam *e, int w
         dfree(d_o);
         return rc;
     }
-    T.rb = d_rb;
+    T.rb = T.rr = d_rb;
     T.Ft = d_Ft;
     cudaError_t err = cudaMemcpy(d_rb, rb.data(), sizeof(double) * rb.size(), cudaMemcpyHostToDevice);
     if (!err)
