@@ -507,19 +507,58 @@ __device__ __forceinline__ void nbr_build_atom(AtomsView const &A, int i, unsign
     }
 }
 
-// Grid-striding warps over the atoms of the replicas k_nbr_cells left (all when
-// !cells_done); the padding slots keep the zero counts of their allocation.
-__global__ void k_nbr_build(AtomsView A, int cells_done) {
+// Rows of up to kRowThreads replicas, thread t's n of its replica: s_first[t] the first of replica
+// t's rows among them all, s_first[kRowThreads] their number, which is returned. Blocks of
+// kRowThreads threads.
+constexpr int kRowThreads = 256;
+__device__ __forceinline__ int scan_rows(int n, int *s_first, int *s_wsum) {
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!__syncthreads_or(n))
+        return 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        int const v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += v;
+    }
+    if (lane == 31)
+        s_wsum[warp] = incl;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w)
+        incl += s_wsum[w];
+    s_first[threadIdx.x + 1] = incl;
+    if (threadIdx.x == 0)
+        s_first[0] = 0;
+    __syncthreads();
+    return s_first[kRowThreads];
+}
+
+// The atoms of the replicas k_nbr_cells left (all when !cells_done), dealt to the warps of the
+// whole grid; the padding slots keep the zero counts of their allocation. (Each replica
+// over all warps in turn, the first warps did every replica's few atoms: 64 x 500 atoms 0.52 ms
+// with the refresh, now 0.12; without work, 64 replicas asked one after the other, 79 us, now 5.)
+__global__ void __launch_bounds__(kRowThreads) k_nbr_build(AtomsView A, int cells_done) {
     chain_begin();
+    __shared__ int s_first[kRowThreads + 1], s_wsum[kRowThreads / 32];
     unsigned const lane = threadIdx.x & 31u;
     int const w0 = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     int const n_warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
-    for (int r = 0; r < A.n_rep; ++r) {
-        Replica const &R = A.rep[r];
-        if (cells_done && R.nc[0] != 0 && !narrow_cells(R, A.r_list_sq))
-            continue;
-        for (int a = w0; a < R.n_atoms; a += n_warps)
-            nbr_build_atom(A, R.atom_begin + a, lane, cells_done);
+    for (int r0 = 0; r0 < A.n_rep; r0 += kRowThreads) {
+        int const r = r0 + static_cast<int>(threadIdx.x);
+        int n = 0;
+        if (r < A.n_rep) {
+            Replica const &R = A.rep[r];
+            if (!(cells_done && R.nc[0] != 0 && !narrow_cells(R, A.r_list_sq)))
+                n = R.n_atoms;
+        }
+        int const total = scan_rows(n, s_first, s_wsum);
+        for (int q = w0, k = 0; q < total; q += n_warps) {
+            while (s_first[k + 1] <= q)
+                ++k;
+            nbr_build_atom(A, A.rep[r0 + k].atom_begin + q - s_first[k], lane, cells_done);
+        }
+        __syncthreads(); // s_first is read until here
     }
 }
 
@@ -1020,11 +1059,12 @@ __global__ void __launch_bounds__(kBlock) k_kick_drift(AtomsView A, TablesView T
 // FP64 min-image test on both atoms of a pair (so the list is symmetric). A replica's rows
 // are rebuilt when its list was rebuilt or when some atom has moved by more than half the
 // radius margin since the last refresh: then every pair now within r_cut is still in the
-// list. One warp per atom slot at a time, grid-striding over the slots; the warp tests 32
-// entries at a time and compacts the kept ones with a ballot. The kernel runs every step
-// and most steps refresh nothing: each block first asks whether any replica is due (one
-// flag per thread) and returns at once if none is, so a step without a refresh costs one
-// short wave instead of a warp per atom slot.
+// list. One warp per row; the warp tests 32 entries at a time. The kernel runs every step and
+// most steps refresh few replicas or none: each block first lists the rows of the replicas that
+// are due (one flag per thread, a scan of their atom counts), returns at once if there are
+// none, and otherwise all warps share just those rows. A refresh is bound by instruction issue and
+// by the unit that serves match_any and votes (74 %): 0.099 ms for 54,000 rows of 190 entries;
+// ballots per key bit instead, with 64 or 16 keys, took 0.114 and 0.098 ms.
 //
 // Halves: the force pass forms a pair's global sums on one of its two visits, that of the atom
 // whose row holds it in its upper half, and walks the halves in two loops; lanes of a warp wait
@@ -1037,10 +1077,10 @@ __global__ void __launch_bounds__(kBlock) k_kick_drift(AtomsView A, TablesView T
 // 0.0513 ms (13,500 atoms, FP64).
 //
 // Row order (`sorted`, when the row fits the warp's shared-memory scratch): each half of a
-// row is ordered by distance shell, shells kSubShell wide
-// in r/r_cut, in list order within a shell (a stable counting sort: the warp counts the
-// shells with shared-memory atomics, scans the counts, and places each chunk of 32 entries
-// with match_any). The lanes of a warp walk their rows in step, so at every iteration they
+// row is ordered by distance shell, shells kSubShell wide in r/r_cut, in list order within a
+// shell (a stable counting sort over 64 keys, half and shell: as entries pass the test,
+// match_any gives each its rank among the entries of its key; one scan of the key counts then
+// gives every entry its slot). The lanes of a warp walk their rows in step, so at every iteration they
 // look up the tables at about the same r (the same neighbour shell of the lattice) and
 // read a few nearby intervals instead of scattered ones. Only the order in which an atom's
 // pair terms are summed changes; which pairs are kept does not.
@@ -1063,15 +1103,11 @@ __device__ __forceinline__ SubConst sub_const(AtomsView const &A) {
 // whether atom i's row holds partner j in its upper half (of i and j exactly one's does)
 __device__ __forceinline__ bool pair_owner(int i, int j) { return (j > i) == (((i ^ j) & 4) == 0); }
 
-__device__ __forceinline__ void sublist_row(AtomsView const &A, int i, int lane, bool sorted,
-                                            int *s_j, int *s_cnt, SubConst const &sc) {
-    int const r = A.rep_of[i];
-    if (r < 0)
-        return;
-    Replica const *R = A.rep + r;
-    if (!(R->sub_force || R->sub_d2 > A.sub_half2))
-        return;
-    sorted = sorted && R->n_atoms <= (1 << 26); // the packing holds 26-bit offsets
+// one row; s_e, s_rank, s_cnt: this warp's scratch (SORTED); F32: mixed precision's keep test
+template <bool SORTED, bool F32>
+__device__ __forceinline__ void sublist_row(AtomsView const &A, Replica const *R, int i, int lane,
+                                            unsigned *s_e, unsigned short *s_rank, int *s_cnt,
+                                            SubConst const &sc) {
     double4 const ci = A.crd[i];
     double const hx = R->h[0], hy = R->h[1], hz = R->h[2];
     int const nu = A.n_up[i], nd = A.n_dn[i];
@@ -1079,107 +1115,105 @@ __device__ __forceinline__ void sublist_row(AtomsView const &A, int i, int lane,
     int *out = A.pnbr + static_cast<size_t>(i) * A.pmaxn;
     uint16_t *out16 = A.pnbr16 ? A.pnbr16 + static_cast<size_t>(i) * A.pmaxn : nullptr;
     int const base = R->atom_begin;
-    auto put = [&](int slot, int j) {
+    auto put = [&](int slot, int offset) {
         if (out16)
-            out16[slot] = static_cast<uint16_t>(j - base);
+            out16[slot] = static_cast<uint16_t>(offset);
         else
-            out[slot] = j;
+            out[slot] = base + offset;
     };
     unsigned const lt = (1u << lane) - 1u;
-    // Mixed precision: the keep test runs in FP32 on the positions the pair passes read, with
-    // the minimum image they use (the same on both atoms of a pair, so the list stays
-    // symmetric), against the radius widened by 1e-5: every pair within it in exact arithmetic is
-    // kept, a few just beyond it too, which add zeros. FP64: the reference's min image and the
-    // exact radius.
-    bool const f32 = A.posf != nullptr;
+    // Mixed precision: the keep test runs in FP32 on the wrapped positions the pair passes
+    // read, with the minimum image they use (the same on both atoms of a pair, so the list
+    // stays symmetric), against the radius widened by 1e-5: every pair within it in exact
+    // arithmetic is kept, a few just beyond it too, which add zeros. FP64: the reference's
+    // min image and the exact radius.
     float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
     float3 L = make_float3(0.f, 0.f, 0.f), iL = L;
-    if (f32) {
+    if (F32) {
         pi = A.posf[i];
         box_f(R, L, iL);
     }
-    float const sub_r2f = sc.r2f, ish = f32 ? sc.inv_shell_a : sc.inv_shell;
-    if (sorted) {
+    float const sub_r2f = sc.r2f, ish = F32 ? sc.inv_shell_a : sc.inv_shell;
+    int const n = nu + nd;
+    auto entry = [&](int k) { return k < n ? row[k < nu ? k : A.maxn - 1 - (k - nu)] : i; };
+    // the next 32 entries are loaded one pass ahead, their records with them
+    int jn = entry(lane);
+    float4 pn = F32 ? A.posf[jn] : pi;
+    if (SORTED) {
         s_cnt[lane] = 0;
-        s_cnt[kSubShells + lane] = 0;
+        s_cnt[32 + lane] = 0;
         __syncwarp();
     }
-    int ku = 0, kd = 0;
-    for (int k0 = 0; k0 < nu + nd; k0 += 32) {
-        int const k = k0 + lane;
-        bool keep = false, upper = k < nu;
-        int j = -1;
-        float r2s = 0.f; // r^2 in the units of ish (A^2 or cm^2)
-        if (k < nu + nd) {
-            j = row[upper ? k : A.maxn - 1 - (k - nu)];
-            upper = pair_owner(i, j);
-            if (f32) {
-                float dx, dy, dz;
-                r2s = min_image_f(pi, A.posf[j], L, iL, dx, dy, dz);
-                keep = r2s <= sub_r2f;
-            } else {
-                double px, py, pz;
-                double const r2 = min_image_r2(ci, A.crd[j], hx, hy, hz, px, py, pz);
-                keep = r2 <= A.sub_r2;
-                r2s = static_cast<float>(r2);
-            }
-        }
-        unsigned const bu = __ballot_sync(0xffffffffu, keep && upper);
-        unsigned const bd = __ballot_sync(0xffffffffu, keep && !upper);
-        if (sorted) {
-            // kept entries to the scratch in list order (upper from the front, lower from
-            // the back) with their shell in the top bits; shells counted per half
-            if (keep) {
-                int const q = upper ? ku + __popc(bu & lt) : A.maxn - 1 - (kd + __popc(bd & lt));
-                int const sh = min(kSubShells - 1, static_cast<int>(sqrtf(r2s) * ish));
-                s_j[q] = (sh << 26) | (j - base);
-                atomicAdd(&s_cnt[(upper ? 0 : kSubShells) + sh], 1);
-            }
+    int kept = 0, ku = 0, kd = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        bool const in = k0 + lane < n;
+        int const j = jn;
+        float4 const pj = pn;
+        jn = entry(k0 + 32 + lane);
+        if (F32)
+            pn = A.posf[jn];
+        bool const upper = pair_owner(i, j);
+        bool keep;
+        float r2s; // r^2 in the units of ish (A^2 or cm^2)
+        if (F32) {
+            float dx, dy, dz;
+            r2s = min_image_f(pi, pj, L, iL, dx, dy, dz);
+            keep = in && r2s <= sub_r2f;
         } else {
-            if (keep && upper)
-                put(ku + __popc(bu & lt), j);
-            if (keep && !upper)
-                put(A.pmaxn - 1 - (kd + __popc(bd & lt)), j);
+            double px, py, pz;
+            double const r2 = min_image_r2(ci, A.crd[j], hx, hy, hz, px, py, pz);
+            keep = in && r2 <= A.sub_r2;
+            r2s = static_cast<float>(r2);
         }
-        ku += __popc(bu);
-        kd += __popc(bd);
+        if (SORTED) {
+            // key and rank of each kept entry (other lanes: keys of their own)
+            int const sh = min(kSubShells - 1, __float2int_rz(r2s * rsqrtf(r2s) * ish));
+            int const key = keep ? (upper ? sh : kSubShells + sh) : 2 * kSubShells + lane;
+            unsigned const all = __ballot_sync(0xffffffffu, keep);
+            unsigned const peers = __match_any_sync(0xffffffffu, key);
+            int const before = keep ? s_cnt[key] : 0;
+            __syncwarp();
+            if (keep) {
+                int const q = kept + __popc(all & lt);
+                s_e[q] = static_cast<unsigned>(key) << 26 | static_cast<unsigned>(j - base);
+                s_rank[q] = static_cast<unsigned short>(before + __popc(peers & lt));
+                if ((peers & lt) == 0)
+                    s_cnt[key] = before + __popc(peers);
+            }
+            __syncwarp();
+            kept += __popc(all);
+        } else {
+            unsigned const bu = __ballot_sync(0xffffffffu, keep && upper);
+            unsigned const bd = __ballot_sync(0xffffffffu, keep && !upper);
+            if (keep)
+                put(upper ? ku + __popc(bu & lt) : A.pmaxn - 1 - (kd + __popc(bd & lt)), j - base);
+            ku += __popc(bu);
+            kd += __popc(bd);
+        }
     }
-    if (sorted) {
-        __syncwarp();
-        for (int half = 0; half < 2; ++half) {
-            // exclusive scan of this half's shell counts: the shells' first output slots
-            int const c = s_cnt[half * kSubShells + lane];
-            int incl = c;
+    if (SORTED) {
+        // exclusive scans of both halves' shell counts: the shells' first slots
+        int const cu = s_cnt[lane], cd = s_cnt[32 + lane];
+        int iu = cu, id = cd;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int const v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o)
-                    incl += v;
-            }
-            __syncwarp();
-            s_cnt[half * kSubShells + lane] = incl - c;
-            __syncwarp();
-            int const n_half = half ? kd : ku;
-            for (int e0 = 0; e0 < n_half; e0 += 32) {
-                int const e = e0 + lane;
-                bool const act = e < n_half;
-                int packed = 0, sh = kSubShells; // inactive lanes: a shell no entry has
-                if (act) {
-                    packed = s_j[half ? A.maxn - 1 - e : e];
-                    sh = packed >> 26;
-                }
-                unsigned const peers = __match_any_sync(0xffffffffu, sh);
-                if (act) {
-                    int const slot = s_cnt[half * kSubShells + sh] + __popc(peers & lt);
-                    put(half ? A.pmaxn - 1 - slot : slot, base + (packed & 0x3ffffff));
-                }
-                __syncwarp();
-                // the lowest lane of each shell's group advances that shell's next slot
-                if (act && (peers & lt) == 0)
-                    s_cnt[half * kSubShells + sh] += __popc(peers);
-                __syncwarp();
+        for (int o = 1; o < 32; o <<= 1) {
+            int const vu = __shfl_up_sync(0xffffffffu, iu, o), vd = __shfl_up_sync(0xffffffffu, id, o);
+            if (lane >= o) {
+                iu += vu;
+                id += vd;
             }
         }
+        s_cnt[lane] = iu - cu;
+        s_cnt[32 + lane] = id - cd;
+        ku = __shfl_sync(0xffffffffu, iu, 31);
+        kd = __shfl_sync(0xffffffffu, id, 31);
+        __syncwarp();
+        for (int q = lane; q < kept; q += 32) {
+            unsigned const e = s_e[q];
+            int const key = static_cast<int>(e >> 26), slot = s_cnt[key] + s_rank[q];
+            put(key < kSubShells ? slot : A.pmaxn - 1 - slot, static_cast<int>(e & 0x3ffffffu));
+        }
+        __syncwarp(); // the scratch is the next row's
     }
     if (lane == 0) {
         A.pn_up[i] = ku;
@@ -1188,35 +1222,64 @@ __device__ __forceinline__ void sublist_row(AtomsView const &A, int i, int lane,
     }
 }
 
-// dynamic shared memory of k_sublist: per warp of its 256-thread blocks, one row of packed
-// entries (maxn) and two halves' shell counters; 0 when that exceeds kSublistSortMax or a
-// replica offset does not fit the packing (the rows then keep list order)
+// dynamic shared memory of k_sublist: per warp of its 256-thread blocks, a row of packed entries and
+// one of ranks (maxn each) and the 64 key counters; 0 when that exceeds kSublistSortMax (the
+// rows then keep list order)
 __host__ __device__ size_t sublist_smem(int maxn) {
-    size_t const b = static_cast<size_t>(256 / 32) * (maxn + 2 * kSubShells) * sizeof(int);
+    size_t const b = (256 / 32) * (sizeof(int) * (static_cast<size_t>(maxn) + 2 * kSubShells) +
+                                   sizeof(short) * ((static_cast<size_t>(maxn) + 1) / 2 * 2));
     return b <= kSublistSortMax ? b : 0;
 }
 
 // 5 blocks of 256 threads per SM (the launch is 5 blocks per SM): at most 48 registers
-__global__ void __launch_bounds__(256, 5) k_sublist(AtomsView A) {
+template <bool F32>
+__global__ void __launch_bounds__(kRowThreads, 5) k_sublist(AtomsView A) {
     chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
     extern __shared__ int s_sub[];
-    int due = 0;
-    for (int r = threadIdx.x; r < A.n_rep; r += blockDim.x) {
-        Replica const *R = A.rep + r;
-        due |= R->sub_force || R->sub_d2 > A.sub_half2;
-    }
-    if (!__syncthreads_or(due))
-        return;
+    __shared__ int s_first[kRowThreads + 1]; // first row of each replica among the rows due
+    __shared__ int s_wsum[kRowThreads / 32];
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    bool const sorted = sublist_smem(A.maxn) > 0;
-    int *s_j = s_sub + static_cast<size_t>(warp) * (A.maxn + 2 * kSubShells);
-    int *s_cnt = s_j + A.maxn;
-    int const n_warps = gridDim.x * (blockDim.x >> 5);
+    int const n_warps = gridDim.x * (kRowThreads / 32), w0 = blockIdx.x * (kRowThreads / 32) + warp;
+    bool const fits = sublist_smem(A.maxn) > 0;
+    int *s_cnt = s_sub + 2 * kSubShells * warp;
+    unsigned *s_e = reinterpret_cast<unsigned *>(s_sub + 2 * kSubShells * (kRowThreads / 32)) +
+                    static_cast<size_t>(warp) * A.maxn;
+    unsigned short *s_rank =
+        reinterpret_cast<unsigned short *>(s_sub + (2 * kSubShells + A.maxn) * (kRowThreads / 32)) +
+        static_cast<size_t>(warp) * ((A.maxn + 1) / 2 * 2);
     SubConst const sc = sub_const(A);
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < A.n_pad; i += n_warps)
-        sublist_row(A, i, lane, sorted, s_j, s_cnt, sc);
+    for (int r0 = 0; r0 < A.n_rep; r0 += kRowThreads) {
+        // the rows due of 256 replicas at a time
+        int const r = r0 + static_cast<int>(threadIdx.x);
+        int n = 0;
+        if (r < A.n_rep) {
+            Replica const *R = A.rep + r;
+            if (R->sub_force || R->sub_d2 > A.sub_half2)
+                n = R->n_atoms;
+        }
+        int const total = scan_rows(n, s_first, s_wsum);
+        for (int q = w0, k = 0; q < total; q += n_warps) {
+            while (s_first[k + 1] <= q)
+                ++k;
+            Replica const *R = A.rep + r0 + k;
+            int const i = R->atom_begin + q - s_first[k];
+            if (fits && R->n_atoms <= (1 << 26)) // the packing holds 26-bit offsets
+                sublist_row<true, F32>(A, R, i, lane, s_e, s_rank, s_cnt, sc);
+            else
+                sublist_row<false, F32>(A, R, i, lane, s_e, s_rank, s_cnt, sc);
+        }
+        __syncthreads(); // s_first is read until here
+    }
+}
+
+void launch_sublist(int grid, size_t smem, cudaStream_t s, AtomsView const &A) {
+    auto const kernel = A.posf ? k_sublist<true> : k_sublist<false>;
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem));
+    launch_chain(kernel, grid, kRowThreads, smem, s, A);
 }
 
 __global__ void k_sub_invalidate(AtomsView A) {

@@ -321,11 +321,7 @@ struct mdelast_driver_s {
     void point_pair_list();
     void refresh_pair_list(cudaStream_t s) {
         if (A.crd_ref) {
-            size_t const smem = sublist_smem(A.maxn);
-            if (smem > 48 * 1024)
-                cudaFuncSetAttribute(k_sublist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem));
-            launch_chain(k_sublist, std::min(n_pad / 8, kSublistBlocks), 256, smem, s, A);
+            launch_sublist(std::min(n_pad / 8, kSublistBlocks), sublist_smem(A.maxn), s, A);
         }
     }
     double *d_pd = nullptr, *d_pf = nullptr, *d_red = nullptr;
@@ -792,6 +788,13 @@ void mdelast_driver_s::drop_graphs() {
         }
 }
 
+// All-pairs search even where cells fit: replicas of at most kBruteAtoms atoms, and up to
+// kBruteIdle while the batch's 2 x 2 x 2 groups of half cells (a block each) leave SMs idle. A warp per atom
+// fills them. List build and pair-list refresh, cells against all pairs: 500 atoms 0.051 / 0.028 ms,
+// 2,048 atoms 0.141 / 0.053 ms, 2,916 atoms 0.151 / 0.067 ms; 4,000 atoms on cells
+// 0.101 ms.
+constexpr int kBruteAtoms = 1000, kBruteIdle = 3000;
+
 // Half cells per edge for the current box: twice the number of cells no thinner than the
 // list radius (with a margin for the box changes of an NPT run between rebuilds); fewer
 // than 3 such cells along any edge means an all-pairs search.
@@ -799,6 +802,19 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
     // per replica: cells per edge from its box, and its block of the global cell arrays
     std::vector<Replica> R(static_cast<size_t>(n_rep));
     CK(cudaMemcpy(R.data(), d_rep, sizeof(Replica) * n_rep, cudaMemcpyDeviceToHost));
+    // whether the groups of every replica with cells together are fewer than the SMs
+    double groups = 0.;
+    for (int q = 0; q < n_rep; ++q) {
+        double g = 1.;
+        bool fits = rep_count[q] > kBruteAtoms;
+        for (int a = 0; a < 3; ++a) {
+            double const c = std::floor(boxes[3 * q + a] / (r_list * 1.05));
+            fits = fits && c >= 3.;
+            g *= c;
+        }
+        groups += fits ? g : 0.;
+    }
+    bool const idle = groups < 148.;
     bool changed = false, all_brute = true;
     int n_cells = 0, cap = std::max(A.cell_cap, 32);
     for (int q = 0; q < n_rep; ++q) {
@@ -810,6 +826,7 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
                 brute = true;
             nc[a] *= 2;
         }
+        brute = brute || rep_count[q] <= kBruteAtoms || (idle && rep_count[q] <= kBruteIdle);
         if (brute)
             nc[0] = nc[1] = nc[2] = 0;
         Replica &r = R[static_cast<size_t>(q)];

@@ -73,9 +73,10 @@ __global__ void k_pre(AtomsView A);
 __global__ void k_reduce(AtomsView A);
 __global__ void k_post(AtomsView A, int mode, int obs, mdelast_observables *host);
 __global__ void k_samples_reset(AtomsView A, int what);
-__global__ void k_sublist(AtomsView A);
+// the pair-list refresh, with sublist_smem(maxn) bytes of dynamic shared memory
+void launch_sublist(int grid, size_t smem, cudaStream_t s, AtomsView const &A);
 // k_sublist's dynamic shared memory for rows of capacity maxn (0: rows keep list order)
-constexpr size_t kSublistSortMax = 96 * 1024;
+constexpr size_t kSublistSortMax = 150 * 1024;
 __host__ __device__ size_t sublist_smem(int maxn);
 __global__ void k_sub_invalidate(AtomsView A);
 __global__ void k_readout(AtomsView A, TablesView T, int r, int field, double *out,
