@@ -427,8 +427,8 @@ struct mdelast_mlp_s {
     // activations for a batch of cap samples: per layer Z and A; A[0] is the input
     int cap = 0;
     std::vector<float *> Z, A, dA;
-    float *Yt = nullptr, *dZ = nullptr, *loss = nullptr;
-    // the two-kernel step: per-block gradients and loss sums (kStepBlocks of them)
+    float *Yt = nullptr, *dZ = nullptr, *loss = nullptr, *act = nullptr;
+    // the two-kernel step: per-block gradients and loss sums (for the blocks of cap samples)
     bool fused = false;
     size_t fused_smem = 0;
     float *part = nullptr, *part_loss = nullptr, *pp = nullptr; // pp: the padded parameters
@@ -470,11 +470,8 @@ struct mdelast_mlp_s {
         cudaSetDevice(device);
         if (graph)
             cudaGraphExecDestroy(graph);
-        for (float *q : {p, Yt, dZ}) // p: the slab of all that is sized by the parameters
-            cudaFree(q);
-        for (auto *v : {&Z, &A, &dA})
-            for (float *q : *v)
-                cudaFree(q);
+        cudaFree(p);   // the slab of all that is sized by the parameters
+        cudaFree(act); // ... and by the samples
         if (stream)
             cudaStreamDestroy(stream);
     }
@@ -487,26 +484,42 @@ struct mdelast_mlp_s {
             graph = nullptr;
             graph_n = -1;
         }
-        for (auto *v : {&Z, &A, &dA})
-            for (float *&q : *v) {
-                cudaFree(q);
-                q = nullptr;
-            }
-        cudaFree(Yt);
-        cudaFree(dZ);
+        cudaFree(act);
+        act = nullptr;
+        cap = 0;
+        // one allocation for everything sized by the samples
+        int wmax = 0;
+        size_t total = 0;
+        auto at = [&](size_t floats) {
+            size_t const o = total;
+            total += (floats + 63) / 64 * 64;
+            return o;
+        };
+        size_t const m = static_cast<size_t>(n);
+        std::vector<size_t> oA, oD, oZ;
+        for (int k = 0; k <= L; ++k) {
+            oA.push_back(at(m * w[k]));
+            oD.push_back(at(m * w[k]));
+            oZ.push_back(k > 0 ? at(m * w[k]) : 0);
+            wmax = std::max(wmax, w[k]);
+        }
+        size_t const oY = at(m * w[L]), odZ = at(m * wmax);
+        size_t const nb = static_cast<size_t>(std::min((n + kTile16 - 1) / kTile16, kStepBlocks));
+        size_t const oP = at(fused ? nb * padded_params(view(1)) : 0), oL = at(fused ? nb : 0);
+        MCK(cudaMalloc(&act, sizeof(float) * total));
         Z.assign(L + 1, nullptr);
         A.assign(L + 1, nullptr);
         dA.assign(L + 1, nullptr);
-        int wmax = 0;
         for (int k = 0; k <= L; ++k) {
-            MCK(cudaMalloc(&A[k], sizeof(float) * static_cast<size_t>(n) * w[k]));
-            MCK(cudaMalloc(&dA[k], sizeof(float) * static_cast<size_t>(n) * w[k]));
+            A[k] = act + oA[k];
+            dA[k] = act + oD[k];
             if (k > 0)
-                MCK(cudaMalloc(&Z[k], sizeof(float) * static_cast<size_t>(n) * w[k]));
-            wmax = std::max(wmax, w[k]);
+                Z[k] = act + oZ[k];
         }
-        MCK(cudaMalloc(&Yt, sizeof(float) * static_cast<size_t>(n) * w[L]));
-        MCK(cudaMalloc(&dZ, sizeof(float) * static_cast<size_t>(n) * wmax));
+        Yt = act + oY;
+        dZ = act + odZ;
+        part = act + oP;
+        part_loss = act + oL;
         cap = n;
         return MDELAST_OK;
     }
@@ -587,12 +600,12 @@ int mdelast_mlp_create(int32_t n_layers, const int32_t *widths, uint64_t seed, i
     size_t const bytes = sizeof(float) * static_cast<size_t>(m->np);
     cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
     // one allocation: p, g, m1, m2 (zero but p), the step counter, the loss, and the two-kernel
-    // step's per-block sums
+    // step's copy of the parameters
     m->fused_smem = step_smem(m->view(1));
     m->fused = m->fused_smem <= kStepSmemMax;
     size_t const np = (static_cast<size_t>(m->np) + 63) / 64 * 64,
                  npp = static_cast<size_t>(padded_params(m->view(1))),
-                 extra = m->fused ? npp * (kStepBlocks + 1) + kStepBlocks : 0;
+                 extra = m->fused ? npp : 0;
     if (e == cudaSuccess)
         e = cudaMalloc(&m->p, sizeof(float) * (4 * np + 64 + extra));
     if (e == cudaSuccess)
@@ -603,8 +616,6 @@ int mdelast_mlp_create(int32_t n_layers, const int32_t *widths, uint64_t seed, i
     m->t = reinterpret_cast<int *>(m->p + 4 * np);
     m->loss = m->p + 4 * np + 32;
     m->pp = m->p + 4 * np + 64;
-    m->part = m->pp + npp;
-    m->part_loss = m->part + npp * kStepBlocks;
     if (e == cudaSuccess && m->fused)
         e = cudaFuncSetAttribute(k_step_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(kStepSmemMax));
