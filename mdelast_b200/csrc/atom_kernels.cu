@@ -590,9 +590,9 @@ __device__ __forceinline__ void pair_distance(double r2, double &dr, double &idr
 // into shared accumulators the pass took 0.0397 instead of 0.0306 ms on 13,500 atoms (16 lanes
 // per atom; 0.0266 ms with 8 lanes and pair_distance). Bound by the L1 data pipe (75 % of its
 // wavefront rate, FP64 pipe 39 %). 6 blocks per SM: 5 and 7 are slower by 3 and 5 % on 108,000
-// atoms.
+// atoms; 3 with 32 lanes, whose launches have no more (6 spill).
 template <bool OBS, int TPA, int IP, typename IX>
-__global__ void __launch_bounds__(kBlock, 6) k_density(AtomsView A, TablesView T) {
+__global__ void __launch_bounds__(kBlock, TPA == 32 ? 3 : 6) k_density(AtomsView A, TablesView T) {
     chain_begin();
     if (halted(A)) // a list build ran out of capacity: nothing until the host regrows
         return;
@@ -1434,7 +1434,8 @@ void density_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, Table
     case 1: launch_chain(k_density<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 4: launch_chain(k_density<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 8: launch_chain(k_density<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_density<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_chain(k_density<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_density<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -1450,7 +1451,8 @@ void force_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesV
     case 1: launch_chain(k_force<OBS, KICK, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 4: launch_chain(k_force<OBS, KICK, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 8: launch_chain(k_force<OBS, KICK, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_force<OBS, KICK, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_chain(k_force<OBS, KICK, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_force<OBS, KICK, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>

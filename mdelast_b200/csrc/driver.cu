@@ -206,6 +206,23 @@ int default_tpa(long n_atoms, bool mixed) {
 // atom group of kBlock/tpa atoms. Fills each replica's block range and the block ->
 // replica map; returns the grid size.
 constexpr int kTargetBlocks = 148 * 32;
+
+// Lanes per atom a pass is launched with: 16 becomes 32, a warp per atom, while all atoms at 32
+// lanes stay within 3 blocks per SM (1,536 atoms), what the FP64 force pass holds at once. A pass over
+// so few atoms is the latency of its longest row, which 32 lanes walk in half the iterations. Density /
+// force pass / step in us, 16 and 32 lanes per atom:
+//   atoms       FP64 16               FP64 32               mixed 16              mixed 32
+//   500         14.2 / 16.3 / 46.2    10.8 / 12.3 / 41.1    12.2 / 12.5 / 40.2    10.3 / 12.3 / 38.1
+//   1,372       14.3 / 17.3 / 48.9    12.2 / 14.4 / 44.7    12.3 / 14.3 / 44.0    10.3 / 12.4 / 41.1
+//   2,048       14.4 / 18.4 / 51.4    12.3 / 20.5 / 53.4    12.3 / 14.3 / 45.4    11.1 / 14.4 / 45.3
+//   4,000       16.4 / 28.9 / 69.8    18.4 / 28.7 / 67.2    12.3 / 16.5 / 54.0    12.5 / 20.5 / 54.1
+constexpr long kWideBlocks = 148 * 3;
+int lanes_per_atom(std::vector<Replica *> const &reps, int tpa) {
+    long total = 0;
+    for (Replica const *r : reps)
+        total += r->n_blocks;
+    return tpa == 16 && total * 32 <= kWideBlocks ? 32 : tpa;
+}
 // shared memory for the staged force tables: the rest of the SM's 228 KB is the L1 of the
 // partner gathers
 constexpr long kStageBudget = 184 * 1024;
@@ -267,7 +284,8 @@ struct mdelast_driver_s {
     bool cell_staging = true;
     cudaStream_t stream = nullptr;
     int N = 0, n_pad = 0, n_rep = 1, ntypes = 0, npot = 0, n_blocks = 0;
-    int tpa_d = 1, tpa_f = 1; // lanes per atom of the density and force passes
+    int tpa_d = 1, tpa_f = 1; // lanes per atom of the density and force passes, as chosen ...
+    int lanes_d = 1, lanes_f = 1; // ... and as launched (lanes_per_atom)
     int grid_d = 1, grid_f = 1; // blocks of the density and force passes
     int *d_dblk_rep = nullptr, *d_fblk_rep = nullptr;
     int neighbors = 0;
@@ -288,9 +306,9 @@ struct mdelast_driver_s {
     float *d_phf = nullptr, *d_rrf = nullptr, *d_rdf = nullptr;
     void pass_density(bool obs, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED)
-            launch_density_mx(obs, tpa_d, grid_d, s, A, T);
+            launch_density_mx(obs, lanes_d, grid_d, s, A, T);
         else
-            launch_density(obs, tpa_d, grid_d, s, A, T);
+            launch_density(obs, lanes_d, grid_d, s, A, T);
     }
     // force pass with the staged shared-memory tables (mixed precision, quintic, when the
     // tables were staged; chosen by the autotuner or set_force_staging)
@@ -301,11 +319,11 @@ struct mdelast_driver_s {
     }
     void pass_force(bool obs, bool kick, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED && stage_f && T.st_n > 0)
-            launch_force_mx_staged(obs, kick, tpa_f, grid_f, s, A, T);
+            launch_force_mx_staged(obs, kick, lanes_f, grid_f, s, A, T);
         else if (precision == MDELAST_PRECISION_MIXED)
-            launch_force_mx(obs, kick, tpa_f, grid_f, s, A, T);
+            launch_force_mx(obs, kick, lanes_f, grid_f, s, A, T);
         else
-            launch_force(obs, kick, tpa_f, grid_f, s, A, T);
+            launch_force(obs, kick, lanes_f, grid_f, s, A, T);
     }
     int *d_nbr = nullptr, *d_nup = nullptr, *d_ndn = nullptr;
     // pair list of the pair passes (see AtomsView::pnbr); pair_factor 0: the neighbour list
@@ -579,8 +597,9 @@ int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, i
     for (auto &x : R)
         reps.push_back(&x);
     std::vector<int> dmap, fmap;
-    int const gd = deal_blocks(reps, tpa_d_, true, dmap, tgt_d);
-    int const gf = deal_blocks(reps, tpa_f_, false, fmap, tgt_f, st ? kStagedBlock : kBlock);
+    int const ld = lanes_per_atom(reps, tpa_d_), lf = lanes_per_atom(reps, tpa_f_);
+    int const gd = deal_blocks(reps, ld, true, dmap, tgt_d);
+    int const gf = deal_blocks(reps, lf, false, fmap, tgt_f, st ? kStagedBlock : kBlock);
     int chunks = 1;
     for (Replica const *x : reps)
         chunks = std::max(chunks, (std::max(x->dblk_n, x->fblk_n) + kChunk - 1) / kChunk);
@@ -612,6 +631,8 @@ int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, i
     CK(cudaMemcpy(d_rep, R.data(), sizeof(Replica) * n_rep, cudaMemcpyHostToDevice));
     tpa_d = tpa_d_;
     tpa_f = tpa_f_;
+    lanes_d = ld;
+    lanes_f = lf;
     target_d = tgt_d;
     target_f = tgt_f;
     stage_f = st;
@@ -1579,8 +1600,9 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
     }
     d->tpa_d = d->tpa_f = default_tpa(n_total, c0.precision == MDELAST_PRECISION_MIXED);
     std::vector<int> dmap, fmap;
-    d->grid_d = deal_blocks(reps, d->tpa_d, true, dmap);
-    d->grid_f = deal_blocks(reps, d->tpa_f, false, fmap);
+    d->lanes_d = d->lanes_f = lanes_per_atom(reps, d->tpa_d);
+    d->grid_d = deal_blocks(reps, d->lanes_d, true, dmap);
+    d->grid_f = deal_blocks(reps, d->lanes_f, false, fmap);
     TRY(dalloc_later(&d->d_dblk_rep, dmap.size()));
     TRY(dalloc_later(&d->d_fblk_rep, fmap.size()));
     d->cap_dmap = dmap.size();

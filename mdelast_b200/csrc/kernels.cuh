@@ -60,8 +60,8 @@ void launch_density_mx(bool obs, int tpa, int grid, cudaStream_t s, AtomsView co
                        TablesView const &T);
 void launch_force_mx(bool obs, bool kick, int tpa, int grid, cudaStream_t s, AtomsView const &A,
                      TablesView const &T);
-// the mixed force pass with the quintic tables staged in shared memory (T.st_n > 0; tpa 4,
-// 8 or 16; blocks of kStagedBlock threads); prepare_force_mx_staged raises the kernels'
+// the mixed force pass with the quintic tables staged in shared memory (T.st_n > 0; tpa 4, 8,
+// 16 or 32; blocks of kStagedBlock threads); prepare_force_mx_staged raises the kernels'
 // dynamic shared-memory limit (to the staging budget) before any launch or capture
 constexpr int kStagedBlock = 512;
 void launch_force_mx_staged(bool obs, bool kick, int tpa, int grid, cudaStream_t s,

@@ -689,7 +689,8 @@ void density_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
     case 1: launch_chain(k_density_mx<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 4: launch_chain(k_density_mx<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
     case 8: launch_chain(k_density_mx<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_density_mx<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_chain(k_density_mx<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_density_mx<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -706,7 +707,8 @@ void force_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
     case 1: launch_chain(k_force_mx<OBS, KICK, 1, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
     case 4: launch_chain(k_force_mx<OBS, KICK, 4, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
     case 8: launch_chain(k_force_mx<OBS, KICK, 8, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_force_mx<OBS, KICK, 16, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_chain(k_force_mx<OBS, KICK, 16, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_chain(k_force_mx<OBS, KICK, 32, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>
@@ -716,7 +718,7 @@ void force_mx_tpa(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesV
     else
         force_mx_tpa_ix<OBS, KICK, IP, int>(tpa, grid, s, A, T);
 }
-// the staged kernels: lanes per atom 4, 8 or 16
+// the staged kernels: lanes per atom 4, 8, 16 or 32
 template <bool OBS, bool KICK, typename IX>
 void force_mx_staged_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                         TablesView const &T) {
@@ -725,9 +727,8 @@ void force_mx_staged_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
     switch (tpa) {
     case 4: launch_chain(k_force_mx<OBS, KICK, 4, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
     case 8: launch_chain(k_force_mx<OBS, KICK, 8, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
-    default:
-        launch_chain(k_force_mx<OBS, KICK, 16, Q, true, IX>, grid, kBlockStaged, smem, s, A, T);
-        break;
+    case 16: launch_chain(k_force_mx<OBS, KICK, 16, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    default: launch_chain(k_force_mx<OBS, KICK, 32, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK>
@@ -746,6 +747,8 @@ template <bool OBS, bool KICK, typename IX> cudaError_t staged_attr_ix(int bytes
         e = cudaFuncSetAttribute(k_force_mx<OBS, KICK, 8, Q, true, IX>, a, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_force_mx<OBS, KICK, 16, Q, true, IX>, a, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_force_mx<OBS, KICK, 32, Q, true, IX>, a, bytes);
     return e;
 }
 template <bool OBS, bool KICK> cudaError_t staged_attr(int bytes) {
