@@ -104,9 +104,11 @@ struct TablesView {
     // mixed precision: the r tables in FP32 with lengths in angstrom and values in eV
     // (phi) or angstrom^-3 (rho), one record of TabFmt<IP>::kFf floats per function and
     // interval: phf phi_ab of every type pair (a <= b), rrf rho of every type (quintic records
-    // hold c0..c5, 3 c3, 5 c5); rdf, quintic only, rho for the force pass, which needs its
-    // derivatives alone: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5. Cutoffs in angstrom.
-    const float *phf, *rrf, *rdf;
+    // hold c0..c5, 3 c3, 5 c5). Quintic, for the force pass, which needs rho's derivatives
+    // alone: phf holds phi's c0..c5 and rho_a's c1, 2 c2, and phq, 4 floats, rho_a's 3 c3, 4 c4, 5 c5
+    // and phi's 3 c3, so a pair of one type reads 48 bytes; rdf holds rho for the second
+    // type of a pair: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5. Cutoffs in angstrom.
+    const float *phf, *phq, *rrf, *rdf;
     float finv_hr, finv_hr2, fr_cut_sq, frmin_max; // frmin_max: the largest fpot_rmin
     uint2 slots[kMaxTypes]; // byte b of slots[a]: pair_slot(a, b)
     // Staged copy for the shared-memory force pass (quintic only): the intervals

@@ -303,7 +303,7 @@ struct mdelast_driver_s {
     int precision = MDELAST_PRECISION_FP64;
     float4 *d_posf = nullptr;
     float2 *d_dF2f = nullptr;
-    float *d_phf = nullptr, *d_rrf = nullptr, *d_rdf = nullptr;
+    float *d_phf = nullptr, *d_phq = nullptr, *d_rrf = nullptr, *d_rdf = nullptr;
     void pass_density(bool obs, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED)
             launch_density_mx(obs, lanes_d, grid_d, s, A, T);
@@ -438,6 +438,7 @@ mdelast_driver_s::~mdelast_driver_s() {
     dfree_idle(d_posf);
     dfree_idle(d_dF2f);
     dfree_idle(d_phf);
+    dfree_idle(d_phq);
     dfree_idle(d_rrf);
     dfree_idle(d_rdf);
     dfree_idle(d_stf);
@@ -1449,24 +1450,35 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
                 pack(fun(c0.eam[t]->rho, k), a3,
                      rrf.data() + (static_cast<size_t>(t) * nri + k) * kFf);
         if (!bsp) { // the products of the records, rounded as the kernels round them
-            std::vector<float> rdf(rrf.size());
-            for (std::vector<float> *v : {&phf, &rrf})
-                for (size_t q = 0; q < v->size(); q += kFf) {
-                    float *c = v->data() + q;
-                    c[6] = 3.f * c[3];
-                    c[7] = 5.f * c[5];
-                }
+            std::vector<float> rdf(rrf.size()), phq(phf.size() / kFf * 4);
             for (size_t q = 0; q < rrf.size(); q += kFf) {
-                float const *c = rrf.data() + q;
+                float *c = rrf.data() + q;
+                c[6] = 3.f * c[3];
+                c[7] = 5.f * c[5];
                 float const d[8] = {c[1],       2.f * c[2], c[6],        4.f * c[4],
                                     c[7],       6.f * c[3], 12.f * c[4], 20.f * c[5]};
                 std::copy(d, d + 8, rdf.data() + q);
             }
+            for (int b = 0; b < nt; ++b)
+                for (int a = 0; a <= b; ++a)
+                    for (int k = 0; k < nri; ++k) {
+                        size_t const q = static_cast<size_t>(pair_slot(a, b)) * nri + k;
+                        float const *r = rdf.data() + (static_cast<size_t>(a) * nri + k) * kFf;
+                        float *c = phf.data() + q * kFf;
+                        float const x[4] = {r[2], r[3], r[4], 3.f * c[3]};
+                        c[6] = r[0];
+                        c[7] = r[1];
+                        std::copy(x, x + 4, phq.data() + q * 4);
+                    }
             TRY(dalloc_later(&d->d_rdf, rdf.size()));
+            TRY(dalloc_later(&d->d_phq, phq.size()));
             if (cudaMemcpy(d->d_rdf, rdf.data(), sizeof(float) * rdf.size(),
+                           cudaMemcpyHostToDevice) ||
+                cudaMemcpy(d->d_phq, phq.data(), sizeof(float) * phq.size(),
                            cudaMemcpyHostToDevice))
                 return bail(fail(MDELAST_ERR_CUDA, "table upload failed"));
             T.rdf = d->d_rdf;
+            T.phq = d->d_phq;
         }
         TRY(dalloc_later(&d->d_phf, phf.size()));
         TRY(dalloc_later(&d->d_rrf, rrf.size()));

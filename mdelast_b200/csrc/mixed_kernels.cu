@@ -26,7 +26,7 @@ __device__ __forceinline__ int tab_locate_f(float x, float inv_h, int n, float &
     return i;
 }
 
-// Quintic records (8 floats, TablesView::phf and rrf: c0..c5, 3 c3, 5 c5) and derivative records
+// Quintic records (8 floats, TablesView::rrf: c0..c5, 3 c3, 5 c5) and derivative records
 // (rdf: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5). The pair force is evaluated from
 // both of its atoms, in different code paths of the force pass; its arithmetic is written with
 // explicit rounding (no contraction left to the compiler) so that both evaluations, and those
@@ -298,23 +298,26 @@ struct RowIn {
     float3 L, iL;
 };
 
-// The quintic record of phi_s and the derivative records of rho_ti and rho_tj on interval k:
-// from the staged shared-memory copy (STAGED and k staged; c0..c5 alone, the products formed
-// here) or from the global records. Both give the same FP32 values, so the pair terms do not
-// depend on where they were read. A pair of one type reads its one rho once: dj is left
-// undefined and the caller takes the terms of di.
+// The quintic record of phi_s and the derivative records of rho of the pair's types lo <= hi on
+// interval k: from the staged shared-memory copy (STAGED and k staged; c0..c5 alone, the
+// products formed here) or from the global records. Both give the same FP32 values (a product
+// by 2 or 4 is exact), so the pair terms do not depend on where they were read. A pair of one
+// type reads its one rho once: dh is left undefined and the caller takes the terms of dl.
+//
+// phi and rho_lo lie in one 32-byte and one 16-byte record: the L1 data pipe takes 27 and 16
+// wavefronts for them, two 32-byte records 54.
 template <bool STAGED>
 __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *stab, int s,
-                                           int ti, int tj, int k, float (&cp)[8],
-                                           float (&di)[8], float (&dj)[8]) {
+                                           int lo, int hi, int k, float (&cp)[8],
+                                           float (&dl)[8], float (&dh)[8]) {
     if (STAGED) {
         unsigned const q = static_cast<unsigned>(k - T.st_lo);
         if (q < static_cast<unsigned>(T.st_n)) {
             int const n6 = 6 * T.st_n;
             const float *b = stab + 6 * q;
             const float2 *pp = reinterpret_cast<const float2 *>(b + s * n6);
-            const float2 *pi = reinterpret_cast<const float2 *>(b + (T.npot + ti) * n6);
-            const float2 *pj = reinterpret_cast<const float2 *>(b + (T.npot + tj) * n6);
+            const float2 *pi = reinterpret_cast<const float2 *>(b + (T.npot + lo) * n6);
+            const float2 *pj = reinterpret_cast<const float2 *>(b + (T.npot + hi) * n6);
             float ci[6], cj[6];
 #pragma unroll
             for (int u = 0; u < 3; ++u) {
@@ -328,15 +331,26 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
             }
             cp[6] = __fmul_rn(3.f, cp[3]);
             cp[7] = __fmul_rn(5.f, cp[5]);
-            derivative_record(ci, di);
-            derivative_record(cj, dj);
+            derivative_record(ci, dl);
+            derivative_record(cj, dh);
             return;
         }
     }
     constexpr int kFf = TabFmt<MDELAST_QUINTIC>::kFf;
-    ld256(T.phf + static_cast<unsigned>(s * T.nri + k) * kFf, cp);
-    ld256(T.rdf + static_cast<unsigned>(ti * T.nri + k) * kFf, di);
-    ld256_if(ti != tj, T.rdf + static_cast<unsigned>(tj * T.nri + k) * kFf, dj);
+    unsigned const q = static_cast<unsigned>(s * T.nri + k);
+    float4 const x = __ldg(reinterpret_cast<const float4 *>(T.phq) + q);
+    ld256(T.phf + q * kFf, cp);
+    ld256_if(lo != hi, T.rdf + static_cast<unsigned>(hi * T.nri + k) * kFf, dh);
+    dl[0] = cp[6];
+    dl[1] = cp[7];
+    dl[2] = x.x;
+    dl[3] = x.y;
+    dl[4] = x.z;
+    dl[5] = __fmul_rn(2.f, x.x);
+    dl[6] = __fmul_rn(3.f, x.y);
+    dl[7] = __fmul_rn(4.f, x.z);
+    cp[6] = x.w;
+    cp[7] = __fmul_rn(5.f, cp[5]);
 }
 
 // One lane's walk over list slots [s0, s1) of an atom row (slots of the upper half when
@@ -388,22 +402,22 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         bool const eam_j = UC || (T.has_eam && !(dr > T.feam_rcut[tj]));
         if constexpr (IP == MDELAST_QUINTIC) {
             // the three functions' coefficients first (independent loads), then the math
-            float cp[8], di[8], dj[8];
-            pair_coefs<STAGED>(T, stab, s, ti, tj, k, cp, di, dj);
+            float cp[8], dl[8], dh[8];
+            pair_coefs<STAGED>(T, stab, s, min(ti, tj), max(ti, tj), k, cp, dl, dh);
             if (UC || !(dr > T.fpot_rcut[s])) {
                 V = tabf_v(cp, t);
                 dV = tabf_d1(cp, t, T.finv_hr);
                 if (OBS)
                     d2V = tabf_d2(cp, t, T.finv_hr2);
             }
-            bool const one = ti == tj;
-            drho_i = tabd_d1(di, t, T.finv_hr);
-            drho_j = tabd_d1(dj, t, T.finv_hr);
-            drho_j = one ? drho_i : drho_j;
+            // rho' and rho'' of the types lo and hi, then of i and j
+            float const l1 = tabd_d1(dl, t, T.finv_hr), h1 = tabd_d1(dh, t, T.finv_hr);
+            drho_i = ti <= tj ? l1 : h1;
+            drho_j = ti < tj ? h1 : l1;
             if (OBS) {
-                d2rho_i = tabd_d2(di, t, T.finv_hr2);
-                d2rho_j = tabd_d2(dj, t, T.finv_hr2);
-                d2rho_j = one ? d2rho_i : d2rho_j;
+                float const l2 = tabd_d2(dl, t, T.finv_hr2), h2 = tabd_d2(dh, t, T.finv_hr2);
+                d2rho_i = ti <= tj ? l2 : h2;
+                d2rho_j = ti < tj ? h2 : l2;
             }
             if (!eam_i)
                 drho_i = d2rho_i = 0.f;
@@ -515,8 +529,9 @@ __device__ __forceinline__ bool below_rmin(AtomsView const &A, TablesView const 
 // issue (about half) behind it, at 4 blocks of 4 warps per SM. At 16 x 13,500 atoms and 4 lanes per
 // atom: 0.416 ms when the sums' shuffles and shared accumulators were 19 % of the data pipe's
 // work and the third table function of one-type pairs another 20 %, 0.362 ms without them, 0.345 with
-// even row halves, 0.312 with the products of the coefficients in the table records, the r_min test
-// once per row, pair slots from a byte table and no unrolling.
+// even row halves, 0.314 with the products of the coefficients in the table records, the r_min test
+// once per row, pair slots from a byte table and no unrolling, 0.300 with 48 instead of 64 bytes of
+// tables for a one-type pair.
 //
 // STAGED: the block first copies the staged quintic tables (T.stf, T.st_bytes, about 180 KB
 // for a two-element alloy) into dynamic shared memory and reads every staged interval from
