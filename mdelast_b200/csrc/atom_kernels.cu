@@ -588,7 +588,7 @@ __device__ __forceinline__ void pair_distance(double r2, double &dr, double &idr
 // F''_i g_i g_i^T and the Laplacian term) are formed in every lane of the atom and spread
 // over the lanes by warp_slots, one running sum per lane; with 23 warp sums per atom group
 // into shared accumulators the pass took 0.0397 instead of 0.0306 ms on 13,500 atoms (16 lanes
-// per atom; 0.0266 ms with 8 lanes and pair_distance). Bound by the L1 data pipe (75 % of its
+// per atom; 0.0254 ms with 8 lanes, pair_distance and ld_crd). Bound by the L1 data pipe (75 % of its
 // wavefront rate, FP64 pipe 39 %). 6 blocks per SM: 5 and 7 are slower by 3 and 5 % on 108,000
 // atoms; 3 with 32 lanes, whose launches have no more (6 spill).
 template <bool OBS, int TPA, int IP, typename IX>
@@ -618,12 +618,12 @@ __global__ void __launch_bounds__(kBlock, TPA == 32 ? 3 : 6) k_density(AtomsView
             int const nu = A.pn_up[i], ntot = nu + A.pn_dn[i];
             PairRow<IX> const row = pair_row<IX>(A, i, R->atom_begin);
             // the next partner's record is loaded one iteration ahead, its list entry two
-            double4 cn = A.crd[sub < ntot ? row.at(list_slot(sub, nu, A.pmaxn)) : i];
+            double4 cn = ld_crd(A.crd + (sub < ntot ? row.at(list_slot(sub, nu, A.pmaxn)) : i));
             int jn = sub < ntot ? row.at(list_slot(min(sub + TPA, ntot - 1), nu, A.pmaxn)) : i;
             for (int kk = sub; kk < ntot; kk += TPA) {
                 double4 const cj = cn;
                 if (kk + TPA < ntot) {
-                    cn = A.crd[jn];
+                    cn = ld_crd(A.crd + jn);
                     jn = row.at(list_slot(min(kk + 2 * TPA, ntot - 1), nu, A.pmaxn));
                 }
                 double px, py, pz;
@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(kBlock, TPA == 32 ? 3 : 6) k_density(AtomsView
 // atoms: 0.0717 -> 0.0580 ms against a shuffle reduction per atom into shared accumulators (16
 // lanes per atom), 0.0513 with 8 lanes and even row halves, 0.0481 with one rho read per one-type
 // pair instead of a bundle of three functions (L1 wavefronts 38.4 -> 30.5 M at 54,000 atoms, 75 ->
-// 63 % of the rate), 0.0469 with pair_distance. Bound by the latency of the L1 gathers at 12 warps per
+// 63 % of the rate), 0.0461 with pair_distance and ld_crd. Bound by the latency of the L1 gathers at 12 warps per
 // SM.
 
 template <bool OBS> struct RowSums64 {
@@ -765,14 +765,14 @@ __device__ __forceinline__ void force_row(AtomsView const &A, TablesView const &
     double const dFi = in.dFi, d2Fi = in.d2Fi;
     // the next partner's record and F' are loaded one iteration ahead, its list entry two
     int jn = row.at(slot(sub));
-    double4 cn = A.crd[jn];
+    double4 cn = ld_crd(A.crd + jn);
     double2 fn = A.dF2[jn];
     jn = row.at(slot(min(sub + TPA, n - 1)));
     for (int kk = sub; kk < n; kk += TPA) {
         double4 const cj = cn;
         double2 const dFj2 = fn;
         if (kk + TPA < n) {
-            cn = A.crd[jn];
+            cn = ld_crd(A.crd + jn);
             fn = A.dF2[jn];
             jn = row.at(slot(min(kk + 2 * TPA, n - 1)));
         }
