@@ -68,9 +68,10 @@ int mdelast_abi_version(void);
 int mdelast_device_available(void);
 /* Drivers take their device buffers from a stream-ordered memory pool of the library's
  * own (one per device; the device's default pool is not touched), which keeps freed memory
- * for the next driver, and stage their atom uploads in a pinned host buffer kept for the
- * next creation; this hands the unused part of the pool back to the device and frees the
- * pinned buffer. No reference counterpart (the reference holds host memory only). */
+ * for the next driver, stage their atom uploads in a pinned host buffer kept for the
+ * next creation, and leave their own pinned blocks (observables, readouts) to the next driver, up to
+ * 16 blocks and 64 MB; this hands the unused part of the pool back to the device and frees the
+ * pinned memory. No reference counterpart (the reference holds host memory only). */
 int mdelast_release_cached_memory(int32_t device);
 
 /* ---------------------------------------------------------------------------------

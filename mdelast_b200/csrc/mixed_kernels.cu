@@ -525,8 +525,8 @@ __device__ __forceinline__ bool below_rmin(AtomsView const &A, TablesView const 
 // over atoms go through warp_slots (31 and, at 4 lanes per atom, 4 exchanges) into two FP64
 // registers per lane; the virial is the trace of the Born stress.
 //
-// What bounds it: the L1 data pipe (about two thirds of its wavefront rate) with instruction
-// issue (about half) behind it, at 4 blocks of 4 warps per SM. At 16 x 13,500 atoms and 4 lanes per
+// What bounds it: scattered gathers, by their wavefronts (67 per 32 visits, 52 % of the L1 data
+// pipe's rate) and their latency at 4 blocks of 4 warps per SM, with instruction issue (47 %) behind. At 16 x 13,500 atoms and 4 lanes per
 // atom: 0.416 ms when the sums' shuffles and shared accumulators were 19 % of the data pipe's
 // work and the third table function of one-type pairs another 20 %, 0.362 ms without them, 0.345 with
 // even row halves, 0.314 with the products of the coefficients in the table records, the r_min test
