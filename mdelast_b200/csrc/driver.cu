@@ -179,15 +179,18 @@ double nint_host(double x) { // md_driver.hpp:48-50
 // while a pass is a wave of latency-bound warps (a few thousand atoms), then 8, and in mixed
 // precision 4 once those fill the SMs too (FP64 rows are long enough in instructions for 8 at
 // any size). One lane per atom leaves every load of a row uncoalesced. Density + force pass in
-// ms, by lanes per atom (cells of the two-element alloy):
+// ms, by lanes per atom (cells of the two-element alloy), launched back to back:
 //   atoms     FP64 4 / 8 / 16             mixed 1 / 4 / 8 / 16
-//   5,324     0.080 / 0.053 / 0.051       0.131 / 0.051 / 0.038 / 0.040
-//   8,788     0.082 / 0.072 / 0.072       0.135 / 0.053 / 0.041 / 0.045
-//   13,500    0.094 / 0.082 / 0.090       0.139 / 0.058 / 0.058 / 0.061
-//   19,652    0.132 / 0.118 / 0.123       0.136 / 0.079 / 0.078 / 0.083
-//   32,000    0.195 / 0.175 / 0.190       0.139 / 0.098 / 0.102 / 0.116
-//   216,000   1.037 / 1.033 / 1.119       0.668 / 0.532 / 0.547 / 0.655
-//   640,000   3.03 / 3.03 / 3.27          1.83 / 1.48 / 1.58 / 1.93
+//   5,324     0.068 / 0.046 / 0.046       0.116 / 0.044 / 0.035 / 0.038
+//   8,788     0.070 / 0.066 / 0.066       0.116 / 0.044 / 0.038 / 0.043
+//   13,500    0.074 / 0.072 / 0.081       0.118 / 0.049 / 0.053 / 0.056
+//   19,652    0.110 / 0.102 / 0.111       0.124 / 0.071 / 0.071 / 0.078
+//   32,000    0.170 / 0.153 / 0.166       0.130 / 0.087 / 0.094 / 0.107
+//   216,000   0.869 / 0.870 / 0.979       0.603 / 0.469 / 0.474 / 0.578
+//   640,000   2.55 / 2.56 / 2.86          1.72 / 1.31 / 1.37 / 1.69
+// In a mixed step, whose passes find colder caches, 8 lanes lead longer: 0.0755 against 0.0903 ms at
+// 13,500 atoms, 0.0833 / 0.0952 at 16,384, 0.0950 / 0.0950 at 19,652, 0.1026 / 0.1008 at 23,328
+// (ternary 0.1156 / 0.1178).
 // MDELAST_TPA overrides it.
 int default_tpa(long n_atoms, bool mixed) {
     if (char const *e = std::getenv("MDELAST_TPA")) {
