@@ -609,8 +609,10 @@ int mdelast_mlp_create(int32_t n_layers, const int32_t *widths, uint64_t seed, i
                  extra = m->fused ? npp : 0;
     if (e == cudaSuccess)
         e = cudaMalloc(&m->p, sizeof(float) * (4 * np + 64 + extra));
+    // in the order of the network's own stream, as everything that touches these buffers (that
+    // stream does not wait for the legacy one), and complete on return
     if (e == cudaSuccess)
-        e = cudaMemset(m->p, 0, sizeof(float) * (4 * np + 64));
+        e = cudaMemsetAsync(m->p, 0, sizeof(float) * (4 * np + 64), m->stream);
     m->g = m->p + np;
     m->m1 = m->p + 2 * np;
     m->m2 = m->p + 3 * np;
@@ -621,7 +623,9 @@ int mdelast_mlp_create(int32_t n_layers, const int32_t *widths, uint64_t seed, i
         e = cudaFuncSetAttribute(k_step_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(kStepSmemMax));
     if (e == cudaSuccess)
-        e = cudaMemcpy(m->p, h.data(), bytes, cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(m->p, h.data(), bytes, cudaMemcpyHostToDevice, m->stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) {
         delete m;
         return fail(MDELAST_ERR_CUDA, "MLP set-up: %s", cudaGetErrorString(e));
@@ -656,12 +660,12 @@ int mdelast_mlp_set_params(mdelast_mlp *m, const float *in) {
     if (!m || !in)
         return fail(MDELAST_ERR_ARGUMENT, "bad argument");
     MCK(cudaSetDevice(m->device));
-    MCK(cudaStreamSynchronize(m->stream));
     size_t const bytes = sizeof(float) * static_cast<size_t>(m->np);
-    MCK(cudaMemcpy(m->p, in, bytes, cudaMemcpyHostToDevice));
-    MCK(cudaMemset(m->m1, 0, bytes)); // a new starting point resets the optimiser
-    MCK(cudaMemset(m->m2, 0, bytes));
-    MCK(cudaMemset(m->t, 0, sizeof(int)));
+    MCK(cudaMemcpyAsync(m->p, in, bytes, cudaMemcpyHostToDevice, m->stream));
+    MCK(cudaMemsetAsync(m->m1, 0, bytes, m->stream)); // a new starting point resets the optimiser
+    MCK(cudaMemsetAsync(m->m2, 0, bytes, m->stream));
+    MCK(cudaMemsetAsync(m->t, 0, sizeof(int), m->stream));
+    MCK(cudaStreamSynchronize(m->stream));
     return MDELAST_OK;
 }
 
