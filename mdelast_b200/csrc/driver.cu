@@ -85,6 +85,15 @@ template <typename T> int dalloc(T **p, size_t n) {
     return allocs_done();
 }
 
+// Host data into a buffer that kernels on stream s read, in that stream's order and complete on
+// return. A cudaMemcpy goes through the legacy stream, which a driver's non-blocking stream does
+// not wait for, and from pageable memory it may return before the copy has landed.
+int upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
+    return MDELAST_OK;
+}
+
 // Returned to the pool; the caller has waited for all work on the device, as cudaFree would.
 template <typename T> void dfree_idle(T *&p) {
     if (p)
@@ -630,9 +639,12 @@ int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, i
         return rc;
     if (int rc = grow(d_red, cap_red, static_cast<size_t>(n_rep) * chunks * 64))
         return rc;
-    CK(cudaMemcpy(d_dblk_rep, dmap.data(), sizeof(int) * dmap.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_fblk_rep, fmap.data(), sizeof(int) * fmap.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_rep, R.data(), sizeof(Replica) * n_rep, cudaMemcpyHostToDevice));
+    if (int rc = upload(d_dblk_rep, dmap.data(), sizeof(int) * dmap.size(), stream))
+        return rc;
+    if (int rc = upload(d_fblk_rep, fmap.data(), sizeof(int) * fmap.size(), stream))
+        return rc;
+    if (int rc = upload(d_rep, R.data(), sizeof(Replica) * n_rep, stream))
+        return rc;
     tpa_d = tpa_d_;
     tpa_f = tpa_f_;
     lanes_d = ld;
@@ -826,7 +838,9 @@ constexpr int kBruteAtoms = 1000, kBruteIdle = 3000;
 int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
     // per replica: cells per edge from its box, and its block of the global cell arrays
     std::vector<Replica> R(static_cast<size_t>(n_rep));
-    CK(cudaMemcpy(R.data(), d_rep, sizeof(Replica) * n_rep, cudaMemcpyDeviceToHost));
+    // after what the stream still holds (a resumed launch clears status bits there)
+    CK(cudaMemcpyAsync(R.data(), d_rep, sizeof(Replica) * n_rep, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
     // whether the groups of every replica with cells together are fewer than the SMs
     double groups = 0.;
     for (int q = 0; q < n_rep; ++q) {
@@ -868,7 +882,8 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
         all_brute = all_brute && brute;
     }
     if (changed)
-        CK(cudaMemcpy(d_rep, R.data(), sizeof(Replica) * n_rep, cudaMemcpyHostToDevice));
+        if (int rc = upload(d_rep, R.data(), sizeof(Replica) * n_rep, stream))
+            return rc;
     if (!d_cell_count || n_cells > cells_alloc || cap > A.cell_cap)
         if (int rc = alloc_cells(std::max(n_cells, cells_alloc), cap))
             return rc;
@@ -880,8 +895,8 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
     }
     if (crep != cell_rep_host) {
         if (!crep.empty())
-            CK(cudaMemcpy(d_cell_rep, crep.data(), sizeof(int) * crep.size(),
-                          cudaMemcpyHostToDevice));
+            if (int rc = upload(d_cell_rep, crep.data(), sizeof(int) * crep.size(), stream))
+                return rc;
         cell_rep_host = crep;
     }
     if (changed || all_pairs != all_brute || A.n_cells != n_cells)
@@ -2006,7 +2021,8 @@ static int get_neighbors_r(mdelast_driver *d, int r, int32_t *point, int32_t *ne
         dfree(d_point);
         return rc;
     }
-    cudaError_t e = cudaMemcpy(d_point, point, sizeof(int) * (N + 1), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(d_point, point, sizeof(int) * (N + 1),
+                                    cudaMemcpyHostToDevice, d->stream);
     if (e == cudaSuccess) {
         k_half_list_fill<<<(N + 255) / 256, 256, 0, d->stream>>>(d->A, r, d_point, d_list);
         e = cudaMemcpyAsync(neighbors, d_list,
