@@ -109,7 +109,9 @@ struct TablesView {
     // and phi's 3 c3, so a pair of one type reads 48 bytes; rdf holds rho for the second
     // type of a pair: c1, 2 c2, 3 c3, 4 c4, 5 c5, 6 c3, 12 c4, 20 c5. Cutoffs in angstrom.
     const float *phf, *phq, *rrf, *rdf;
-    float finv_hr, finv_hr2, fr_cut_sq, frmin_max; // frmin_max: the largest fpot_rmin
+    float finv_hr, finv_hr2, fr_cut_sq;
+    // the r_min of every pair type, where they share one below the cutoff (0 if negative); else -1
+    float frmin;
     uint2 slots[kMaxTypes]; // byte b of slots[a]: pair_slot(a, b)
     // Staged copy for the shared-memory force pass (quintic only): the intervals
     // [st_lo, st_lo + st_n) of every phi_ab (slot s at s * st_n) followed by every rho_a

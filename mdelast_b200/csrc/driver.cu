@@ -1554,9 +1554,6 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         }
         for (int t = 0; t < nt; ++t)
             T.feam_rcut[t] = static_cast<float>(T.eam_rcut[t] / kAng);
-        T.frmin_max = 0.f;
-        for (int s = 0; s < npot; ++s)
-            T.frmin_max = std::max(T.frmin_max, T.fpot_rmin[s]);
         for (int a = 0; a < nt; ++a) {
             unsigned char b[kMaxTypes] = {};
             for (int q = 0; q < nt; ++q)
@@ -1564,6 +1561,11 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
             std::memcpy(&T.slots[a], b, sizeof(b));
         }
         float const rcf = static_cast<float>(rcut / kAng);
+        // below 0.999 of the cutoff every distance under r_min is one of a pair within the cutoff
+        T.frmin = T.fpot_rmin[0] < 0.999f * rcf ? std::max(T.fpot_rmin[0], 0.f) : -1.f;
+        for (int s = 1; s < npot; ++s)
+            if (!(T.fpot_rmin[s] == T.fpot_rmin[0]))
+                T.frmin = -1.f;
         T.fuc = T.has_eam;
         for (int s = 0; s < npot; ++s)
             T.fuc &= T.fpot_rcut[s] >= rcf;

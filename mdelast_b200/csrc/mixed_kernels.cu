@@ -356,7 +356,9 @@ __device__ __forceinline__ void pair_coefs(TablesView const &T, const float *sta
 // One lane's walk over list slots [s0, s1) of an atom row (slots of the upper half when
 // UPPER, else of the lower half, addressed from the end of the row); every pair adds its
 // force and half its energy to the atom, and the upper half also adds to the global sums.
-// STAGED: quintic tables read from the staged shared-memory copy `stab` where staged.
+// STAGED: quintic tables read from the staged shared-memory copy `stab` where staged. UC: no
+// test of a pair's own against the functions' cutoffs or its r_min; dr_min takes the row's smallest
+// distance, else -1 when a pair within the cutoff lies below its r_min (potential.hpp:92-104 warns).
 template <bool OBS, bool UPPER, int TPA, int IP, bool STAGED, typename IX, bool UC>
 __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView const &T,
                                              RowIn const &in, PairRow<IX> const &row, int n,
@@ -391,9 +393,12 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
         bool const in_cut = !(r2 > T.fr_cut_sq);
         float const idr = rsqrtf(r2);
         float const dr = __fmul_rn(r2, idr);
-        dr_min = fminf(dr_min, dr);
         int const ti = in.ti, tj = __float_as_int(pj.w);
         int const s = __byte_perm(in.slots.x, in.slots.y, tj) & 0xff;
+        if (UC)
+            dr_min = fminf(dr_min, dr);
+        else if (in_cut && dr < T.fpot_rmin[s])
+            dr_min = -1.f;
         float t;
         int const k = tab_locate_f(dr, T.finv_hr, T.nri, t);
         float V = 0.f, dV = 0.f, d2V = 0.f;
@@ -500,24 +505,6 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
     }
 }
 
-// whether one of this lane's pairs lies within the cutoff and below its r_min (potential.hpp:
-// 92-104 warns); walked only when the smallest distance of the row asks for it
-template <int TPA, typename IX>
-__device__ __forceinline__ bool below_rmin(AtomsView const &A, TablesView const &T,
-                                           RowIn const &in, PairRow<IX> const &row, int nu,
-                                           int nd, int sub) {
-    bool warn = false;
-    for (int half = 0; half < 2; ++half)
-        for (int k = sub; k < (half ? nd : nu); k += TPA) {
-            float4 const pj = A.posf[row.at(half ? A.pmaxn - 1 - k : k)];
-            float dx, dy, dz;
-            float const r2 = min_image_f(in.pi, pj, in.L, in.iL, dx, dy, dz);
-            float const dr = __fmul_rn(r2, rsqrtf(r2));
-            warn |= !(r2 > T.fr_cut_sq) && dr < T.fpot_rmin[pair_slot(in.ti, __float_as_int(pj.w))];
-        }
-    return warn;
-}
-
 // Force pass of md_driver.cpp:300-430 (with the closing kick) in mixed precision; see
 // k_force for the roles of the terms. Each atom row is walked in two loops, its upper
 // half (which also feeds the global sums) and its lower half, so the lanes of a warp do not
@@ -585,8 +572,11 @@ __global__ void __launch_bounds__(NB, STAGED ? 1 : 4) k_force_mx(AtomsView A, Ta
             PairRow<IX> const row = pair_row<IX>(A, i, R->atom_begin);
             float dr_min = 3.4e38f; // of this lane's pairs
             PairSums<OBS> ps;
-            // uniform cutoffs (every setfl potential): no per-function cutoff tests
-            if (T.fuc) {
+            // one cutoff and one r_min (every setfl potential): no tests per function and pair
+            // (16 x 13,500 atoms: 0.294 ms; with them, for an r_min of its own per pair type,
+            // 0.311; a second walk over the rows with a distance below the largest, 0.472)
+            bool const uc = T.fuc && T.frmin >= 0.f;
+            if (uc) {
                 force_row_mx<OBS, true, TPA, IP, STAGED, IX, true>(
                     A, T, in, row, nu, sub, fx, fy, fz, epot, ps, dr_min, stab);
                 force_row_mx<OBS, false, TPA, IP, STAGED, IX, true>(
@@ -598,7 +588,7 @@ __global__ void __launch_bounds__(NB, STAGED ? 1 : 4) k_force_mx(AtomsView A, Ta
                     A, T, in, row, nd, sub, fx, fy, fz, epot, ps, dr_min, stab);
             }
             epot *= 0.5;
-            if (dr_min < T.frmin_max && below_rmin<TPA>(A, T, in, row, nu, nd, sub))
+            if (dr_min < (uc ? T.frmin : 0.f))
                 status_or(A.rep + r, MDELAST_WARN_RMIN);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
