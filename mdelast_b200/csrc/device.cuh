@@ -121,8 +121,8 @@ struct TablesView {
     int st_lo, st_n, st_bytes;
     // fuc: there is EAM and every function's FP32 cutoff is at least the pair cutoff, so no
     // per-function test applies to a pair within it; the mixed passes then skip them. uc64: the
-    // same in FP64, exactly: every cutoff is at least sqrt(r_cut_sq), the largest distance
-    // the FP64 passes compute for a pair with r^2 <= r_cut_sq (sqrt is correctly rounded)
+    // same in FP64: r^2 <= r_cut_sq decides whether a pair counts, and every cutoff is at least
+    // sqrt(r_cut_sq), so no r of such a pair lies beyond one
     int fuc, uc64;
     float fpot_rcut[kMaxTypes * (kMaxTypes + 1) / 2];
     float fpot_rmin[kMaxTypes * (kMaxTypes + 1) / 2];
