@@ -289,9 +289,11 @@ int mdelast_batch_get_gr(mdelast_driver *d, int32_t replica, double *gr, double 
  * for each pass and recomputes the per-atom state with it; the state does not advance.
  * choice (4 values, may be NULL): lanes per atom of the density and force passes, block
  * targets of the density and force passes; ms_out (2, may be NULL): their mean times in
- * ms. set_launch sets a shape directly (keeping the force-pass variant). Both drop the
- * captured step graphs (recaptured on the next step). A driver of up to 1,536 atoms in all
- * runs 16 lanes per atom as 32. */
+ * ms. set_launch sets a shape directly, lanes per atom 1, 4, 8 or 16 (keeping the force-pass
+ * variant). Both drop the captured step graphs (recaptured on the next step). On drivers of up to
+ * 1,536 atom slots (each replica padded to a multiple of 256) a warp per atom, 32 lanes, is the
+ * default and one more candidate of the tuners; where one keeps it, choice reports it as 16, the
+ * nearest shape that set_launch takes. */
 int mdelast_driver_autotune(mdelast_driver *d, int32_t n_repeat, int32_t *choice,
                             double *ms_out);
 int mdelast_driver_set_launch(mdelast_driver *d, int32_t tpa_density, int32_t tpa_force,

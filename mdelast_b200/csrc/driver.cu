@@ -198,19 +198,48 @@ double nint_host(double x) { // md_driver.hpp:48-50
 //   216,000   0.869 / 0.870 / 0.979       0.603 / 0.469 / 0.474 / 0.578
 //   640,000   2.55 / 2.56 / 2.86          1.72 / 1.31 / 1.37 / 1.69
 // In a mixed step, whose passes find colder caches, 8 lanes lead longer: 0.0755 against 0.0903 ms at
-// 13,500 atoms, 0.0833 / 0.0952 at 16,384, 0.0950 / 0.0950 at 19,652, 0.1026 / 0.1008 at 23,328
-// (ternary 0.1156 / 0.1178).
+// 13,500 atoms, 0.0833 / 0.0952 at 16,384, 0.0950 / 0.0950 at 19,652, 0.1026 / 0.1008 at 23,328;
+// from 28,000 on 4 lead for two elements and for three (0.1125 / 0.1206 and 0.1485 / 0.1522 at 32,000;
+// ternary at 27,436 0.1406 / 0.1242).
+//
+// A warp per atom (kWideTpa) while all atom slots at 32 lanes stay within 3 blocks per SM (1,536
+// slots, each replica padded to 256), what the FP64 force pass holds at once. A pass over so few atoms
+// is the latency of its longest row, which 32 lanes walk in half the iterations. Density / force pass /
+// step in us, 16 and 32 lanes per atom:
+//   atoms       FP64 16               FP64 32               mixed 16              mixed 32
+//   500         14.2 / 16.3 / 46.2    10.8 / 12.3 / 41.1    12.2 / 12.5 / 40.2    10.3 / 12.3 / 38.1
+//   1,372       14.3 / 17.3 / 48.9    12.2 / 14.4 / 44.7    12.3 / 14.3 / 44.0    10.3 / 12.4 / 41.1
+//   2,048       14.4 / 18.4 / 51.4    12.3 / 20.5 / 53.4    12.3 / 14.3 / 45.4    11.1 / 14.4 / 45.3
+//   4,000       16.4 / 28.9 / 69.8    18.4 / 28.7 / 67.2    12.3 / 16.5 / 54.0    12.5 / 20.5 / 54.1
+// It is the default and a candidate of the tuners there; set_launch and MDELAST_TPA name 1, 4, 8 and
+// 16 and get what they name.
+constexpr int kWideTpa = 32;
+constexpr long kWideBlocks = 148 * 3;
+bool wide_fits(long slots) { return slots / kBlock * kWideTpa <= kWideBlocks; }
+
 // MDELAST_TPA overrides it.
-int default_tpa(long n_atoms, bool mixed) {
+int default_tpa(long n_atoms, long slots, bool mixed) {
     if (char const *e = std::getenv("MDELAST_TPA")) {
         int const v = std::atoi(e);
         if (valid_tpa(v))
             return v;
     }
+    if (wide_fits(slots))
+        return kWideTpa;
     if (n_atoms < (mixed ? 5000 : 8000))
         return 16;
     return mixed && n_atoms >= 28000 ? 4 : 8;
 }
+
+// the tuners' lanes per atom, and how their choice is reported: the wide shape as 16, the nearest that
+// set_launch takes
+std::vector<int> tuner_tpas(long slots) {
+    std::vector<int> v{1, 4, 8, 16};
+    if (wide_fits(slots))
+        v.push_back(kWideTpa);
+    return v;
+}
+int named_tpa(int tpa) { return std::min(tpa, 16); }
 
 // Deal the blocks of a pair pass out to the replicas in proportion to their atom counts:
 // about `target` in all (a multiple of the 148 SMs: a block then loops over several atom
@@ -219,22 +248,6 @@ int default_tpa(long n_atoms, bool mixed) {
 // replica map; returns the grid size.
 constexpr int kTargetBlocks = 148 * 32;
 
-// Lanes per atom a pass is launched with: 16 becomes 32, a warp per atom, while all atoms at 32
-// lanes stay within 3 blocks per SM (1,536 atoms), what the FP64 force pass holds at once. A pass over
-// so few atoms is the latency of its longest row, which 32 lanes walk in half the iterations. Density /
-// force pass / step in us, 16 and 32 lanes per atom:
-//   atoms       FP64 16               FP64 32               mixed 16              mixed 32
-//   500         14.2 / 16.3 / 46.2    10.8 / 12.3 / 41.1    12.2 / 12.5 / 40.2    10.3 / 12.3 / 38.1
-//   1,372       14.3 / 17.3 / 48.9    12.2 / 14.4 / 44.7    12.3 / 14.3 / 44.0    10.3 / 12.4 / 41.1
-//   2,048       14.4 / 18.4 / 51.4    12.3 / 20.5 / 53.4    12.3 / 14.3 / 45.4    11.1 / 14.4 / 45.3
-//   4,000       16.4 / 28.9 / 69.8    18.4 / 28.7 / 67.2    12.3 / 16.5 / 54.0    12.5 / 20.5 / 54.1
-constexpr long kWideBlocks = 148 * 3;
-int lanes_per_atom(std::vector<Replica *> const &reps, int tpa) {
-    long total = 0;
-    for (Replica const *r : reps)
-        total += r->n_blocks;
-    return tpa == 16 && total * 32 <= kWideBlocks ? 32 : tpa;
-}
 // shared memory for the staged force tables: the rest of the SM's 228 KB is the L1 of the
 // partner gathers
 constexpr long kStageBudget = 184 * 1024;
@@ -296,8 +309,7 @@ struct mdelast_driver_s {
     bool cell_staging = true;
     cudaStream_t stream = nullptr;
     int N = 0, n_pad = 0, n_rep = 1, ntypes = 0, npot = 0, n_blocks = 0;
-    int tpa_d = 1, tpa_f = 1; // lanes per atom of the density and force passes, as chosen ...
-    int lanes_d = 1, lanes_f = 1; // ... and as launched (lanes_per_atom)
+    int tpa_d = 1, tpa_f = 1; // lanes per atom of the density and force passes
     int grid_d = 1, grid_f = 1; // blocks of the density and force passes
     int *d_dblk_rep = nullptr, *d_fblk_rep = nullptr;
     int neighbors = 0;
@@ -318,9 +330,9 @@ struct mdelast_driver_s {
     float *d_phf = nullptr, *d_phq = nullptr, *d_rrf = nullptr, *d_rdf = nullptr;
     void pass_density(bool obs, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED)
-            launch_density_mx(obs, lanes_d, grid_d, s, A, T);
+            launch_density_mx(obs, tpa_d, grid_d, s, A, T);
         else
-            launch_density(obs, lanes_d, grid_d, s, A, T);
+            launch_density(obs, tpa_d, grid_d, s, A, T);
     }
     // force pass with the staged shared-memory tables (mixed precision, quintic, when the
     // tables were staged; chosen by the autotuner or set_force_staging)
@@ -331,11 +343,11 @@ struct mdelast_driver_s {
     }
     void pass_force(bool obs, bool kick, cudaStream_t s) {
         if (precision == MDELAST_PRECISION_MIXED && stage_f && T.st_n > 0)
-            launch_force_mx_staged(obs, kick, lanes_f, grid_f, s, A, T);
+            launch_force_mx_staged(obs, kick, tpa_f, grid_f, s, A, T);
         else if (precision == MDELAST_PRECISION_MIXED)
-            launch_force_mx(obs, kick, lanes_f, grid_f, s, A, T);
+            launch_force_mx(obs, kick, tpa_f, grid_f, s, A, T);
         else
-            launch_force(obs, kick, lanes_f, grid_f, s, A, T);
+            launch_force(obs, kick, tpa_f, grid_f, s, A, T);
     }
     int *d_nbr = nullptr, *d_nup = nullptr, *d_ndn = nullptr;
     // pair list of the pair passes (see AtomsView::pnbr); pair_factor 0: the neighbour list
@@ -595,7 +607,8 @@ int mdelast_driver_s::alloc_cells(int n_cells, int cell_cap) {
 // ranges, block -> replica maps, per-block and per-chunk partial-sum buffers. The step
 // graphs hold the old shapes and are dropped. Call with no work in flight.
 int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, int staged) {
-    if (!valid_tpa(tpa_d_) || !valid_tpa(tpa_f_) || tgt_d < 1 || tgt_f < 1)
+    auto runs = [&](int tpa) { return valid_tpa(tpa) || (tpa == kWideTpa && wide_fits(n_pad)); };
+    if (!runs(tpa_d_) || !runs(tpa_f_) || tgt_d < 1 || tgt_f < 1)
         return fail(MDELAST_ERR_ARGUMENT, "bad launch shape");
     bool const st = staged < 0 ? stage_f : staged != 0;
     if (st && !staging_available())
@@ -610,9 +623,8 @@ int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, i
     for (auto &x : R)
         reps.push_back(&x);
     std::vector<int> dmap, fmap;
-    int const ld = lanes_per_atom(reps, tpa_d_), lf = lanes_per_atom(reps, tpa_f_);
-    int const gd = deal_blocks(reps, ld, true, dmap, tgt_d);
-    int const gf = deal_blocks(reps, lf, false, fmap, tgt_f, st ? kStagedBlock : kBlock);
+    int const gd = deal_blocks(reps, tpa_d_, true, dmap, tgt_d);
+    int const gf = deal_blocks(reps, tpa_f_, false, fmap, tgt_f, st ? kStagedBlock : kBlock);
     int chunks = 1;
     for (Replica const *x : reps)
         chunks = std::max(chunks, (std::max(x->dblk_n, x->fblk_n) + kChunk - 1) / kChunk);
@@ -647,8 +659,6 @@ int mdelast_driver_s::set_launch(int tpa_d_, int tpa_f_, int tgt_d, int tgt_f, i
         return rc;
     tpa_d = tpa_d_;
     tpa_f = tpa_f_;
-    lanes_d = ld;
-    lanes_f = lf;
     target_d = tgt_d;
     target_f = tgt_f;
     stage_f = st;
@@ -718,7 +728,7 @@ int mdelast_driver_s::time_steps(int n, int rebuild_every, double *ms_d, double 
 int mdelast_driver_s::tune_on_steps(int n, int rebuild_every, int *choice, double *ms) {
     double best_d = 1e300, best_f = 1e300;
     int bd[2] = {tpa_d, target_d}, bf[3] = {tpa_f, target_f, stage_f ? 1 : 0};
-    for (int tp : {1, 4, 8, 16})
+    for (int tp : tuner_tpas(n_pad))
         for (int tg : {148 * 16, 148 * 32, 148 * 64}) {
             if (int rc = set_launch(tp, bf[0], tg, bf[1], bf[2]))
                 return rc;
@@ -735,7 +745,7 @@ int mdelast_driver_s::tune_on_steps(int n, int rebuild_every, int *choice, doubl
         int tpa, target, staged;
     };
     std::vector<Shape> shapes;
-    for (int tp : {1, 4, 8, 16})
+    for (int tp : tuner_tpas(n_pad))
         for (int tg : {148 * 8, 148 * 16, 148 * 32})
             shapes.push_back({tp, tg, 0});
     if (staging_available())
@@ -757,8 +767,8 @@ int mdelast_driver_s::tune_on_steps(int n, int rebuild_every, int *choice, doubl
     }
     if (int rc = set_launch(bd[0], bf[0], bd[1], bf[1], bf[2]))
         return rc;
-    choice[0] = bd[0];
-    choice[1] = bf[0];
+    choice[0] = named_tpa(bd[0]);
+    choice[1] = named_tpa(bf[0]);
     choice[2] = bd[1];
     choice[3] = bf[1];
     ms[0] = best_d;
@@ -1630,11 +1640,10 @@ static int create_system(const mdelast_driver_config *cfgs, int n_rep, mdelast_d
         set_chain(x.bth, c.baro_thermo_T, c.baro_nchain, c.baro_q, c.baro_p_eta, c.baro_Nf);
         reps.push_back(&x);
     }
-    d->tpa_d = d->tpa_f = default_tpa(n_total, c0.precision == MDELAST_PRECISION_MIXED);
+    d->tpa_d = d->tpa_f = default_tpa(n_total, np, c0.precision == MDELAST_PRECISION_MIXED);
     std::vector<int> dmap, fmap;
-    d->lanes_d = d->lanes_f = lanes_per_atom(reps, d->tpa_d);
-    d->grid_d = deal_blocks(reps, d->lanes_d, true, dmap);
-    d->grid_f = deal_blocks(reps, d->lanes_f, false, fmap);
+    d->grid_d = deal_blocks(reps, d->tpa_d, true, dmap);
+    d->grid_f = deal_blocks(reps, d->tpa_f, false, fmap);
     TRY(dalloc_later(&d->d_dblk_rep, dmap.size()));
     TRY(dalloc_later(&d->d_fblk_rep, fmap.size()));
     d->cap_dmap = dmap.size();
@@ -2146,11 +2155,10 @@ int mdelast_driver_autotune(mdelast_driver *d, int32_t n_repeat, int32_t *choice
     CK(cudaSetDevice(d->device));
     if (int rc = d->wait_step())
         return rc;
-    int const tpas[4] = {1, 4, 8, 16};
     int const targets[4] = {148 * 8, 148 * 16, 148 * 32, 148 * 64};
     double best_d = 1e300, best_f = 1e300;
     int bd[2] = {d->tpa_d, d->target_d}, bf[3] = {d->tpa_f, d->target_f, d->stage_f ? 1 : 0};
-    for (int tp : tpas)
+    for (int tp : tuner_tpas(d->n_pad))
         for (int tg : targets) {
             if (int rc = d->set_launch(tp, tp, tg, tg, 0))
                 return rc;
@@ -2171,8 +2179,10 @@ int mdelast_driver_autotune(mdelast_driver *d, int32_t n_repeat, int32_t *choice
         }
     // the staged force pass: one 512-thread block per SM, one to four waves
     if (d->staging_available())
-        for (int tp : {4, 8, 16})
+        for (int tp : tuner_tpas(d->n_pad))
             for (int tg : {148, 148 * 2, 148 * 4}) {
+                if (tp == 1)
+                    continue; // not a staged shape
                 if (int rc = d->set_launch(bd[0], tp, bd[1], tg, 1))
                     return rc;
                 double md = 0., mf = 0.;
@@ -2192,8 +2202,8 @@ int mdelast_driver_autotune(mdelast_driver *d, int32_t n_repeat, int32_t *choice
     if (int rc = d->time_passes(1, 1, &md, &mf))
         return rc;
     if (choice) {
-        choice[0] = bd[0];
-        choice[1] = bf[0];
+        choice[0] = named_tpa(bd[0]);
+        choice[1] = named_tpa(bf[0]);
         choice[2] = bd[1];
         choice[3] = bf[1];
     }
@@ -2237,6 +2247,8 @@ int mdelast_driver_set_launch(mdelast_driver *d, int32_t tpa_density, int32_t tp
     CK(cudaSetDevice(d->device));
     if (int rc = d->wait_step())
         return rc;
+    if (!valid_tpa(tpa_density) || !valid_tpa(tpa_force))
+        return fail(MDELAST_ERR_ARGUMENT, "bad launch shape");
     if (int rc = d->set_launch(tpa_density, tpa_force, blocks_density, blocks_force))
         return rc;
     double md = 0., mf = 0.;

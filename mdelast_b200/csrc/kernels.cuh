@@ -49,7 +49,7 @@ constexpr int kCellSortWarps = 8;      // half cells per k_cell_sort block (one 
 constexpr int kNbrCellsThreads = 256;   // threads of a k_nbr_cells block (one 2x2x2 half-cell group)
 constexpr size_t kNbrCellsStaticSmem = 4 * 1024; // bound on k_nbr_cells' static shared memory
 // launchers of the templated pair kernels (defined beside them); tpa = lanes per atom,
-// one of 1, 4, 8, 16 (valid_tpa)
+// one of 1, 4, 8, 16 (valid_tpa: what callers may name) or 32
 bool valid_tpa(int tpa);
 void launch_density(bool obs, int tpa, int grid, cudaStream_t s, AtomsView const &A,
                     TablesView const &T);
