@@ -1296,16 +1296,16 @@ __global__ void k_sub_invalidate(AtomsView A) {
 
 // ------------------------------------------------------------------------------------
 // Readout of one per-atom field in the C-ABI layout (x, y, z interleaved per atom) for
-// replica r, applying the deferred velocity factor. One value per thread: `out` is pinned host memory,
-// and a warp's stores are contiguous.
+// replica r, applying the deferred velocity factor: the values from `first` on, `n` of them, to
+// out[0..n). One value per thread: `out` is pinned host memory, and a warp's stores are contiguous.
 
-__global__ void k_readout(AtomsView A, TablesView T, int r, int field, double *out,
+__global__ void k_readout(AtomsView A, TablesView T, int r, int field, int first, int n, double *out,
                           const double *pos0, int stepped) {
     Replica const *R = A.rep + r;
-    int const e = blockIdx.x * blockDim.x + threadIdx.x;
+    int const q = blockIdx.x * blockDim.x + threadIdx.x, e = first + q;
     bool const vec = field <= MDELAST_ATOM_FORCES;
     int const a = vec ? e / 3 : e, k = vec ? e - 3 * a : 0;
-    if (a >= R->n_atoms)
+    if (q >= n || a >= R->n_atoms)
         return;
     int const i = R->atom_begin + a;
     size_t const at = static_cast<size_t>(k) * A.n_pad + i; // component k of an SoA field
@@ -1349,7 +1349,7 @@ __global__ void k_readout(AtomsView A, TablesView T, int r, int field, double *o
     default:
         return;
     }
-    out[e] = v;
+    out[q] = v;
 }
 
 // The reference-format half list of replica r: for each atom its partners j > i, in

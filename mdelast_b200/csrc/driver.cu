@@ -116,6 +116,9 @@ struct PinnedBlock {
     size_t bytes = 0;
 };
 constexpr size_t kPinnedKeep = 16, kPinnedKeepBytes = 64u << 20;
+// a driver's readout block at most: larger fields take several pieces, so that no driver holds pinned
+// memory in proportion to its atoms
+constexpr size_t kReadoutBytes = 4u << 20;
 std::mutex g_pinned_mutex;
 std::vector<PinnedBlock> g_pinned;
 
@@ -133,7 +136,12 @@ int pinned_take(PinnedBlock &b, size_t bytes) {
             return MDELAST_OK;
         }
     }
-    CK(cudaHostAlloc(&b.p, bytes, cudaHostAllocPortable));
+    cudaError_t const e = cudaHostAlloc(&b.p, bytes, cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+        cudaGetLastError(); // callers may go on without
+        b = PinnedBlock{};
+        return fail(MDELAST_ERR_CUDA, "pinned host memory: %s", cudaGetErrorString(e));
+    }
     b.bytes = bytes;
     return MDELAST_OK;
 }
@@ -1948,22 +1956,42 @@ static int get_atoms_r(mdelast_driver *d, int r, int32_t field, double *out) {
     CK(cudaSetDevice(d->device));
     if (int rc = d->wait_step())
         return rc;
-    // the kernel writes the field straight into pinned memory
-    int const N = d->rep_count[r];
-    size_t const n = field <= MDELAST_ATOM_FORCES ? 3 * static_cast<size_t>(N) : N;
+    int const N = d->rep_count[r], n = field <= MDELAST_ATOM_FORCES ? 3 * N : N;
+    auto read = [&](int first, int m, double *to) {
+        k_readout<<<static_cast<unsigned>((m + 255) / 256), 256, 0, d->stream>>>(
+            d->A, d->T, r, field, first, m, to, d->d_pos0 + d->pos0_off[r], d->stepped ? 1 : 0);
+        return cudaGetLastError();
+    };
     if (!d->out_block.p) {
         size_t most = 0;
         for (int c : d->rep_count)
             most = std::max(most, static_cast<size_t>(c));
-        if (int rc = pinned_take(d->out_block, 3 * sizeof(double) * most))
-            return rc;
+        if (pinned_take(d->out_block, std::min(3 * sizeof(double) * most, kReadoutBytes)))
+            clear_error();
     }
+    if (!d->out_block.p) { // no pinned memory to be had: through a device buffer
+        double *tmp = nullptr;
+        if (int rc = dalloc(&tmp, static_cast<size_t>(n)))
+            return rc;
+        cudaError_t e = read(0, n, tmp);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(out, tmp, sizeof(double) * n, cudaMemcpyDeviceToHost, d->stream);
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(d->stream);
+        dfree(tmp);
+        if (e != cudaSuccess)
+            return fail(MDELAST_ERR_CUDA, "atom readout: %s", cudaGetErrorString(e));
+        return MDELAST_OK;
+    }
+    // the kernel writes the field straight into pinned memory, a block's worth at a time
     double *const host = static_cast<double *>(d->out_block.p);
-    k_readout<<<static_cast<unsigned>((n + 255) / 256), 256, 0, d->stream>>>(
-        d->A, d->T, r, field, host, d->d_pos0 + d->pos0_off[r], d->stepped ? 1 : 0);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(d->stream));
-    std::memcpy(out, host, sizeof(double) * n);
+    int const piece = static_cast<int>(std::min(d->out_block.bytes, kReadoutBytes) / sizeof(double));
+    for (int first = 0; first < n; first += piece) {
+        int const m = std::min(piece, n - first);
+        CK(read(first, m, host));
+        CK(cudaStreamSynchronize(d->stream));
+        std::memcpy(out + first, host, sizeof(double) * m);
+    }
     return MDELAST_OK;
 }
 

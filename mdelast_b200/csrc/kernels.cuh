@@ -79,7 +79,7 @@ void launch_sublist(int grid, size_t smem, cudaStream_t s, AtomsView const &A);
 constexpr size_t kSublistSortMax = 150 * 1024;
 __host__ __device__ size_t sublist_smem(int maxn);
 __global__ void k_sub_invalidate(AtomsView A);
-__global__ void k_readout(AtomsView A, TablesView T, int r, int field, double *out,
+__global__ void k_readout(AtomsView A, TablesView T, int r, int field, int first, int n, double *out,
                           const double *pos0, int stepped);
 __global__ void k_half_list_counts(AtomsView A, int r, int *counts);
 __global__ void k_half_list_fill(AtomsView A, int r, const int *point, int *out);
