@@ -843,12 +843,25 @@ void mdelast_driver_s::drop_graphs() {
         }
 }
 
-// All-pairs search even where cells fit: replicas of at most kBruteAtoms atoms, and up to
-// kBruteIdle while the batch's 2 x 2 x 2 groups of half cells (a block each) leave SMs idle. A warp per atom
-// fills them. List build and pair-list refresh, cells against all pairs: 500 atoms 0.051 / 0.028 ms,
-// 2,048 atoms 0.141 / 0.053 ms, 2,916 atoms 0.151 / 0.067 ms; 4,000 atoms on cells
-// 0.101 ms.
-constexpr int kBruteAtoms = 1000, kBruteIdle = 3000;
+// All-pairs search even where cells fit (a warp per atom fills the SMs where the groups of 2 x 2 x 2 half
+// cells, a block each, leave them idle): replicas of at most kBruteAtoms atoms; of at most kBruteFew
+// while the batch has at most kBruteRows atoms in replicas of that size; and of at most kBruteIdle
+// while the batch's groups are fewer than the SMs. List build and pair-list refresh in ms, cells / all
+// pairs (mixed; FP64 within 4 %), generic alloy of the list radius given:
+//   atoms   radius   1 replica         16                64                256
+//   500     5.4 A    0.050 / 0.027     -                 0.155 / 0.113     0.492 / 0.395
+//   600     5.4      -                 0.072 / 0.057     0.164 / 0.144     0.539 / 0.511
+//   700     5.4      -                 0.085 / 0.063     0.197 / 0.172     0.654 / 0.648
+//   700     4.2      -                 0.086 / 0.060     0.217 / 0.160     0.763 / 0.598
+//   720     5.4      -                 0.069 / 0.065     0.172 / 0.180     0.569 / 0.685
+//   864     5.4      0.050 / 0.032     0.072 / 0.076     0.192 / 0.232     0.658 / 0.918
+//   864     6.6      0.055 / 0.032     0.082 / 0.080     0.228 / 0.244     0.799 / 0.969
+//   1,000   5.4      0.050 / 0.034     0.096 / 0.096     0.263 / 0.297     0.931 / 1.195
+// From 720 atoms on the two cross between 10,000 atoms in all (864 at 5.4 A: 12 replicas 0.070 / 0.068) and
+// 35,000 (720 at 5.4 A). One replica: 2,048 atoms 0.141 / 0.053, 2,916 atoms 0.151 / 0.067, 4,000 on
+// cells 0.101.
+constexpr int kBruteAtoms = 700, kBruteFew = 1000, kBruteIdle = 3000;
+constexpr long kBruteRows = 18000;
 
 // Half cells per edge for the current box: twice the number of cells no thinner than the
 // list radius (with a margin for the box changes of an NPT run between rebuilds); fewer
@@ -859,18 +872,22 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
     // after what the stream still holds (a resumed launch clears status bits there)
     CK(cudaMemcpyAsync(R.data(), d_rep, sizeof(Replica) * n_rep, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    // whether the groups of every replica with cells together are fewer than the SMs
-    double groups = 0.;
+    // what the all-pairs search is worth here: the atoms in replicas between its two limits, and
+    // whether the groups of all replicas with cells together are fewer than the SMs
+    std::vector<double> group(static_cast<size_t>(n_rep), 1.); // 0: too narrow for cells
+    long rows = 0;
     for (int q = 0; q < n_rep; ++q) {
-        double g = 1.;
-        bool fits = rep_count[q] > kBruteAtoms;
         for (int a = 0; a < 3; ++a) {
             double const c = std::floor(boxes[3 * q + a] / (r_list * 1.05));
-            fits = fits && c >= 3.;
-            g *= c;
+            group[q] *= c >= 3. ? c : 0.;
         }
-        groups += fits ? g : 0.;
+        if (group[q] > 0. && rep_count[q] > kBruteAtoms && rep_count[q] <= kBruteFew)
+            rows += rep_count[q];
     }
+    int const small = rows <= kBruteRows ? kBruteFew : kBruteAtoms;
+    double groups = 0.;
+    for (int q = 0; q < n_rep; ++q)
+        groups += rep_count[q] > small ? group[q] : 0.;
     bool const idle = groups < 148.;
     bool changed = false, all_brute = true;
     int n_cells = 0, cap = std::max(A.cell_cap, 32);
@@ -883,7 +900,7 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
                 brute = true;
             nc[a] *= 2;
         }
-        brute = brute || rep_count[q] <= kBruteAtoms || (idle && rep_count[q] <= kBruteIdle);
+        brute = brute || rep_count[q] <= small || (idle && rep_count[q] <= kBruteIdle);
         if (brute)
             nc[0] = nc[1] = nc[2] = 0;
         Replica &r = R[static_cast<size_t>(q)];
