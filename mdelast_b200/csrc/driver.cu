@@ -846,7 +846,8 @@ void mdelast_driver_s::drop_graphs() {
 // All-pairs search even where cells fit (a warp per atom fills the SMs where the groups of 2 x 2 x 2 half
 // cells, a block each, leave them idle): replicas of at most kBruteAtoms atoms; of at most kBruteFew
 // while the batch has at most kBruteRows atoms in replicas of that size; and of at most kBruteIdle
-// while the batch's groups are fewer than the SMs. List build and pair-list refresh in ms, cells / all
+// while the batch's groups are fewer than the SMs and the pair tests of these replicas at most
+// kBruteTests per atom of a group. List build and pair-list refresh in ms, cells / all
 // pairs (mixed; FP64 within 4 %), generic alloy of the list radius given:
 //   atoms   radius   1 replica         16                64                256
 //   500     5.4 A    0.050 / 0.027     -                 0.155 / 0.113     0.492 / 0.395
@@ -858,10 +859,19 @@ void mdelast_driver_s::drop_graphs() {
 //   864     6.6      0.055 / 0.032     0.082 / 0.080     0.228 / 0.244     0.799 / 0.969
 //   1,000   5.4      0.050 / 0.034     0.096 / 0.096     0.263 / 0.297     0.931 / 1.195
 // From 720 atoms on the two cross between 10,000 atoms in all (864 at 5.4 A: 12 replicas 0.070 / 0.068) and
-// 35,000 (720 at 5.4 A). One replica: 2,048 atoms 0.141 / 0.053, 2,916 atoms 0.151 / 0.067, 4,000 on
-// cells 0.101.
+// 35,000 (720 at 5.4 A). Above 1,000, groups idle: all pairs take 0.035 ms and 0.0043 per million tests,
+// the cells the latency of a group, which grows with its atoms:
+//   atoms   radius   atoms a group   1 replica         2                 3                 5
+//   1,372   6.6 A    51              0.073 / 0.040     0.074 / 0.041     0.075 / 0.046     0.084 / 0.070
+//   2,048   7.2      76              0.116 / 0.052     0.118 / 0.060     0.127 / 0.090     -
+//   2,048   8.2      76              0.139 / 0.054     0.142 / 0.062     0.153 / 0.094     0.156 / 0.127
+//   2,916   8.2      108             0.147 / 0.067     0.153 / 0.113     0.162 / 0.127     0.172 / 0.218
+//   2,916   6.6      46              0.068 / 0.064     0.073 / 0.107     0.083 / 0.118     -
+//   2,916   6.0      23              0.056 / 0.064     0.066 / 0.107     -                 -
+// 4,000 atoms at 8.2 A on cells 0.101.
 constexpr int kBruteAtoms = 700, kBruteFew = 1000, kBruteIdle = 3000;
 constexpr long kBruteRows = 18000;
+constexpr double kBruteTests = 280000.;
 
 // Half cells per edge for the current box: twice the number of cells no thinner than the
 // list radius (with a margin for the box changes of an NPT run between rebuilds); fewer
@@ -872,8 +882,9 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
     // after what the stream still holds (a resumed launch clears status bits there)
     CK(cudaMemcpyAsync(R.data(), d_rep, sizeof(Replica) * n_rep, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    // what the all-pairs search is worth here: the atoms in replicas between its two limits, and
-    // whether the groups of all replicas with cells together are fewer than the SMs
+    // what the all-pairs search is worth here: the atoms in replicas between its first two limits;
+    // whether the groups of all replicas with cells together are fewer than the SMs, and the pair tests,
+    // atoms and groups of those up to the last limit
     std::vector<double> group(static_cast<size_t>(n_rep), 1.); // 0: too narrow for cells
     long rows = 0;
     for (int q = 0; q < n_rep; ++q) {
@@ -885,10 +896,18 @@ int mdelast_driver_s::configure_cells(std::vector<double> const &boxes) {
             rows += rep_count[q];
     }
     int const small = rows <= kBruteRows ? kBruteFew : kBruteAtoms;
-    double groups = 0.;
-    for (int q = 0; q < n_rep; ++q)
-        groups += rep_count[q] > small ? group[q] : 0.;
-    bool const idle = groups < 148.;
+    double groups = 0., tests = 0., atoms = 0., tested = 0.;
+    for (int q = 0; q < n_rep; ++q) {
+        if (rep_count[q] <= small)
+            continue;
+        groups += group[q];
+        if (group[q] > 0. && rep_count[q] <= kBruteIdle) {
+            tests += static_cast<double>(rep_count[q]) * rep_count[q];
+            atoms += rep_count[q];
+            tested += group[q];
+        }
+    }
+    bool const idle = groups < 148. && tests * tested <= kBruteTests * atoms;
     bool changed = false, all_brute = true;
     int n_cells = 0, cap = std::max(A.cell_cap, 32);
     for (int q = 0; q < n_rep; ++q) {
