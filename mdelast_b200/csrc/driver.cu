@@ -2129,6 +2129,8 @@ static int pair_correlation_r(mdelast_driver *d, int r, int32_t mode) {
     GrArgs g{};
     g.crd = d->d_crd + d->rep_begin[r];
     g.rep = d->d_rep + r;
+    for (int a = 0; a < 3; ++a)
+        g.box[a] = d->h_obs[r].box[4 * a];
     g.n = d->rep_count[r];
     g.ntypes = d->ntypes;
     g.n_rg = d->gr_n[r];

@@ -8,6 +8,9 @@
 // the normalisation repeats the reference's operation order without contraction, so g(r)
 // equals the reference's to the last bit.
 //
+// Two kernels: k_gr_count with an FP32 estimate, described here, and k_gr_count_far without, for
+// what gr_enqueue's rule leaves to it.
+//
 // Work split: units of one pair of 128-atom tiles (I <= J) of the replica, dealt to as many
 // blocks as fit the SMs; the J tile is staged in shared memory and each thread scans half of it for
 // its own atom of tile I. A block keeps its histogram in shared memory over all its units and
@@ -37,7 +40,16 @@ constexpr size_t kGrSharedMax = 96 * 1024;
 constexpr int kGrThreads = 2 * kGrTile;
 constexpr int kGrQueue = 1024;                  // pairs of a unit that wait for the FP64 test
 constexpr long kGrFlushUnits = 100000;          // 32-bit counts: flushed before 2^32 pairs
-constexpr float kGrMaxMargin = 0.05f;           // beyond it every pair takes the FP64 test
+constexpr float kGrMaxMargin = 0.05f;           // beyond it k_gr_count_far counts
+// A total histogram beyond shared memory takes k_gr_count_far above this number of units: below, the
+// estimate's shorter chain counts, above, its share of the SMs' threads (38,000 bins, far / estimate: 2,048
+// atoms 0.175 / 0.163 ms, 4,000 0.184 / 0.194, 42,592 4.21 / 4.91).
+constexpr long kGrFarUnits = 148 * 2;
+// Partial histograms are kept per block up to kGrSharedFew bytes, beyond that (two blocks or three per
+// SM) where at least kGrFew of all pairs lie within rmaxg and would be atomics elsewhere (42,592 atoms, three
+// of 8,000 bins: to 8 A 2.17 ms in shared memory, 1.73 not; to half the box 2.99 and above 4).
+constexpr size_t kGrSharedFew = 48 * 1024;
+constexpr double kGrFew = 0.05;
 static_assert(kGrTile == 128, "a queue entry holds two 7-bit tile offsets");
 
 // Bound on |estimate - dr / drg| in bins, for box edges of at most H bins and distances of at most
@@ -45,7 +57,7 @@ static_assert(kGrTile == 128, "a queue entry holds two 7-bit tile offsets");
 // the box edge (2^-24 H) and the image (2^-25 H), 2^-22 H with room to spare, the same for either
 // image near half the box; the three squares, the sum, rsqrt.approx (2^-22.4) and the product
 // add less than 2^-21 of the distance.
-__device__ __forceinline__ float gr_margin(float H, float u) {
+__host__ __device__ __forceinline__ float gr_margin(float H, float u) {
     return 1.7321f * 2.3842e-7f * H + 4.7684e-7f * u;
 }
 
@@ -55,11 +67,17 @@ __device__ __forceinline__ float round_small(float x) {
     return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f);
 }
 
-// the reference's operations: the pair's bin, or -1
+// the reference's operations: the pair's bin, or -1. From r2_skip on certainly dr >= rmaxg.
+__device__ __forceinline__ double gr_r2_skip(GrArgs const &g) {
+    return g.rmaxg * g.rmaxg * (1. + 1e-12);
+}
 __device__ __forceinline__ int gr_bin_exact(GrArgs const &g, double4 ci, double4 cj, double hx,
-                                            double hy, double hz) {
+                                            double hy, double hz, double r2_skip) {
     double px, py, pz;
-    double const dr = __dsqrt_rn(min_image_r2(ci, cj, hx, hy, hz, px, py, pz));
+    double const r2 = min_image_r2(ci, cj, hx, hy, hz, px, py, pz);
+    if (r2 >= r2_skip)
+        return -1;
+    double const dr = __dsqrt_rn(r2);
     if (!(dr < g.rmaxg))
         return -1;
     int const b = static_cast<int>(floor(__ddiv_rn(dr, g.drg)));
@@ -80,7 +98,7 @@ __global__ void __launch_bounds__(kGrThreads) k_gr_count(GrArgs g, long units) {
     if (SHARED)
         for (int k = threadIdx.x; k < nbins; k += kGrThreads)
             s_hist[k] = 0u;
-    double const hx = g.rep->h[0], hy = g.rep->h[1], hz = g.rep->h[2];
+    double const hx = g.rep->h[0], hy = g.rep->h[1], hz = g.rep->h[2], r2_skip = gr_r2_skip(g);
     // positions and box in bins
     double const sx = hx / g.drg, sy = hy / g.drg, sz = hz / g.drg;
     float const Lx = static_cast<float>(sx), Ly = static_cast<float>(sy), Lz = static_cast<float>(sz);
@@ -88,8 +106,7 @@ __global__ void __launch_bounds__(kGrThreads) k_gr_count(GrArgs g, long units) {
     float const umax = static_cast<float>(g.rmaxg / g.drg);
     float const margin = gr_margin(fmaxf(Lx, fmaxf(Ly, Lz)), umax);
     // estimates below u_in are within rmaxg, from u_out on outside
-    bool const estimate = margin < kGrMaxMargin;
-    float const u_in = estimate ? umax - margin : -1.f, u_out = estimate ? umax + margin : 3.4e38f;
+    float const u_in = umax - margin, u_out = umax + margin;
     float const f_in = 0.5f - margin; // |fraction - 1/2| below it: away from both bin edges
     auto in_bins = [&](double4 c) {
         return make_float4(static_cast<float>((c.x - nint_ref(c.x)) * sx),
@@ -159,7 +176,7 @@ __global__ void __launch_bounds__(kGrThreads) k_gr_count(GrArgs g, long units) {
                     s_queue[at] = static_cast<unsigned short>(il << 7 | k);
                 } else {
                     double4 const cj = g.crd[j0 + k];
-                    int const b = gr_bin_exact(g, g.crd[i0 + il], cj, hx, hy, hz);
+                    int const b = gr_bin_exact(g, g.crd[i0 + il], cj, hx, hy, hz, r2_skip);
                     if (b >= 0)
                         count(b, ti, static_cast<int>(cj.w));
                 }
@@ -168,7 +185,7 @@ __global__ void __launch_bounds__(kGrThreads) k_gr_count(GrArgs g, long units) {
         __syncthreads();
         for (int e = threadIdx.x; e < min(s_n, kGrQueue); e += kGrThreads) {
             double4 const ci = g.crd[i0 + (s_queue[e] >> 7)], cj = g.crd[j0 + (s_queue[e] & 127)];
-            int const b = gr_bin_exact(g, ci, cj, hx, hy, hz);
+            int const b = gr_bin_exact(g, ci, cj, hx, hy, hz, r2_skip);
             if (b >= 0)
                 count(b, static_cast<int>(ci.w), static_cast<int>(cj.w));
         }
@@ -177,6 +194,40 @@ __global__ void __launch_bounds__(kGrThreads) k_gr_count(GrArgs g, long units) {
     }
     if (SHARED)
         flush();
+}
+
+// Every pair by the reference's operations, straight to the global counters, a block per unit: for
+// bins too fine for the estimate, and for a total histogram beyond shared memory, where the atomics
+// are the bound and the estimate gains nothing. In k_gr_count, bins too fine queued every pair, those
+// beyond rmaxg too: 42,592 atoms, bins of 0.0005 A to 6 A, 4.84 ms, here 1.71; bins of 0.0004 A to half
+// the box (100,000), total 5.72 ms, here 3.11.
+template <bool PARTIAL>
+__global__ void __launch_bounds__(kGrTile) k_gr_count_far(GrArgs g) {
+    __shared__ double4 sj[kGrTile];
+    int const T = (g.n + kGrTile - 1) / kGrTile;
+    long q = blockIdx.x;
+    int I = 0;
+    for (; q >= T - I; ++I)
+        q -= T - I;
+    int const j0 = (I + static_cast<int>(q)) * kGrTile, kmax = min(kGrTile, g.n - j0);
+    for (int k = threadIdx.x; k < kmax; k += kGrTile)
+        sj[k] = g.crd[j0 + k];
+    __syncthreads();
+    double const hx = g.rep->h[0], hy = g.rep->h[1], hz = g.rep->h[2], r2_skip = gr_r2_skip(g);
+    int const i = I * kGrTile + static_cast<int>(threadIdx.x);
+    if (i >= g.n)
+        return;
+    double4 const ci = g.crd[i];
+    int const ti = static_cast<int>(ci.w);
+    // the diagonal tile counts only j > i
+#pragma unroll 4
+    for (int k = q == 0 ? static_cast<int>(threadIdx.x) + 1 : 0; k < kmax; ++k) {
+        double4 const cj = sj[k];
+        int const b = gr_bin_exact(g, ci, cj, hx, hy, hz, r2_skip);
+        if (b >= 0)
+            atomicAdd(&g.counts[(PARTIAL ? 1 + pair_slot(ti, static_cast<int>(cj.w)) : 0) * g.n_rg + b],
+                      1ull);
+    }
 }
 
 __global__ void k_count_types(GrArgs g) {
@@ -247,20 +298,31 @@ cudaError_t gr_enqueue(GrArgs const &g, cudaStream_t s) {
         long const units = gr_count_blocks(g.n);
         int const rows = g.mode != 0 ? g.ntypes * (g.ntypes + 1) / 2 : 1;
         size_t const hist = sizeof(unsigned) * static_cast<size_t>(rows) * g.n_rg;
-        bool const shared_hist = hist <= kGrSharedMax;
-        size_t const smem = shared_hist ? hist : 0;
-        auto const kernel = g.mode != 0 ? (shared_hist ? k_gr_count<true, true> : k_gr_count<false, true>)
-                                        : (shared_hist ? k_gr_count<true, false> : k_gr_count<false, false>);
-        if (shared_hist)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kGrSharedMax));
-        int per_sm = 1;
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGrThreads, smem);
-        if (e != cudaSuccess)
-            return e;
-        long const blocks = std::min(units, 148L * std::max(per_sm, 1));
-        kernel<<<static_cast<unsigned>(blocks), kGrThreads, smem, s>>>(g, units);
+        // the part of all pairs that lies within rmaxg
+        double const V = g.box[0] * (g.box[1] * g.box[2]);
+        double const part = 4.2 * g.rmaxg * g.rmaxg * g.rmaxg / V;
+        double const edge = std::max(g.box[0], std::max(g.box[1], g.box[2]));
+        bool const estimate = gr_margin(static_cast<float>(edge / g.drg),
+                                        static_cast<float>(g.rmaxg / g.drg)) < kGrMaxMargin;
+        bool const shared_hist = hist <= kGrSharedMax && (g.mode == 0 || hist <= kGrSharedFew || part > kGrFew);
+        if (!estimate || (g.mode == 0 && !shared_hist && units > kGrFarUnits)) {
+            auto const far = g.mode == 0 ? k_gr_count_far<false> : k_gr_count_far<true>;
+            far<<<static_cast<unsigned>(units), kGrTile, 0, s>>>(g);
+        } else {
+            size_t const smem = shared_hist ? hist : 0;
+            auto const kernel = g.mode != 0 ? (shared_hist ? k_gr_count<true, true> : k_gr_count<false, true>)
+                                            : (shared_hist ? k_gr_count<true, false> : k_gr_count<false, false>);
+            if (shared_hist)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kGrSharedMax));
+            int per_sm = 1;
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGrThreads, smem);
+            if (e != cudaSuccess)
+                return e;
+            long const blocks = std::min(units, 148L * std::max(per_sm, 1));
+            kernel<<<static_cast<unsigned>(blocks), kGrThreads, smem, s>>>(g, units);
+        }
     }
     if (g.n > 0)
         k_count_types<<<(g.n + 255) / 256, 256, 0, s>>>(g);

@@ -12,6 +12,7 @@ struct Replica;
 struct GrArgs {
     const double4 *crd;      // the replica's scaled coordinates, type in .w (n entries)
     const Replica *rep;      // its state on the device: the current box edges h[3]
+    double box[3];           // the same edges, by which the host chooses the kernel
     int n, ntypes, n_rg, mode; // mode 0 total, 1 total + partial, 2 partial only
     const double *rg;        // bin centres (device), evenly spaced, rg[0] > 0
     double drg, rmaxg;       // rg[1] - rg[0], rg[n_rg - 1] + drg / 2 (md_driver.cpp:41)
