@@ -1437,11 +1437,11 @@ namespace {
 template <bool OBS, int IP, typename IX>
 void density_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesView const &T) {
     switch (tpa) {
-    case 1: launch_chain(k_density<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 4: launch_chain(k_density<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 8: launch_chain(k_density<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 16: launch_chain(k_density<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_density<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 1: launch_pass(tpa, k_density<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_pass(tpa, k_density<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_pass(tpa, k_density<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_pass(tpa, k_density<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_pass(tpa, k_density<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -1454,11 +1454,11 @@ void density_tpa(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesVi
 template <bool OBS, bool KICK, int IP, typename IX>
 void force_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A, TablesView const &T) {
     switch (tpa) {
-    case 1: launch_chain(k_force<OBS, KICK, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 4: launch_chain(k_force<OBS, KICK, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 8: launch_chain(k_force<OBS, KICK, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 16: launch_chain(k_force<OBS, KICK, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_force<OBS, KICK, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 1: launch_pass(tpa, k_force<OBS, KICK, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_pass(tpa, k_force<OBS, KICK, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_pass(tpa, k_force<OBS, KICK, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_pass(tpa, k_force<OBS, KICK, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_pass(tpa, k_force<OBS, KICK, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>

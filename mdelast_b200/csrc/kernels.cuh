@@ -11,19 +11,17 @@ namespace mdelast {
 // before every other access to memory and lets the next kernel of the chain do the same; a
 // kernel launched with launch_chain must call it first. It costs nothing in a plain launch.
 //
-// A grid of more than kChainBlocks blocks (4 per SM: more than an SM's worth of pair-pass blocks)
-// is launched plainly: its first blocks would start on SMs that still hold the previous kernel,
-// with the split of L1 and shared memory that one asked for, and a pass bound by the L1 loses more there
-// than a launch costs (64 x 2,048 atoms mixed: 0.416 ms per step plain, 0.440 chained
-// throughout, 0.404 so; one 500-atom cell: 0.063, 0.0505, 0.0505).
+// A grid of more than kChainBlocks blocks (4 per SM) is launched plainly: its first blocks would
+// start on SMs that still hold the previous kernel, with the split of L1 and shared memory that one
+// asked for. One 500-atom cell: 0.063 ms per step plain, 0.0505 chained.
 constexpr unsigned kChainBlocks = 148 * 4;
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
 }
 template <typename... P, typename... V>
-inline cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
-                                cudaStream_t s, V const &...args) {
+inline cudaError_t launch_chain_up_to(unsigned blocks, void (*kernel)(P...), dim3 grid, dim3 block,
+                                      size_t smem, cudaStream_t s, V const &...args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -33,8 +31,34 @@ inline cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, siz
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &at;
-    cfg.numAttrs = grid.x * grid.y <= kChainBlocks ? 1 : 0;
+    cfg.numAttrs = grid.x * grid.y <= blocks ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... V>
+inline cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t s, V const &...args) {
+    return launch_chain_up_to(kChainBlocks, kernel, grid, block, smem, s, args...);
+}
+
+// A pair pass with tpa lanes per atom is bound by the L1 and by its longest SM, and loses more to that
+// split and to blocks crowded onto the SMs that were free first than a launch costs, unless it is
+// latency alone: a warp per atom, or up to a block per SM of 16 lanes. Steps in ms, passes chained up
+// to 592 blocks / by this rule:
+//   atoms     FP64              mixed             FP64, 1 lane      mixed, 1 lane
+//   500       0.0381 / 0.0381   0.0379 / 0.0379   -                 -
+//   4,000     0.0625 / 0.0605   0.0505 / 0.0481   0.160 / 0.161     0.098 / 0.097
+//   8,788     0.0946 / 0.0894   0.0721 / 0.0684   -                 -
+//   13,500    0.0961 / 0.0959   0.0811 / 0.0812   0.226 / 0.178     0.153 / 0.115
+//   32,000    0.164 / 0.164     0.109 / 0.108     0.258 / 0.192     0.180 / 0.127
+// (64 x 2,048 atoms, mixed: 0.440 chained throughout, 0.404 plain.) With 4 or 8 lanes, 2,048 atoms
+// mixed 0.0517 / 0.0498 and 0.0453 / 0.0434. A warp per atom, 2 x 500 atoms FP64 (256
+// blocks): 0.0401 chained, 0.0404 to 0.0415 not; 1,372 atoms 0.0426 both.
+constexpr unsigned kChainPassBlocks = 148;
+template <typename... P, typename... V>
+inline cudaError_t launch_pass(int tpa, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t s, V const &...args) {
+    unsigned const most = tpa == 32 ? kChainBlocks : (tpa == 16 ? kChainPassBlocks : 0);
+    return launch_chain_up_to(most, kernel, grid, block, smem, s, args...);
 }
 
 // scalar-kernel modes

@@ -691,11 +691,11 @@ template <bool OBS, int IP, typename IX>
 void density_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                        TablesView const &T) {
     switch (tpa) {
-    case 1: launch_chain(k_density_mx<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 4: launch_chain(k_density_mx<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 8: launch_chain(k_density_mx<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    case 16: launch_chain(k_density_mx<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_density_mx<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 1: launch_pass(tpa, k_density_mx<OBS, 1, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_pass(tpa, k_density_mx<OBS, 4, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_pass(tpa, k_density_mx<OBS, 8, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_pass(tpa, k_density_mx<OBS, 16, IP, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_pass(tpa, k_density_mx<OBS, 32, IP, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, int IP>
@@ -709,11 +709,11 @@ template <bool OBS, bool KICK, int IP, typename IX>
 void force_mx_tpa_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
                      TablesView const &T) {
     switch (tpa) {
-    case 1: launch_chain(k_force_mx<OBS, KICK, 1, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
-    case 4: launch_chain(k_force_mx<OBS, KICK, 4, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
-    case 8: launch_chain(k_force_mx<OBS, KICK, 8, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
-    case 16: launch_chain(k_force_mx<OBS, KICK, 16, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
-    default: launch_chain(k_force_mx<OBS, KICK, 32, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 1: launch_pass(tpa, k_force_mx<OBS, KICK, 1, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 4: launch_pass(tpa, k_force_mx<OBS, KICK, 4, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 8: launch_pass(tpa, k_force_mx<OBS, KICK, 8, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    case 16: launch_pass(tpa, k_force_mx<OBS, KICK, 16, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
+    default: launch_pass(tpa, k_force_mx<OBS, KICK, 32, IP, false, IX>, grid, kBlock, 0, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK, int IP>
@@ -730,10 +730,10 @@ void force_mx_staged_ix(int tpa, int grid, cudaStream_t s, AtomsView const &A,
     size_t const smem = static_cast<size_t>(T.st_bytes);
     constexpr int Q = MDELAST_QUINTIC;
     switch (tpa) {
-    case 4: launch_chain(k_force_mx<OBS, KICK, 4, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
-    case 8: launch_chain(k_force_mx<OBS, KICK, 8, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
-    case 16: launch_chain(k_force_mx<OBS, KICK, 16, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
-    default: launch_chain(k_force_mx<OBS, KICK, 32, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    case 4: launch_pass(tpa, k_force_mx<OBS, KICK, 4, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    case 8: launch_pass(tpa, k_force_mx<OBS, KICK, 8, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    case 16: launch_pass(tpa, k_force_mx<OBS, KICK, 16, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
+    default: launch_pass(tpa, k_force_mx<OBS, KICK, 32, Q, true, IX>, grid, kBlockStaged, smem, s, A, T); break;
     }
 }
 template <bool OBS, bool KICK>
