@@ -1297,7 +1297,7 @@ __global__ void k_sub_invalidate(AtomsView A) {
 // ------------------------------------------------------------------------------------
 // Readout of one per-atom field in the C-ABI layout (x, y, z interleaved per atom) for
 // replica r, applying the deferred velocity factor: the values from `first` on, `n` of them, to
-// out[0..n). One value per thread: `out` is pinned host memory, and a warp's stores are contiguous.
+// out[0..n). One value per thread: `out` may be pinned host memory, and a warp's stores are contiguous.
 
 __global__ void k_readout(AtomsView A, TablesView T, int r, int field, int first, int n, double *out,
                           const double *pos0, int stepped) {

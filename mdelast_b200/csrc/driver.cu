@@ -116,9 +116,17 @@ struct PinnedBlock {
     size_t bytes = 0;
 };
 constexpr size_t kPinnedKeep = 16, kPinnedKeepBytes = 64u << 20;
-// a driver's readout block at most: larger fields take several pieces, so that no driver holds pinned
-// memory in proportion to its atoms
-constexpr size_t kReadoutBytes = 4u << 20;
+// Atom readouts of up to kReadoutBytes: the kernel writes the field straight into a pinned block, in
+// pieces of kReadoutPiece bytes that the host copies out while the next are written. Larger ones, and all
+// where pinned memory is refused, go through a device buffer. Positions in us, into memory in use /
+// into fresh pages:
+//   atoms      device buffer    pinned, one piece    512 KB pieces    256 KB
+//   13,500     46 / 171         37 / 127             38 / 122         36 / 121
+//   48,668     105 / 571        110 / 429            97 / 401         107 / 428
+//   108,000    190 / 1,205      227 / 1,008          195 / 990        235 / 1,020
+//   186,624    299 / 1,620      370 / 1,340          338 / 1,330      405 / 1,350
+//   500,000    727 / 3,450      -                    876 / 2,910      960 / 3,000
+constexpr size_t kReadoutPiece = 512u << 10, kReadoutBytes = 8 * kReadoutPiece;
 std::mutex g_pinned_mutex;
 std::vector<PinnedBlock> g_pinned;
 
@@ -395,7 +403,7 @@ struct mdelast_driver_s {
     int *d_cell_rep = nullptr;
     std::vector<int> cell_rep_host; // replica of each cell, as uploaded
     double *d_rb = nullptr, *d_Ft = nullptr;
-    double *d_pos0 = nullptr;
+    double *d_pos0 = nullptr, *d_out = nullptr; // d_out: large readouts (allocated at the first one)
     int *d_tmp_i = nullptr;
     size_t tmp_i_cap = 0;
 
@@ -415,9 +423,9 @@ struct mdelast_driver_s {
     AtomsView A{};
     TablesView T{};
     mdelast_observables *h_obs = nullptr; // pinned, n_rep entries (obs_block)
-    // pinned: the observables, and one replica's field of an atom readout (taken at the first one)
+    // pinned: the observables, and the block of atom readouts (taken at the first one)
     PinnedBlock obs_block, out_block;
-    cudaEvent_t ev_step = nullptr;
+    cudaEvent_t ev_step = nullptr, ev_out[kReadoutBytes / kReadoutPiece] = {}; // ev_out: pieces of a readout
     cudaGraphExec_t graph[8] = {}; // [4 * last + 2 * rebuild + obs]
     unsigned long long host_cycle = 0; // steps launched (the reference's cycle counter)
     int list_regrowths = 0;            // launches resumed after a list overflow
@@ -455,6 +463,9 @@ mdelast_driver_s::~mdelast_driver_s() {
             cudaGraphExecDestroy(g);
     if (ev_step)
         cudaEventDestroy(ev_step);
+    for (cudaEvent_t e : ev_out)
+        if (e)
+            cudaEventDestroy(e);
     cudaDeviceSynchronize(); // once for all buffers
     pinned_give(obs_block);
     pinned_give(out_block);
@@ -493,6 +504,7 @@ mdelast_driver_s::~mdelast_driver_s() {
     dfree_idle(d_rb);
     dfree_idle(d_Ft);
     dfree_idle(d_pos0);
+    dfree_idle(d_out);
     dfree_idle(d_tmp_i);
     dfree_idle(d_dblk_rep);
     dfree_idle(d_fblk_rep);
@@ -1998,35 +2010,36 @@ static int get_atoms_r(mdelast_driver *d, int r, int32_t field, double *out) {
             d->A, d->T, r, field, first, m, to, d->d_pos0 + d->pos0_off[r], d->stepped ? 1 : 0);
         return cudaGetLastError();
     };
-    if (!d->out_block.p) {
-        size_t most = 0;
-        for (int c : d->rep_count)
-            most = std::max(most, static_cast<size_t>(c));
-        if (pinned_take(d->out_block, std::min(3 * sizeof(double) * most, kReadoutBytes)))
-            clear_error();
-    }
-    if (!d->out_block.p) { // no pinned memory to be had: through a device buffer
-        double *tmp = nullptr;
-        if (int rc = dalloc(&tmp, static_cast<size_t>(n)))
-            return rc;
-        cudaError_t e = read(0, n, tmp);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(out, tmp, sizeof(double) * n, cudaMemcpyDeviceToHost, d->stream);
-        if (e == cudaSuccess)
-            e = cudaStreamSynchronize(d->stream);
-        dfree(tmp);
-        if (e != cudaSuccess)
-            return fail(MDELAST_ERR_CUDA, "atom readout: %s", cudaGetErrorString(e));
+    size_t const bytes = sizeof(double) * static_cast<size_t>(n);
+    size_t most = 0;
+    for (int c : d->rep_count)
+        most = std::max(most, 3 * sizeof(double) * static_cast<size_t>(c));
+    if (bytes <= kReadoutBytes && !d->out_block.p && pinned_take(d->out_block, std::min(most, kReadoutBytes)))
+        clear_error();
+    if (bytes > kReadoutBytes || !d->out_block.p) {
+        if (!d->d_out)
+            if (int rc = dalloc(&d->d_out, most / sizeof(double)))
+                return rc;
+        CK(read(0, n, d->d_out));
+        CK(cudaMemcpyAsync(out, d->d_out, bytes, cudaMemcpyDeviceToHost, d->stream));
+        CK(cudaStreamSynchronize(d->stream));
         return MDELAST_OK;
     }
-    // the kernel writes the field straight into pinned memory, a block's worth at a time
+    constexpr int kPiece = static_cast<int>(kReadoutPiece / sizeof(double));
     double *const host = static_cast<double *>(d->out_block.p);
-    int const piece = static_cast<int>(std::min(d->out_block.bytes, kReadoutBytes) / sizeof(double));
-    for (int first = 0; first < n; first += piece) {
-        int const m = std::min(piece, n - first);
-        CK(read(first, m, host));
-        CK(cudaStreamSynchronize(d->stream));
-        std::memcpy(out + first, host, sizeof(double) * m);
+    int const pieces = (n + kPiece - 1) / kPiece;
+    auto size = [&](int k) { return std::min(kPiece, n - k * kPiece); };
+    for (int k = 0; k < pieces; ++k) {
+        CK(read(k * kPiece, size(k), host + k * kPiece));
+        if (k + 1 == pieces)
+            break; // its end is the stream's
+        if (!d->ev_out[k])
+            CK(cudaEventCreateWithFlags(&d->ev_out[k], cudaEventDisableTiming));
+        CK(cudaEventRecord(d->ev_out[k], d->stream));
+    }
+    for (int k = 0; k < pieces; ++k) {
+        CK(k + 1 < pieces ? cudaEventSynchronize(d->ev_out[k]) : cudaStreamSynchronize(d->stream));
+        std::memcpy(out + k * kPiece, host + k * kPiece, sizeof(double) * size(k));
     }
     return MDELAST_OK;
 }
