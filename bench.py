@@ -813,8 +813,8 @@ def half_list_nbar(m, t, cell):
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_force_mx launch, keyed by
 # (precision, replicas, staged tables): single-pass captures of the bench command at 16
 # replicas without cache flushing (the launches of timed-region steps, so the L2 holds
-# what the preceding kernels of the step left in it), mean over the captured launches;
-# profiles/launches_bench_mixed_16x13500.md has the capture. None where not captured.
+# what the preceding kernels of the step left in it), mean over the captured launches.
+# None where not captured.
 TRAFFIC_PER_LAUNCH: dict = {("mixed", 16, False): 80.14e6 + 1.19e6,
                             ("mixed", 16, True): 78.89e6 + 0.77e6}
 

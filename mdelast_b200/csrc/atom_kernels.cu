@@ -595,8 +595,8 @@ __device__ __forceinline__ void pair_distance(double r2, double &dr, double &idr
 // over the lanes by warp_slots, one running sum per lane; with 23 warp sums per atom group
 // into shared accumulators the pass took 0.0397 instead of 0.0306 ms on 13,500 atoms (16 lanes
 // per atom; 0.0254 ms with 8 lanes, pair_distance and ld_crd). Bound by the L1 data pipe (75 % of its
-// wavefront rate, FP64 pipe 39 %). 6 blocks per SM: 5 and 7 are slower by 3 and 5 % on 108,000
-// atoms; 3 with 32 lanes, whose launches have no more (6 spill).
+// wavefront rate, FP64 pipe 39 %). 6 blocks per SM, where the sampled variant spills 28 bytes: 5 and 7
+// are slower by 3 and 5 % on 108,000 atoms; 3 with 32 lanes, whose launches have no more (6 spill).
 template <bool OBS, int TPA, int IP, typename IX>
 __global__ void __launch_bounds__(kBlock, TPA == 32 ? 3 : 6) k_density(AtomsView A, TablesView T) {
     chain_begin();
@@ -1237,7 +1237,8 @@ __host__ __device__ size_t sublist_smem(int maxn) {
     return b <= kSublistSortMax ? b : 0;
 }
 
-// 5 blocks of 256 threads per SM (the launch is 5 blocks per SM): at most 48 registers
+// 5 blocks of 256 threads per SM (the launch is 5 blocks per SM): at most 48 registers, 80 bytes of
+// spills in mixed precision
 template <bool F32>
 __global__ void __launch_bounds__(kRowThreads, 5) k_sublist(AtomsView A) {
     chain_begin();

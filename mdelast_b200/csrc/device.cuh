@@ -94,7 +94,7 @@ struct TablesView {
     const double *Ft; // [ntypes][nfi][6]
     int nfi, ntypes;
     double inv_hf, inv_hf2;
-    int has_eam, interp; // interp: MDELAST_QUINTIC or MDELAST_BSPLINE (bundle layout)
+    int has_eam, interp; // interp: MDELAST_QUINTIC or MDELAST_BSPLINE (record layout)
     double r_cut_sq; // pow<2>(pot[0]->rcut), md_driver.cpp:42
     double pot_rcut[kMaxTypes * (kMaxTypes + 1) / 2];
     double pot_rmin[kMaxTypes * (kMaxTypes + 1) / 2];
@@ -179,6 +179,12 @@ struct AtomsView {
 __device__ __forceinline__ double nint_ref(double x) {
     return static_cast<double>(x < 0. ? static_cast<int>(__dadd_rn(x, -0.5))
                                       : static_cast<int>(__dadd_rn(x, 0.5)));
+}
+
+// rint(x) for |x| < 2^22 by adding 1.5 * 2^23: two FP32 additions instead of a conversion on the
+// narrow unit that also takes the square roots and the conversions to FP64
+__device__ __forceinline__ float round_small(float x) {
+    return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f);
 }
 
 // md_driver.cpp:175-185 with the reference's exact operations (no contraction):

@@ -61,12 +61,6 @@ __host__ __device__ __forceinline__ float gr_margin(float H, float u) {
     return 1.7321f * 2.3842e-7f * H + 4.7684e-7f * u;
 }
 
-// rint(x) for |x| < 2^22 by adding 1.5 * 2^23: two FP32 additions instead of a conversion
-// on the narrow unit that also takes the reciprocal square root
-__device__ __forceinline__ float round_small(float x) {
-    return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f);
-}
-
 // the reference's operations: the pair's bin, or -1. From r2_skip on certainly dr >= rmaxg.
 __device__ __forceinline__ double gr_r2_skip(GrArgs const &g) {
     return g.rmaxg * g.rmaxg * (1. + 1e-12);

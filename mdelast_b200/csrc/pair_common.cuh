@@ -53,11 +53,6 @@ __device__ __forceinline__ float4 position_f(double4 c, Replica const *R) {
                        static_cast<float>((c.z - nint_ref(c.z)) * R->h[2] * u),
                        __int_as_float(static_cast<int>(c.w)));
 }
-// rint(x) for |x| < 2^22 by adding 1.5 * 2^23: two FP32 additions instead of a conversion on the
-// narrow unit that also takes the square roots and the conversions to FP64
-__device__ __forceinline__ float round_small(float x) {
-    return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f);
-}
 // minimum image of pi - pj in a box of edges L (positions wrapped into [-L/2, L/2)) and its
 // square. Every operation is an odd function: the image seen from j is the negative, bit for bit.
 __device__ __forceinline__ float min_image_f(float4 pi, float4 pj, float3 L, float3 iL,
