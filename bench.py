@@ -815,7 +815,7 @@ def half_list_nbar(m, t, cell):
 # replicas without cache flushing (the launches of timed-region steps, so the L2 holds
 # what the preceding kernels of the step left in it), mean over the captured launches.
 # None where not captured.
-TRAFFIC_PER_LAUNCH: dict = {("mixed", 16, False): 80.14e6 + 1.19e6,
+TRAFFIC_PER_LAUNCH: dict = {("mixed", 16, False): 80.09e6 + 1.19e6,
                             ("mixed", 16, True): 78.89e6 + 0.77e6}
 
 

@@ -512,13 +512,13 @@ __device__ __forceinline__ void force_row_mx(AtomsView const &A, TablesView cons
 // over atoms go through warp_slots (31 and, at 4 lanes per atom, 4 exchanges) into two FP64
 // registers per lane; the virial is the trace of the Born stress.
 //
-// What bounds it: scattered gathers, by their wavefronts (67 per 32 visits, 52 % of the L1 data
+// What bounds it: scattered gathers, by their wavefronts (67 per 32 visits, 54 % of the L1 data
 // pipe's rate) and their latency at 4 blocks of 4 warps per SM, with instruction issue (47 %) behind. At 16 x 13,500 atoms and 4 lanes per
 // atom: 0.416 ms when the sums' shuffles and shared accumulators were 19 % of the data pipe's
 // work and the third table function of one-type pairs another 20 %, 0.362 ms without them, 0.345 with
 // even row halves, 0.314 with the products of the coefficients in the table records, the r_min test
 // once per row, pair slots from a byte table and no unrolling, 0.300 with 48 instead of 64 bytes of
-// tables for a one-type pair.
+// tables for a one-type pair, 0.296 without the second walk that r_min could ask for.
 //
 // STAGED: the block first copies the staged quintic tables (T.stf, T.st_bytes, about 180 KB
 // for a two-element alloy) into dynamic shared memory and reads every staged interval from
